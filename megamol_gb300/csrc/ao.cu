@@ -55,24 +55,10 @@ __global__ void __launch_bounds__(256) mip_level_kernel(const float* __restrict_
     }
 }
 
-// One thread per particle: marches all cones (throughput: millions of particles). Particle i's data are
-// read at order[i] (or i) and its AO is written at out_order[i] (or there): the frame's kernels read sorted
-// copies and scatter the AO straight to input order.
-__global__ void __launch_bounds__(128) cone_ao_kernel(const ConeParams cp, const uint32_t* __restrict__ order,
-    const float4* __restrict__ xyzr, const float4* __restrict__ nrm, uint32_t n, const uint32_t* __restrict__ out_order,
-    float* __restrict__ ao) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n)
-        return;
-    const uint32_t o = order ? order[i] : i;
-    const uint32_t w = out_order ? out_order[i] : o;
-    ao[w] = cone_ao_at<true>(cp, xyzr[o], nrm[o]);
-}
-
 // One warp per cone: a block takes one particle with one warp per cone, and the lanes of a warp take the
 // cone's samples (32 at a time: the step positions are tabulated, so all samples load at once). Every lane
 // then runs the march's recurrence over the shuffled samples in step order with the same early exit, the
-// block's first thread adds the cones in cone order: the result has the bits of cone_ao_kernel. A bounded
+// block's first thread adds the cones in cone order: the result has the bits of cone_blocks_kernel. A bounded
 // grid strides over the particles: the learned AO's fallback list (list and its device-side length n_dev,
 // usually tiny, where latency matters), or a whole frame (no list: particle i; P2V_AO_MARCH_WARP), where
 // every lane stays busy whatever step its cone ends at, at the price of the samples past the early exit.
@@ -482,17 +468,13 @@ cudaError_t launch_cone_ao_warp(const ConeParams& cp, const float4* xyzr, const 
     return cudaGetLastError();
 }
 
-cudaError_t launch_cone_ao(const ConeParams& cp, const uint32_t* order, const float4* xyzr, const float4* nrm,
+cudaError_t launch_cone_ao_list(const ConeParams& cp, const uint32_t* list, const float4* xyzr, const float4* nrm,
     uint32_t n, const uint32_t* n_dev, const uint32_t* out_order, float* ao, cudaStream_t st) {
     if (n == 0)
         return cudaSuccess;
-    if (n_dev == nullptr) {
-        cone_ao_kernel<<<ceil_div(n, 128), 128, 0, st>>>(cp, order, xyzr, nrm, n, out_order, ao);
-    } else {
-        // the learned AO's fallback list: one block of ncones warps per particle, a bounded grid
-        const unsigned grd = (unsigned) std::min<uint32_t>(n, 4096u);
-        cone_ao_list_kernel<<<grd, 32 * cp.ncones, 0, st>>>(cp, order, xyzr, nrm, n, n_dev, out_order, ao);
-    }
+    // one block of ncones warps per particle, a bounded grid
+    const unsigned grd = (unsigned) std::min<uint32_t>(n, 4096u);
+    cone_ao_list_kernel<<<grd, 32 * cp.ncones, 0, st>>>(cp, list, xyzr, nrm, n, n_dev, out_order, ao);
     return cudaGetLastError();
 }
 

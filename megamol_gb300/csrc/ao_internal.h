@@ -106,15 +106,33 @@ cudaError_t launch_mip_levels(const float* l0, const int d0[3], float sat_scale,
 // acc: scratch of 4 (unorm8) or 8 bytes per voxel; vol: level 0 of the MDAO volume (x fastest)
 cudaError_t launch_mdao_volume(const MdaoParams& mp, const uint32_t* order, const float4* xyzr, uint32_t n,
     void* acc, float* vol, int sms, cudaStream_t st);
-// n_dev (nullable): device-side particle count, at most n (the cone march of the learned-AO fallback list)
 // xyzr_s[j] = xyzr[order[j]] (skipped when xyzr is null), nrm_s[j] = nrm[order[j]] (sorted order).
 cudaError_t launch_sort_particles(const uint32_t* order, uint32_t n, const float4* xyzr, const float4* nrm,
     float4* xyzr_s, float4* nrm_s, int sms, cudaStream_t st);
-// particle i (or list entry i) reads xyzr / nrm at order[i] (or i); its AO goes to ao[out_order[that index]]
-// when out_order is given (sorted copies in, input order out), else to ao[that index]
-cudaError_t launch_cone_ao(const ConeParams& cp, const uint32_t* order, const float4* xyzr, const float4* nrm,
+// the learned AO's fallback: entry i of list (its length at most n, on the device at n_dev) reads xyzr / nrm at
+// list[i]; its AO goes to ao[out_order[list[i]]] when out_order is given (sorted copies in, input order out), else to
+// ao[list[i]]
+cudaError_t launch_cone_ao_list(const ConeParams& cp, const uint32_t* list, const float4* xyzr, const float4* nrm,
     uint32_t n, const uint32_t* n_dev, const uint32_t* out_order, float* ao, cudaStream_t st);
-// the whole frame with one warp per cone of a particle (the bits of launch_cone_ao)
+// Corner blocks of the mip levels the plain march samples: for every texel corner of a level the eight texels around
+// it, contiguous (32 bytes).
+struct ConeBlocks {
+    struct Level {
+        float fx, fy, fz;    // texels per axis
+        uint32_t off;        // block index bias
+        uint32_t sx, sxy;    // blocks per row and per slice; sxy = 0: the level is sampled from its texels
+        uint32_t first;      // first block of the level
+    };
+    const float* blocks;     // nblocks blocks of 8 floats, 32-byte aligned
+    Level lv[MAX_LEVELS];
+    float wlo, whi;          // normalised coordinates past which every level's samples are zero
+    uint32_t nblocks;
+};
+ConeBlocks cone_block_plan(const ConeParams& cp, uint32_t n);
+// builds the blocks and marches the whole frame: particle i's AO goes to ao[out_order[i]] (or ao[i])
+cudaError_t launch_cone_blocks(const ConeParams& cp, ConeBlocks cb, float* blocks, const float4* xyzr, const float4* nrm,
+                               uint32_t n, const uint32_t* out_order, float* ao, int sms, cudaStream_t st);
+// the whole frame with one warp per cone of a particle (the bits of launch_cone_blocks)
 cudaError_t launch_cone_ao_warp(const ConeParams& cp, const float4* xyzr, const float4* nrm, uint32_t n,
     const uint32_t* out_order, float* ao, int sms, cudaStream_t st);
 cudaError_t launch_aosphere(const AOSphereParams& ap, const float4* xyzr, uint32_t n, unsigned long long* acc,

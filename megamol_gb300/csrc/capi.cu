@@ -73,6 +73,7 @@ struct Pipe {
     DevBuf bcount;                         // particles per cell (the counting sort)
     DevBuf bstart;                         // start of every 64th cell (the radix path's cell starts)
     DevBuf xyzr_s, nrm_s;                  // positions and normals in sorted order (the cone AO stages)
+    DevBuf cblocks;                        // corner blocks of the plain march's mip levels
     DevBuf bk0, bk1, xyzr_b, nrm_b, ord_b;  // the AO stages' brick order (ao_brick_order)
     bool xyzr_sorted = false;              // the binning of this frame wrote xyzr_s
     bool timing = false;                   // this frame records stage events
@@ -125,7 +126,7 @@ struct Pipe {
         for (DevBuf* b : {&raw, &xyzr, &rec_a, &keys0, &keys1, &vals0, &vals1, &status, &hist, &cstart, &gaps,
                           &grid, &tiles, &scal, &nrm, &ao, &mips, &aos_acc, &aos_tex, &mdao_acc, &mdao_vol, &fb_list,
                           &wts, &wsorted, &wsum, &vdens, &vdirs, &vkeys0, &vkeys1, &vvals0, &vvals1, &vout, &bcount, &bstart, &xyzr_s, &nrm_s, &bk0, &bk1, &xyzr_b, &nrm_b,
-                          &ord_b})
+                          &ord_b, &cblocks})
             b->release();
         for (FeatureTex& t : ftex)
             t.release();
@@ -1284,10 +1285,14 @@ p2v_status p2v_ctx::run_ao(Pipe& pp, const p2v_frame* fr, const GridGeo& g, cons
         P2V_CUDA_TRY(ao_inputs());
         if (pp.timing)
             P2V_CUDA_TRY(cudaEventRecord(pp.ev[EV_AOK0], st));
-        if (P.ao_march == P2V_AO_MARCH_WARP)
+        if (P.ao_march == P2V_AO_MARCH_WARP) {
             P2V_CUDA_TRY(launch_cone_ao_warp(cp, axyzr, anrm, n, aorder, ao.as<float>(), sms, st));
-        else
-            P2V_CUDA_TRY(launch_cone_ao(cp, nullptr, axyzr, anrm, n, nullptr, aorder, ao.as<float>(), st));
+        } else {
+            const ConeBlocks cb = cone_block_plan(cp, n);
+            P2V_CUDA_TRY(pp.cblocks.ensure(32 * (size_t) cb.nblocks));
+            P2V_CUDA_TRY(launch_cone_blocks(cp, cb, pp.cblocks.as<float>(), axyzr, anrm, n, aorder, ao.as<float>(), sms,
+                                            st));
+        }
         if (pp.timing) {
             P2V_CUDA_TRY(cudaEventRecord(pp.ev[EV_AOK1], st));
             pp.aok = true;
@@ -1342,8 +1347,8 @@ p2v_status p2v_ctx::run_ao(Pipe& pp, const p2v_frame* fr, const GridGeo& g, cons
             pp.aok = true;
         }
         // the plain cone march for every particle whose features left the training range
-        P2V_CUDA_TRY(launch_cone_ao(cp, fb_list.as<uint32_t>(), axyzr, anrm, n, &fs->ao_fallback, aorder,
-                                    ao.as<float>(), st));
+        P2V_CUDA_TRY(launch_cone_ao_list(cp, fb_list.as<uint32_t>(), axyzr, anrm, n, &fs->ao_fallback, aorder,
+                                         ao.as<float>(), st));
         return P2V_OK;
     }
     if (P.ao_mode == P2V_AO_AOSPHERE_AXES || P.ao_mode == P2V_AO_AOSPHERE_NORMAL) {

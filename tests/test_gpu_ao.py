@@ -211,3 +211,29 @@ def test_brick_order_gives_the_same_bits(ctx, march):
     c, _, _ = run_ao(ctx, f, nrm, ao_brick_order=1, ao_normals=p2v.NORMALS_GRADIENT, **kw)
     d, _, _ = run_ao(ctx, f, nrm, ao_brick_order=0, ao_normals=p2v.NORMALS_GRADIENT, **kw)
     assert np.array_equal(c, d)
+
+
+@pytest.mark.parametrize("n,res,over", [
+    (1, (40, 40, 40), {}),                                        # no level has more samples than texels
+    (3_001, (97, 33, 64), dict(ao_cones=3, ao_steps=0)),          # some levels blocked, one thread per cone
+    (40_000, (31, 64, 45), dict(ao_cones=16, ao_levels=6)),
+    (40_000, (31, 64, 45), dict(ao_cones=5, ao_early_exit=0, ao_volume_scale=3.0)),
+    (20_000, (64, 64, 64), dict(ao_cones=8, ao_offset=0.7, ao_cone_length=0.1)),  # distances that shrink
+    (20_000, (64, 64, 64), dict(ao_cones=8, ao_apex_deg=20.0, ao_volume=p2v.AOVOL_MDAO)),
+    (152 * 2048 + 77, (80, 81, 79), dict(ao_cones=8)),            # one thread per particle
+])
+def test_block_march_has_the_bits_of_the_texel_march(ctx, n, res, over):
+    """The march on corner blocks equals the march on the levels' texels (one warp per cone) bit for bit: particles
+    inside, on and beyond the walls, zero normals and cones along an axis among them."""
+    f = synth.uniform(n=n, edge=30.0, seed=77)
+    f.res = res
+    rng = np.random.default_rng(78)
+    out = rng.random(n) < 0.2
+    f.xyzr[out, :3] = (f.xyzr[out, :3] - 15.0) * 1.3 + 15.0       # some of them outside the box
+    nrm = synth.random_normals(n, 79)
+    nrm[::7] = 0.0
+    nrm[1::11] = (0.0, 0.0, 1.0)
+    kw = dict(dict(ao_mode=p2v.AO_CONE, ao_cones=8, ao_steps=32, ao_levels=3), **over)
+    a, _, _ = run_ao(ctx, f, nrm, ao_march=p2v.AO_MARCH_THREAD, **kw)
+    b, _, _ = run_ao(ctx, f, nrm, ao_march=p2v.AO_MARCH_WARP, **kw)
+    assert np.array_equal(a, b)
