@@ -73,6 +73,7 @@ struct Pipe {
     DevBuf bcount;                         // particles per cell (the counting sort)
     DevBuf bstart;                         // start of every 64th cell (the radix path's cell starts)
     DevBuf xyzr_s, nrm_s;                  // positions and normals in sorted order (the cone AO stages)
+    DevBuf heavy;                          // the exact gather's crowded tiles
     DevBuf cblocks;                        // corner blocks of the plain march's mip levels
     DevBuf bk0, bk1, xyzr_b, nrm_b, ord_b;  // the AO stages' brick order (ao_brick_order)
     bool xyzr_sorted = false;              // the binning of this frame wrote xyzr_s
@@ -126,7 +127,7 @@ struct Pipe {
         for (DevBuf* b : {&raw, &xyzr, &rec_a, &keys0, &keys1, &vals0, &vals1, &status, &hist, &cstart, &gaps,
                           &grid, &tiles, &scal, &nrm, &ao, &mips, &aos_acc, &aos_tex, &mdao_acc, &mdao_vol, &fb_list,
                           &wts, &wsorted, &wsum, &vdens, &vdirs, &vkeys0, &vkeys1, &vvals0, &vvals1, &vout, &bcount, &bstart, &xyzr_s, &nrm_s, &bk0, &bk1, &xyzr_b, &nrm_b,
-                          &ord_b, &cblocks})
+                          &ord_b, &cblocks, &heavy})
             b->release();
         for (FeatureTex& t : ftex)
             t.release();
@@ -513,11 +514,11 @@ p2v_status p2v_ctx::enqueue_frame(Pipe& pp, const p2v_frame* fr, p2v_volume* vol
     if (P.accumulate == P2V_ACCUM_KAHAN) {
         gc = GatherConfig{GATHER_KAHAN, 8, 16, 16, 2048, 1024};
     } else if (P.accumulate == P2V_ACCUM_EXACT) {
-        gc = GatherConfig{GATHER_EXACT, 16, 16, 16, 0, 1024};
+        gc = GatherConfig{GATHER_EXACT, 16, 16, 16, 0, 512};
         if (P.tile_x > 0 || P.tile_y > 0 || P.tile_z > 0)
-            gc = GatherConfig{GATHER_EXACT, P.tile_x, P.tile_y, P.tile_z, 0, 1024};
+            gc = GatherConfig{GATHER_EXACT, P.tile_x, P.tile_y, P.tile_z, 0, 512};
         else if (tuned_tile[0] > 0)
-            gc = GatherConfig{GATHER_EXACT, tuned_tile[0], tuned_tile[1], tuned_tile[2], 0, 1024};
+            gc = GatherConfig{GATHER_EXACT, tuned_tile[0], tuned_tile[1], tuned_tile[2], 0, 512};
     } else {
         return fail(P2V_EINVAL, "unknown accumulate mode %d", P.accumulate);
     }
@@ -778,25 +779,29 @@ p2v_status p2v_ctx::enqueue_frame(Pipe& pp, const p2v_frame* fr, p2v_volume* vol
     } else {
         // aggregator 0: the density; 1: the intensity-weighted sums; 2: three direction-weighted passes into
         // the interleaved vector volume and the plain kernel sums (the weights) into wsum
-        const int passes = agg == 2 ? 4 : 1;
-        for (int pass = 0; pass < passes; ++pass) {
-            GatherWeights gw{};
-            float* out = dgrid;
-            if (agg == 1) {
-                gw.mode = GatherWeights::FIXED;
-                gw.w = pp.wsorted.as<float>();
-            } else if (agg == 2 && pass < 3) {
-                gw.mode = GatherWeights::DOUBLE;
-                gw.w = pp.wsorted.as<float>() + pass;
-                gw.wstride = 3;
-                gw.ostride = 3;
-                out = dgrid + pass;
-            } else if (agg == 2) {
-                gw.mode = GatherWeights::DOUBLE;  // the weights: plain kernel sums in FP64
-                out = pp.wsum.as<float>();
+        GatherPasses ps{};
+        ps.out[0] = dgrid;
+        if (agg == 1) {
+            ps.mode = GatherPasses::FIXED;
+            ps.w[0] = pp.wsorted.as<float>();
+        } else if (agg == 2) {
+            ps.mode = GatherPasses::DOUBLE;
+            ps.count = 4;
+            ps.wstride = 3;
+            for (int c = 0; c < 3; ++c) {
+                ps.w[c] = pp.wsorted.as<float>() + c;
+                ps.out[c] = dgrid + c;
+                ps.ostride[c] = 3;
             }
-            const cudaError_t ge = launch_gather(gc, g, sb.rec_a, sb.rec_b, cstart.as<uint32_t>(),
-                                                 out, tiles.as<TileStats>(), fs, st, gw);
+            ps.out[3] = pp.wsum.as<float>();  // the weights: plain kernel sums
+        }
+        size_t hbytes = 0;
+        const GatherHeavy hv = gather_heavy_plan(gc, n, sms, &hbytes);
+        if (hbytes)
+            P2V_CUDA_TRY(pp.heavy.ensure(hbytes));
+        {
+            const cudaError_t ge = launch_gather(gc, g, sb.rec_a, sb.rec_b, cstart.as<uint32_t>(), ps,
+                                                 tiles.as<TileStats>(), fs, hv, pp.heavy.ptr, sms, st);
             if (ge == cudaErrorInvalidValue)
                 return fail(P2V_EUNSUPPORTED, "density tile %dx%dx%d is not compiled for accumulate=%d", gc.tx, gc.ty,
                             gc.tz, P.accumulate);

@@ -12,7 +12,9 @@
 // the kernel support; nodes outside the support receive exactly zero in the reference as well.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "p2v_common.cuh"
 #include "p2v_internal.h"
@@ -39,6 +41,46 @@ struct Extent {
     float eps2_max;
     int ok;
 };
+
+// Candidate extents and cyclic images of a tile along axis a (its first node at o3[a]), written to ex: threads 0 to 2 of
+// a block take one axis each.
+__device__ __forceinline__ void tile_extent(const GridGeo& g, FrameScalars* fs, const int o3[3], const int T3[3], int a,
+                                            Extent& ex) {
+    const bool bump = g.kernel == 0;
+    const float rmax_r = __uint_as_float(fs->rmax_bits);
+    const float eps_max = bump ? g.sigma * rmax_r : 3.0f * (g.sigma * rmax_r);
+    if (a == 0) {
+        ex.ok = rmax_r > 0.0f;
+        // enlarged slightly so rounding never prunes a contributing cell row
+        ex.eps2_max = eps_max * eps_max * 1.0001f;
+    }
+    if (!(rmax_r > 0.0f))
+        return;
+    int E = static_cast<int>(ceilf(eps_max / g.hhi[a] + 1e-3f));
+    E = E < 1 ? 1 : E;
+    const int F = bump ? static_cast<int>(fminf(ceilf(rmax_r / g.hf[a]), 255.0f)) : E;
+    int L = bump ? min(E, F + 1) : E, H = bump ? min(E - 1, F) : E - 1;
+    if (L > 100) {  // the Kahan gather keeps staged cell offsets in 8 bits
+        atomicOr(&fs->error, ERR_WINDOW_TOO_WIDE);
+        L = 100;
+        H = min(H, 100);
+    }
+    int klo = 0, khi = 0;
+    if (g.cyc[a]) {
+        // images k with [o + k s - L, o + T - 1 + k s + H] meeting the occupied cells
+        const int s = g.s[a];
+        klo = -floor_div(-(fs->cmin[a] - o3[a] - T3[a] + 1 - H), s);
+        khi = floor_div(fs->cmax[a] - o3[a] + L, s);
+        if (khi - klo + 1 > MAX_IMAGES) {
+            atomicOr(&fs->error, ERR_WINDOW_TOO_WIDE);
+            khi = klo + MAX_IMAGES - 1;
+        }
+    }
+    ex.L[a] = L;
+    ex.H[a] = H;
+    ex.klo[a] = klo;
+    ex.khi[a] = khi;
+}
 
 template<int TX, int TY, int TZ>
 __global__ void __launch_bounds__(TY* TZ, 2) gather_kernel(GridGeo g, const float4* __restrict__ rec_a,
@@ -73,40 +115,9 @@ __global__ void __launch_bounds__(TY* TZ, 2) gather_kernel(GridGeo g, const floa
     const bool bump = g.kernel == 0;
     const float E45 = __expf(-4.5f);
     // ---- candidate extents from the largest radius, once per CTA ----
-    if (t == 0) {
-        const float rmax_r = __uint_as_float(fs->rmax_bits);
-        Extent ex;
-        ex.ok = rmax_r > 0.0f;
-        const float eps_max = bump ? g.sigma * rmax_r : 3.0f * (g.sigma * rmax_r);
-        // enlarged slightly so rounding never prunes a contributing cell row
-        ex.eps2_max = eps_max * eps_max * 1.0001f;
+    if (t < 3) {
         const int o3[3] = {x0, y0, z0};
-        for (int a = 0; a < 3 && ex.ok; ++a) {
-            int E = static_cast<int>(ceilf(eps_max / g.hhi[a] + 1e-3f));
-            E = E < 1 ? 1 : E;
-            const int F = bump ? static_cast<int>(fminf(ceilf(rmax_r / g.hf[a]), 255.0f)) : E;
-            ex.L[a] = bump ? min(E, F + 1) : E;
-            ex.H[a] = bump ? min(E - 1, F) : E - 1;
-            if (ex.L[a] > 100) {  // staged cell offsets are kept in 8 bits
-                atomicOr(&fs->error, ERR_WINDOW_TOO_WIDE);
-                ex.L[a] = 100;
-                ex.H[a] = min(ex.H[a], 100);
-            }
-            if (g.cyc[a]) {
-                const int s = g.s[a];
-                // images k with [o + k s - L, o + T - 1 + k s + H] meeting the occupied cells
-                ex.klo[a] = -floor_div(-(fs->cmin[a] - o3[a] - T3[a] + 1 - ex.H[a]), s);
-                ex.khi[a] = floor_div(fs->cmax[a] - o3[a] + ex.L[a], s);
-                if (ex.khi[a] - ex.klo[a] + 1 > MAX_IMAGES) {
-                    atomicOr(&fs->error, ERR_WINDOW_TOO_WIDE);
-                    ex.khi[a] = ex.klo[a] + MAX_IMAGES - 1;
-                }
-            } else {
-                ex.klo[a] = 0;
-                ex.khi[a] = 0;
-            }
-        }
-        s_ex = ex;
+        tile_extent(g, fs, o3, T3, t, s_ex);
     }
     __syncthreads();
     const Extent ex = s_ex;
@@ -361,86 +372,13 @@ __global__ void __launch_bounds__(TY* TZ, 2) gather_kernel(GridGeo g, const floa
     }
 }
 
-// Candidate extents and cyclic images of one tile (shared by both gather kernels).
-__device__ __forceinline__ Extent tile_extent(const GridGeo& g, FrameScalars* fs, const int o3[3], const int T3[3]) {
-    const bool bump = g.kernel == 0;
-    const float rmax_r = __uint_as_float(fs->rmax_bits);
-    Extent ex;
-    ex.ok = rmax_r > 0.0f;
-    const float eps_max = bump ? g.sigma * rmax_r : 3.0f * (g.sigma * rmax_r);
-    ex.eps2_max = eps_max * eps_max * 1.0001f;
-    for (int a = 0; a < 3 && ex.ok; ++a) {
-        int E = static_cast<int>(ceilf(eps_max / g.hhi[a] + 1e-3f));
-        E = E < 1 ? 1 : E;
-        const int F = bump ? static_cast<int>(fminf(ceilf(rmax_r / g.hf[a]), 255.0f)) : E;
-        ex.L[a] = bump ? min(E, F + 1) : E;
-        ex.H[a] = bump ? min(E - 1, F) : E - 1;
-        if (ex.L[a] > 100) {
-            atomicOr(&fs->error, ERR_WINDOW_TOO_WIDE);
-            ex.L[a] = 100;
-            ex.H[a] = min(ex.H[a], 100);
-        }
-        if (g.cyc[a]) {
-            const int s = g.s[a];
-            ex.klo[a] = -floor_div(-(fs->cmin[a] - o3[a] - T3[a] + 1 - ex.H[a]), s);
-            ex.khi[a] = floor_div(fs->cmax[a] - o3[a] + ex.L[a], s);
-            if (ex.khi[a] - ex.klo[a] + 1 > MAX_IMAGES) {
-                atomicOr(&fs->error, ERR_WINDOW_TOO_WIDE);
-                ex.khi[a] = ex.klo[a] + MAX_IMAGES - 1;
-            }
-        } else {
-            ex.klo[a] = 0;
-            ex.khi[a] = 0;
-        }
-    }
-    return ex;
-}
-
-// One particle's node box as the warp-level walk needs it (held in registers, then published to
-// shared memory field by field so that lanes reading different particles never conflict on a bank).
-struct WarpPart {
-    float d0[3];       // (box corner - particle) in cells, per axis
-    float eps2, inv;   // squared support and kernel scale
-    float iby;         // 1/by for decoding a box-local row index
-    int bx, by;        // box extents in x and y
-    int node0;         // tile index of the box corner
-    float w;           // the particle's weight (the weighted aggregators)
-};
-constexpr int WP_FIELDS = 10;
-
-// Fixed-point scale of the exact accumulation: contributions (all below 1) are rounded to multiples of
-// 2^-32 and summed as 64-bit integers held in two 32-bit words per node (a 32-bit shared-memory atomic on
-// the low word; the thread whose add wraps it carries into the high word), so every voxel holds the exact
-// sum of its rounded FP32 contributions, independent of the order in which particles arrive.
-constexpr float FIX_SCALE = 4294967296.0f;          // 2^32
-constexpr float FIX_INV = 2.3283064365386963e-10f;  // 2^-32
-
-// The float nearest (ties to even) to the fixed-point sum hi:lo times 2^-32, from 32-bit integer operations
-// and one exact 32-bit conversion: the same value as __ull2float_rn(hi:lo) * 2^-32, without the 64-bit
-// conversion, which like FP64 arithmetic runs on the narrow FP64 pipe of this part. q receives the rounded
-// sum (v * 2^32, an integer).
-__device__ __forceinline__ float fixed_to_float(uint32_t hi, uint32_t lo, unsigned long long& q) {
-    const unsigned long long x = ((unsigned long long) hi << 32) | lo;
-    const int sh = 40 - __clzll(x);  // bits below a 24-bit significand (x == 0: -24)
-    if (sh <= 0) {
-        q = x;  // below 2^24: exact
-        return __uint2float_rn(lo) * FIX_INV;
-    }
-    unsigned long long m = x >> sh;
-    const unsigned long long rem = x & ((1ull << sh) - 1ull), half = 1ull << (sh - 1);
-    m += (rem > half || (rem == half && (m & 1ull))) ? 1ull : 0ull;  // m <= 2^24
-    q = m << sh;
-    // m * 2^(sh - 32): the significand converts exactly and the scale is a power of two (sh in [1, 40])
-    return __uint2float_rn((uint32_t) m) * __int_as_float((95 + sh) << 23);
-}
-
-// Particle-major gather with exact, order-independent accumulation. A CTA owns a tile of TX*TY*TZ
-// nodes held as 64-bit fixed-point sums in shared memory; for every cyclic image of the tile it walks
-// the sorted particle records of the surrounding cell rows (coalesced 16-byte loads), and each thread
-// adds its particle's kernel values to the nodes of the particle's footprint that lie in the tile.
+// ---------------------------------------------------------------------------------------------
+// Particle-major gather with exact, order-independent accumulation. A CTA owns a tile of TX*TY*TZ nodes held in
+// shared memory; for every cyclic image of the tile it walks the sorted particle records of the surrounding cell
+// rows (16-byte loads) and adds each particle's kernel values to the nodes of its footprint that lie in the tile.
 //
 // ACC selects the accumulation:
-//   ACC_EXACT   the density: contributions < 1 in 2^-32 fixed point (see above);
+//   ACC_EXACT   the density: every contribution (all below 1) is rounded to a multiple of 2^-32 and summed exactly;
 //   ACC_FIXED_W the intensity aggregator (ParticlesToDensity.cpp:509-519): contribution = kernel value times
 //               the particle's weight w (wts[j * wstride], sorted order), rounded to a multiple of 1 / wscale
 //               with wscale = 2^31 / 2^ceil(log2 max|w|) and summed as a signed 64-bit integer (exact, order
@@ -450,7 +388,116 @@ __device__ __forceinline__ float fixed_to_float(uint32_t hi, uint32_t lo, unsign
 //               (a fixed-point quantum would erase voxels reached only by kernel tails); the sums depend on
 //               the arrival order only at the 1e-16 level, below the final rounding to FP32.
 // The result is written with stride ostride.
+//
+// Bound by issue slots, and on sparse frames by the latency of the phases around the walk (row table, output): 68 % of
+// the issue slots on LJ 4M. A warp's 32 lanes take 32 (particle, x-row) items at a time; about 11 lanes add a node in an
+// average step of the x loop, and an item costs about 35 instructions around it (LJ 4M 0.272 ms, mixed 64M 1.23 ms,
+// uniform 16M 3.51 ms, four passes of 500k 0.143 ms). Before: one addition per node whose old value gave the carry, a
+// binary search per item, conversions on the special-function unit and whole batches dealt to the warps: 0.369, 1.75,
+// 5.73 and 0.249 ms. Skipping the x loop, uniform 16M takes 1.79 ms, of that 0.18 the box set-up, 0.73 the row table,
+// 0.59 the output.
 constexpr int ACC_EXACT = 0, ACC_FIXED_W = 1, ACC_DOUBLE = 2;
+
+constexpr int GATHER_RES = 1024;  // threads resident per SM (64 registers each; 1280 at 48 spill: mixed 64M +6 %)
+
+// ACC_EXACT: a contribution of q 2^-32 is added as its two 16-bit halves, q >> 16 to the node's high word and q & 65535
+// to its low word (node sum = high 2^16 + low, in 64 bits), by two shared-memory additions whose old values nobody
+// reads. Neither word overflows below 2^16 contributions. ACC_FIXED_W does the same with a signed high half. A tile that
+// one CTA has to walk with more records than that uses `carry` words instead: q to the low word, the carry of the
+// addition that wraps it to the high word (node sum = high 2^32 + low); ACC_FIXED_W 64-bit additions.
+constexpr uint32_t SPLIT_MAX_RECORDS = 1u << 15;
+constexpr float FIX_INV = 2.3283064365386963e-10f;  // 2^-32
+
+// The two halves of rn(v 2^32), v in [0, 1), from fused multiply-adds: t = floor(v 2^16) and u = rn(rest) sit in the low
+// mantissa bits above 2^23. (The same integer as __float2uint_rn(v 2^32): every product and 2^23 - 2^16 t are exact, and
+// 2^16 t is even. The conversion instruction runs at a quarter of the rate of each of these.)
+__device__ __forceinline__ void fixed_halves(float v, uint32_t& hi, uint32_t& lo) {
+    const float t = __fmaf_rz(v, 65536.0f, 8388608.0f);
+    const float u = __fmaf_rn(v, 4294967296.0f, __fmaf_rn(__fsub_rn(t, 8388608.0f), -65536.0f, 8388608.0f));
+    hi = __float_as_uint(t) - 0x4B000000u;
+    lo = __float_as_uint(u) - 0x4B000000u;
+}
+
+// The float nearest (ties to even) to x 2^-32: sums below 1 take one 32-bit conversion, others 32-bit integer
+// operations and one exact conversion (64-bit conversions run on the narrow FP64 pipe of this part).
+__device__ __forceinline__ float fixed_to_float(unsigned long long x) {
+    if ((uint32_t) (x >> 32) == 0u)
+        return __uint2float_rn((uint32_t) x) * FIX_INV;
+    const int sh = 40 - __clzll(x);  // bits below a 24-bit significand
+    unsigned long long m = x >> sh;
+    const unsigned long long rem = x & ((1ull << sh) - 1ull), half = 1ull << (sh - 1);
+    m += (rem > half || (rem == half && (m & 1ull))) ? 1ull : 0ull;  // m <= 2^24
+    // m * 2^(sh - 32): the significand converts exactly and the scale is a power of two (sh in [9, 40])
+    return __uint2float_rn((uint32_t) m) * __int_as_float((95 + sh) << 23);
+}
+
+// x < 2^23 as a float, from full-rate operations
+__device__ __forceinline__ float small_float(uint32_t x) {
+    return __uint_as_float(0x4B000000u | x) - 8388608.0f;
+}
+
+// exp(x) as __expf computes it, and 1 / w. FTZ: results below the normal floats are 0 (they lie far below the fixed
+// point's quantum), which spares the scaling around the special-function unit; w is never subnormal (1 - x of a float x).
+template<bool FTZ>
+__device__ __forceinline__ float exp_fast(float x) {
+    if (!FTZ)
+        return __expf(x);
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__fmul_rn(x, 1.4426950408889634f)));
+    return y;
+}
+__device__ __forceinline__ float rcp_fast(float w) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(w));
+    return y;
+}
+
+// The kernel at squared distance d2 inside the support. The hardware reciprocal and exponential: the kernel's relative
+// error stays below 1e-6 where it exceeds 1e-7 of its peak (at 1/w = 16, e^-16 = 1.1e-7 of the peak, the reciprocal's
+// 2.4e-7 relative error moves e^-1/w by 3.8e-6 of itself).
+template<bool BUMP, bool FTZ>
+__device__ __forceinline__ float kernel_value(float d2, float inv, float e45) {
+    if (BUMP) {
+        const float w = __fmaf_rn(-d2, inv, 1.0f);
+        return w > 0.0f ? exp_fast<FTZ>(-rcp_fast(w)) : 0.0f;
+    }
+    return fmaxf(exp_fast<FTZ>(-d2 * inv) - e45, 0.0f);
+}
+
+// Adds a kernel value to a node of the CTA's sums (smem: [nn] low and [nn] high words, or [nn] 64-bit sums).
+template<int ACC>
+__device__ __forceinline__ void add_node(unsigned char* smem, int nn, uint32_t node, float v, float weight, float wscale,
+                                         bool carry) {
+    if (ACC == ACC_FIXED_W) {
+        // |w wscale| <= 2^31 and v < 0.99: the rounded contribution fits 32 bits
+        const int q = __float2int_rn(__fmul_rn(__fmul_rn(v, weight), wscale));
+        if (!carry) {
+            uint32_t* lo = reinterpret_cast<uint32_t*>(smem) + node;
+            atomicAdd(lo, (uint32_t) q & 0xFFFFu);
+            atomicAdd(lo + nn, (uint32_t) (q >> 16));
+        } else {
+            atomicAdd(reinterpret_cast<unsigned long long*>(smem) + node, (unsigned long long) (long long) q);
+        }
+    } else if (ACC == ACC_DOUBLE) {
+        const float c = __fmul_rn(v, weight);  // rbf * val, in float
+        if (c != 0.0f)
+            atomicAdd(reinterpret_cast<double*>(smem) + node, (double) c);
+    } else {
+        uint32_t* lo = reinterpret_cast<uint32_t*>(smem) + node;
+        uint32_t* hi = lo + nn;
+        uint32_t qh, ql;
+        fixed_halves(v, qh, ql);
+        if (!carry) {
+            atomicAdd(lo, ql);
+            atomicAdd(hi, qh);
+        } else {
+            const uint32_t q = (qh << 16) + ql;
+            const uint32_t old = atomicAdd(lo, q);
+            if (old + q < old)
+                atomicAdd(hi, 1u);
+        }
+    }
+}
 
 // Sorted position of the f-th staged record: the row r with row_off[r] <= f < row_off[r + 1] holds it.
 __device__ __forceinline__ uint32_t locate_record(const uint32_t* row_off, const uint32_t* row_beg, int nrows,
@@ -465,301 +512,345 @@ __device__ __forceinline__ uint32_t locate_record(const uint32_t* row_off, const
     }
     return row_beg[lo] + (f - row_off[lo]);
 }
-template<int TX, int TY, int TZ, int NT, int ACC>
-__global__ void __launch_bounds__(NT, 1024 / NT) gather_fixed_kernel(GridGeo g, const float4* __restrict__ rec_a,
-    const int4* __restrict__ rec_b, const uint32_t* __restrict__ start, float* __restrict__ grid,
-    TileStats* __restrict__ tiles, FrameScalars* __restrict__ fs, int rmax, const float* __restrict__ wts,
-    int wstride, int ostride) {
+
+// Crowded tiles (a blob trajectory's centres: 250,000 records in one tile, which one CTA walked for 2 ms while the others
+// had finished; 32 frames 26.5 -> 18.7 ms). A tile with more than `limit` records is not walked by its own CTA: that CTA counts its records,
+// clears a slot of 64-bit sums in `acc` and queues the tile in parts of `chunk` records; gather_heavy_kernel's CTAs
+// take the parts, each adds its sums to the slot, and the part that finishes last writes the tile. Integer sums: the
+// same result in any order. fs->heavy counts tiles (from bit 40) and parts; a full queue leaves the tile to its own CTA.
+template<int TX, int TY, int TZ, int NT>
+struct GatherShared {
+    static constexpr int NN = TX * TY * TZ;
+    double dsum[NT / 32];
+    unsigned long long isum[NT / 32], fsum[NT / 32];
+    float fmin[NT / 32], fmax[NT / 32];
+    uint32_t wsum[NT / 32];
+    uint32_t slot;
+    Extent ex;
+};
+
+enum WalkMode { WALK_ALL, WALK_PART, WALK_COUNT };
+constexpr uint32_t WALK_OVER = 0xFFFFFFFFu;
+
+// One CTA's walk of a tile's records (image by image, row by row). WALK_ALL adds every record, WALK_PART those numbered
+// [rlo, rhi), WALK_COUNT none. Returns the number of records, or WALK_OVER as soon as there are more than `limit` (the
+// sums are then void). Every thread returns the same.
+template<int TX, int TY, int TZ, int NT, int ACC, bool BUMP>
+__device__ __forceinline__ uint32_t walk_tile(const GridGeo& g, const float4* __restrict__ rec_a,
+    const int4* __restrict__ rec_b, const uint32_t* __restrict__ start, FrameScalars* __restrict__ fs, int rmax,
+    const float* __restrict__ wts, int wstride, float wscale, const int o3[3], GatherShared<TX, TY, TZ, NT>& sh,
+    unsigned char* smem, WalkMode mode, uint32_t rlo, uint32_t rhi, bool carry, uint32_t limit) {
     constexpr int NN = TX * TY * TZ;
-    extern __shared__ __align__(16) unsigned char smem[];
-    uint32_t* acc_lo = reinterpret_cast<uint32_t*>(smem);  // [NN] low words of the fixed-point sums
-    uint32_t* acc_hi = acc_lo + NN;                        // [NN] high words
-    unsigned long long* acc64 = reinterpret_cast<unsigned long long*>(smem);  // [NN] ACC_FIXED_W sums (same bytes)
-    double* accd = reinterpret_cast<double*>(smem);                          // [NN] ACC_DOUBLE sums (same bytes)
     constexpr bool WEIGHTED = ACC != ACC_EXACT;
-    uint32_t* row_beg = acc_hi + NN;                        // [rmax]
-    uint32_t* row_off = row_beg + rmax;                                      // [rmax + 1]
-    __shared__ double s_dsum[NT / 32];
-    __shared__ unsigned long long s_isum[NT / 32], s_fsum[NT / 32];
-    __shared__ float s_fmin[NT / 32], s_fmax[NT / 32];
-    __shared__ Extent s_ex;
-    __shared__ uint32_t s_part[WP_FIELDS][NT];
-    __shared__ uint32_t s_pre[NT + 32];
-
+    float4* part_a = reinterpret_cast<float4*>(smem + 8 * NN);                  // [NT] (box corner - particle) xyz, eps^2
+    uint4* part_b = reinterpret_cast<uint4*>(part_a + NT);                      // [NT] kernel scale, corner node, rows, weight
+    uint32_t* row_beg = reinterpret_cast<uint32_t*>(part_b + NT);               // [rmax]
+    uint32_t* row_off = row_beg + rmax;                                         // [rmax + 1]
     const int t = threadIdx.x;
-    const uint32_t lane = t & 31u;
-    const uint32_t warp = t >> 5;
-    // tiles cover the slab [zlo, zhi) of the grid (z tile index offset by the slab's first tile)
-    const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, z0 = (blockIdx.z + g.zlo / TZ) * TZ;
-    const int T3[3] = {TX, TY, TZ};
-    const int o3[3] = {x0, y0, z0};
-    for (int n = t; n < NN; n += NT) {
-        acc_lo[n] = 0u;
-        acc_hi[n] = 0u;
-    }
-    const bool bump = g.kernel == 0;
+    const uint32_t lane = t & 31u, warp = t >> 5;
+    const uint32_t le_mask = 0xFFFFFFFFu >> (31u - lane);
     const float E45 = __expf(-4.5f);
-    float wscale = 1.0f, winv = 1.0f;
-    if (ACC == ACC_FIXED_W) {
-        const float wmax = __uint_as_float(fs->wmax_bits);
-        if (wmax > 0.0f) {
-            int e;
-            frexpf(wmax, &e);  // wmax <= 2^e
-            e = max(e, -90);
-            wscale = ldexpf(1.0f, 31 - e);
-            winv = ldexpf(1.0f, e - 31);
-        }
-    }
-    if (t == 0)
-        s_ex = tile_extent(g, fs, o3, T3);
-    __syncthreads();
-    const Extent ex = s_ex;
-
-    if (ex.ok) {
-        for (int kz = ex.klo[2]; kz <= ex.khi[2]; ++kz)
-            for (int ky = ex.klo[1]; ky <= ex.khi[1]; ++ky)
-                for (int kx = ex.klo[0]; kx <= ex.khi[0]; ++kx) {
-                    const int u0[3] = {x0 + kx * g.s[0], y0 + ky * g.s[1], z0 + kz * g.s[2]};
-                    int wlo[3], whi[3];
+    const int T3[3] = {TX, TY, TZ};
+    const Extent& ex = sh.ex;
+    uint32_t seen = 0;
+    for (int kz = ex.klo[2]; kz <= ex.khi[2]; ++kz)
+        for (int ky = ex.klo[1]; ky <= ex.khi[1]; ++ky)
+            for (int kx = ex.klo[0]; kx <= ex.khi[0]; ++kx) {
+                const int u0[3] = {o3[0] + kx * g.s[0], o3[1] + ky * g.s[1], o3[2] + kz * g.s[2]};
+                int wlo[3], whi[3];
 #pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        wlo[a] = min(max(u0[a] - ex.L[a], -1), g.s[a]);
-                        whi[a] = max(min(u0[a] + T3[a] - 1 + ex.H[a], g.s[a]), -1);
-                    }
-                    const int nwy = whi[1] - wlo[1] + 1;
-                    const int nwz = whi[2] - wlo[2] + 1;
-                    if (nwy > rmax) {
-                        if (t == 0)
-                            atomicOr(&fs->error, ERR_STAGE_OVERFLOW);
-                        continue;
-                    }
-                    const int planes_per_chunk = rmax / nwy;
-                    const uint32_t bx_lo = (uint32_t) (wlo[0] + 1), bx_end = (uint32_t) (whi[0] + 2);
-                    for (int pz0 = 0; pz0 < nwz; pz0 += planes_per_chunk) {
-                        const int pz1 = min(nwz, pz0 + planes_per_chunk);
-                        const int nrows = (pz1 - pz0) * nwy;
-                        __syncthreads();
-                        for (int r = t; r < nrows; r += NT) {
-                            const int zz = wlo[2] + pz0 + r / nwy;
-                            const int yy = wlo[1] + r % nwy;
+                for (int a = 0; a < 3; ++a) {
+                    wlo[a] = min(max(u0[a] - ex.L[a], -1), g.s[a]);
+                    whi[a] = max(min(u0[a] + T3[a] - 1 + ex.H[a], g.s[a]), -1);
+                }
+                const int nwy = whi[1] - wlo[1] + 1;
+                const int nwz = whi[2] - wlo[2] + 1;
+                if (nwy > rmax) {
+                    if (t == 0)
+                        atomicOr(&fs->error, ERR_STAGE_OVERFLOW);
+                    continue;
+                }
+                const int planes_per_chunk = rmax / nwy;
+                const uint32_t bx_lo = (uint32_t) (wlo[0] + 1), bx_end = (uint32_t) (whi[0] + 2);
+                for (int pz0 = 0; pz0 < nwz; pz0 += planes_per_chunk) {
+                    const int pz1 = min(nwz, pz0 + planes_per_chunk);
+                    const int nrows = (pz1 - pz0) * nwy;
+                    __syncthreads();
+                    // row table: every cell row's records, and their exclusive scan over the rows, two rows per thread
+                    // (rmax <= 2 NT), all table reads in flight together
+                    uint32_t total = 0, cnt[2], sum = 0;
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int r = 2 * t + e;
+                        cnt[e] = 0;
+                        if (r < nrows) {
+                            const int zr = r / nwy;
+                            const int zz = wlo[2] + pz0 + zr;
+                            const int yy = wlo[1] + r - zr * nwy;
                             const uint32_t rowkey = ((uint32_t) (zz + 1) * g.nb[1] + (uint32_t) (yy + 1)) * g.nb[0];
                             const uint32_t b = start[rowkey + bx_lo];
+                            cnt[e] = start[rowkey + bx_end] - b;
                             row_beg[r] = b;
-                            row_off[r + 1] = start[rowkey + bx_end] - b;
                         }
-                        __syncthreads();
-                        if (t < 32) {
-                            uint32_t carry = 0;
-                            for (int base = 0; base < nrows; base += 32) {
-                                const int r = base + t;
-                                uint32_t v = r < nrows ? row_off[r + 1] : 0u;
+                        sum += cnt[e];
+                    }
+                    uint32_t incl = sum;
 #pragma unroll
-                                for (int o = 1; o < 32; o <<= 1) {
-                                    uint32_t u = __shfl_up_sync(0xffffffffu, v, o);
-                                    if (t >= o)
-                                        v += u;
-                                }
-                                if (r < nrows)
-                                    row_off[r + 1] = carry + v;
-                                carry += __shfl_sync(0xffffffffu, v, 31);
-                            }
-                            if (t == 0)
-                                row_off[0] = 0;
-                        }
-                        __syncthreads();
-                        const uint32_t total = row_off[nrows];
-                        // Each warp takes 32 consecutive records; every lane derives its particle's node
-                        // box, then the warp walks the concatenated boxes 32 nodes at a time (a warp-level
-                        // load-balanced search), so all lanes test nodes in lockstep.
-                        // the warp's next 32 records are located and loaded one iteration ahead (their
-                        // latency overlaps the current batch's nodes)
-                        uint32_t jn = 0;
-                        float4 An = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                        int4 Bn = make_int4(0, 0, 0, 0);
-                        if (warp * 32 + lane < total) {
-                            jn = locate_record(row_off, row_beg, nrows, warp * 32 + lane);
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+                        if (lane >= (uint32_t) o)
+                            incl += u;
+                    }
+                    if (lane == 31)
+                        sh.wsum[warp] = incl;
+                    __syncthreads();
+                    uint32_t pre = incl - sum;
+#pragma unroll
+                    for (int w = 0; w < NT / 32; ++w) {
+                        const uint32_t v = sh.wsum[w];
+                        pre += w < (int) warp ? v : 0u;
+                        total += v;
+                    }
+                    if (2 * t < nrows)
+                        row_off[2 * t] = pre;
+                    if (2 * t + 1 < nrows)
+                        row_off[2 * t + 1] = pre + cnt[0];
+                    const uint32_t first = seen;
+                    seen = seen + total < seen ? WALK_OVER : seen + total;
+                    if (seen > limit)
+                        return WALK_OVER;
+                    if (mode == WALK_COUNT || (mode == WALK_PART && (seen <= rlo || first >= rhi)))
+                        continue;
+                    if (t == 0)
+                        row_off[nrows] = total;
+                    __syncthreads();
+                    const uint32_t flo = mode == WALK_PART && rlo > first ? rlo - first : 0u;
+                    const uint32_t fhi = mode == WALK_PART ? min(total, rhi - first) : total;
+                    // The warps take equal shares of the records, in equal batches of at most 32; every lane derives its
+                    // particle's node box, then the warp walks the concatenated (particle, x-row) items 32 at a time. The
+                    // next batch is located and loaded one iteration ahead (its latency overlaps the current one's nodes).
+                    const uint32_t share = (fhi - flo + NT / 32 - 1u) / (NT / 32);
+                    const uint32_t wlo_r = min(flo + warp * share, fhi), whi_r = min(wlo_r + share, fhi);
+                    const uint32_t nbatch = (share + 31u) / 32u;
+                    const uint32_t step = nbatch > 0 ? (share + nbatch - 1u) / nbatch : 1u;
+                    uint32_t jn = 0;
+                    float4 An = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    int4 Bn = make_int4(0, 0, 0, 0);
+                    if (lane < step && wlo_r + lane < whi_r) {
+                        jn = locate_record(row_off, row_beg, nrows, wlo_r + lane);
+                        An = rec_a[REC_STRIDE * (size_t) jn];
+                        Bn = rec_b[REC_STRIDE * (size_t) jn];
+                    }
+                    for (uint32_t base = wlo_r; base < whi_r; base += step) {
+                        const uint32_t f = base + lane;
+                        const uint32_t j = jn;
+                        const float4 A = An;
+                        const int4 B = Bn;
+                        if (lane < step && f + step < whi_r) {
+                            jn = locate_record(row_off, row_beg, nrows, f + step);
                             An = rec_a[REC_STRIDE * (size_t) jn];
                             Bn = rec_b[REC_STRIDE * (size_t) jn];
                         }
-                        for (uint32_t base = warp * 32; base < total; base += NT) {
-                            const uint32_t f = base + lane;
-                            uint32_t nb = 0;
-                            WarpPart wp;
-                            const uint32_t j = jn;
-                            const float4 A = An;
-                            const int4 B = Bn;
-                            if (f + NT < total) {
-                                jn = locate_record(row_off, row_beg, nrows, f + NT);
-                                An = rec_a[REC_STRIDE * (size_t) jn];
-                                Bn = rec_b[REC_STRIDE * (size_t) jn];
-                            }
-                            if (f < total) {
-                                const float phi[3] = {A.x, A.y, A.z};
-                                const int cf[3] = {B.x, B.y, B.z};
-                                const uint32_t meta = (uint32_t) B.w;
-                                const float r = A.w;
-                                const float eps = bump ? g.sigma * r : 3.0f * (g.sigma * r);
-                                int blo[3], bw[3];
-                                bool empty = false;
+                        uint32_t nb = 0, bx = 0, by = 1, node0 = 0;
+                        float d0[3], eps2 = 0.0f, inv = 0.0f;
+                        if (lane < step && f < whi_r) {
+                            const float phi[3] = {A.x, A.y, A.z};
+                            const int cf[3] = {B.x, B.y, B.z};
+                            const uint32_t meta = (uint32_t) B.w;
+                            const float r = A.w;
+                            const float eps = BUMP ? g.sigma * r : 3.0f * (g.sigma * r);
+                            int blo[3], bw[3];
+                            bool empty = false;
 #pragma unroll
-                                for (int a = 0; a < 3; ++a) {
-                                    const int cr = cf[a] - u0[a];
-                                    const float pos = static_cast<float>(cr) + phi[a];
-                                    const float eh = eps * g.ihh[a];
-                                    // nodes k with |k - pos| < eps / h; a node the rounding drops lies at
-                                    // the edge of the support, where the kernel is zero
-                                    int lo_a = static_cast<int>(floorf(pos - eh)) + 1;
-                                    int hi_a = static_cast<int>(ceilf(pos + eh)) - 1;
-                                    if (bump) {
-                                        const int fa = (int) ((meta >> (8 * a)) & 0xFFu);
-                                        const int ctr = cr + (int) ((meta >> (24 + a)) & 1u);
-                                        lo_a = max(lo_a, ctr - fa);
-                                        hi_a = min(hi_a, ctr + fa);
-                                    }
-                                    lo_a = max(lo_a, 0);
-                                    hi_a = min(hi_a, T3[a] - 1);
-                                    empty = empty || lo_a > hi_a;
-                                    blo[a] = lo_a;
-                                    bw[a] = hi_a - lo_a + 1;
-                                    // node offset from the particle, in cells: (k - cr) - phi = (k - lo) + d0
-                                    wp.d0[a] = static_cast<float>(lo_a - cr) - phi[a];
+                            for (int a = 0; a < 3; ++a) {
+                                const int cr = cf[a] - u0[a];
+                                const float pos = static_cast<float>(cr) + phi[a];
+                                const float eh = eps * g.ihh[a];
+                                // nodes k with |k - pos| < eps / h; a node the rounding drops lies at
+                                // the edge of the support, where the kernel is zero
+                                int lo_a = static_cast<int>(floorf(pos - eh)) + 1;
+                                int hi_a = static_cast<int>(ceilf(pos + eh)) - 1;
+                                if (BUMP) {
+                                    const int fa = (int) ((meta >> (8 * a)) & 0xFFu);
+                                    const int ctr = cr + (int) ((meta >> (24 + a)) & 1u);
+                                    lo_a = max(lo_a, ctr - fa);
+                                    hi_a = min(hi_a, ctr + fa);
                                 }
-                                if (!empty) {
-                                    nb = (uint32_t) (bw[1] * bw[2]);  // x-rows of the box
-                                    if (bump) {
-                                        wp.eps2 = eps * eps;
-                                        wp.inv = __frcp_rn(wp.eps2);
-                                    } else {
-                                        const float sg = g.sigma * r;
-                                        wp.eps2 = 9.0f * sg * sg;
-                                        wp.inv = __frcp_rn(2.0f * sg * sg);
-                                    }
-                                    wp.bx = bw[0];
-                                    wp.by = bw[1];
-                                    wp.node0 = (blo[2] * TY + blo[1]) * TX + blo[0];
-                                    wp.iby = 1.0f / (float) bw[1];
-                                    if (WEIGHTED)
-                                        wp.w = wts ? __ldg(wts + (size_t) j * wstride) : 1.0f;
+                                lo_a = max(lo_a, 0);
+                                hi_a = min(hi_a, T3[a] - 1);
+                                empty = empty || lo_a > hi_a;
+                                blo[a] = lo_a;
+                                bw[a] = hi_a - lo_a + 1;
+                                // node offset from the particle, in cells: (k - cr) - phi = (k - lo) + d0
+                                d0[a] = static_cast<float>(lo_a - cr) - phi[a];
+                            }
+                            if (!empty) {
+                                bx = (uint32_t) bw[0];
+                                by = (uint32_t) bw[1];
+                                nb = by * (uint32_t) bw[2];  // x-rows of the box
+                                if (BUMP) {
+                                    eps2 = eps * eps;
+                                    inv = __frcp_rn(eps2);
+                                } else {
+                                    const float sg = g.sigma * r;
+                                    eps2 = 9.0f * sg * sg;
+                                    inv = __frcp_rn(2.0f * sg * sg);
                                 }
+                                // with the scaled reciprocal that splits a row number into z and y
+                                const uint32_t m = (uint32_t) __fdividef(4096.0f, static_cast<float>(bw[1])) + 1u;
+                                node0 = (uint32_t) ((blo[2] * TY + blo[1]) * TX + blo[0]) | (m << 16);
                             }
-                            // exclusive prefix of the row counts over the warp
-                            uint32_t incl = nb;
-#pragma unroll
-                            for (int o = 1; o < 32; o <<= 1) {
-                                const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
-                                if (lane >= (uint32_t) o)
-                                    incl += u;
-                            }
-                            const uint32_t wtotal = __shfl_sync(0xffffffffu, incl, 31);
-                            if (wtotal == 0)
-                                continue;
-                            const int wl = warp * 32 + lane;
-                            s_part[0][wl] = __float_as_uint(wp.d0[0]);
-                            s_part[1][wl] = __float_as_uint(wp.d0[1]);
-                            s_part[2][wl] = __float_as_uint(wp.d0[2]);
-                            s_part[3][wl] = __float_as_uint(wp.eps2);
-                            s_part[4][wl] = __float_as_uint(wp.inv);
-                            s_part[5][wl] = __float_as_uint(wp.iby);
-                            s_part[6][wl] = (uint32_t) wp.bx;
-                            s_part[7][wl] = (uint32_t) wp.by;
-                            s_part[8][wl] = (uint32_t) wp.node0;
-                            if (WEIGHTED)
-                                s_part[9][wl] = __float_as_uint(wp.w);
-                            s_pre[wl] = incl - nb;
-                            __syncwarp();
-                            const uint32_t* pre = s_pre + warp * 32;
-                            for (uint32_t j0 = 0; j0 < wtotal; j0 += 32) {
-                                const uint32_t jj = j0 + lane;
-                                if (jj < wtotal) {
-                                    // owner: the last lane whose prefix is <= jj (its box is non-empty)
-                                    int o = 0;
-#pragma unroll
-                                    for (int step = 16; step > 0; step >>= 1)
-                                        if (pre[o + step] <= jj)
-                                            o += step;
-                                    const int ow = warp * 32 + o;
-                                    const int local = (int) (jj - pre[o]);
-                                    const int by = (int) s_part[7][ow];
-                                    const int zl = (int) ((static_cast<float>(local) + 0.5f) * __uint_as_float(s_part[5][ow]));
-                                    const int yl = local - zl * by;
-                                    const float dy = g.hhi[1] * (static_cast<float>(yl) + __uint_as_float(s_part[1][ow]));
-                                    const float dz = g.hhi[2] * (static_cast<float>(zl) + __uint_as_float(s_part[2][ow]));
-                                    const float dyz = __fmaf_rn(dy, dy, dz * dz);
-                                    const float eps2 = __uint_as_float(s_part[3][ow]);
-                                    if (dyz < eps2) {
-                                        const float inv = __uint_as_float(s_part[4][ow]);
-                                        const float d0x = __uint_as_float(s_part[0][ow]);
-                                        const int bx = (int) s_part[6][ow];
-                                        const int row = (int) s_part[8][ow] + (zl * TY + yl) * TX;
-                                        const float pw = WEIGHTED ? __uint_as_float(s_part[9][ow]) : 0.0f;
-                                        for (int xl = 0; xl < bx; ++xl) {
-                                            const float dx = g.hhi[0] * (static_cast<float>(xl) + d0x);
-                                            const float d2 = __fmaf_rn(dx, dx, dyz);
-                                            if (!(d2 < eps2))
-                                                continue;
-                                            // the hardware reciprocal (__fdividef, within 2 ulp) and exponential:
-                                            // the kernel's relative error stays below 1e-6 where it exceeds 1e-7 of
-                                            // its peak (at 1/w = 16, e^-16 = 1.1e-7 of the peak, the reciprocal's
-                                            // 2.4e-7 relative error moves e^-1/w by 3.8e-6 of itself)
-                                            float v;
-                                            if (bump) {
-                                                const float w = __fmaf_rn(-d2, inv, 1.0f);
-                                                v = w > 0.0f ? __expf(-__fdividef(1.0f, w)) : 0.0f;
-                                            } else {
-                                                v = fmaxf(__expf(-d2 * inv) - E45, 0.0f);
-                                            }
-                                            if (ACC == ACC_FIXED_W) {
-                                                const long long q = __float2ll_rn(__fmul_rn(__fmul_rn(v, pw), wscale));
-                                                if (q != 0)
-                                                    atomicAdd(acc64 + row + xl, (unsigned long long) q);
-                                            } else if (ACC == ACC_DOUBLE) {
-                                                const float c = __fmul_rn(v, pw);  // rbf * val, in float
-                                                if (c != 0.0f)
-                                                    atomicAdd(accd + row + xl, (double) c);
-                                            } else {
-                                                const uint32_t q = __float2uint_rn(v * FIX_SCALE);
-                                                if (q != 0u) {
-                                                    const uint32_t old = atomicAdd(acc_lo + row + xl, q);
-                                                    if (old + q < old)
-                                                        atomicAdd(acc_hi + row + xl, 1u);
-                                                }
-                                            }
-                                        }
-                                    }
-                                }
-                            }
-                            __syncwarp();
                         }
+                        // exclusive prefix of the row counts over the warp; the particles with rows take consecutive slots
+                        uint32_t rows = nb;
+#pragma unroll
+                        for (int o = 1; o < 32; o <<= 1) {
+                            const uint32_t u = __shfl_up_sync(0xffffffffu, rows, o);
+                            if (lane >= (uint32_t) o)
+                                rows += u;
+                        }
+                        const uint32_t wtotal = __shfl_sync(0xffffffffu, rows, 31);
+                        if (wtotal == 0)
+                            continue;
+                        const uint32_t prow = nb ? rows - nb : 0xFFFFu;  // (at most 32 * 256 rows)
+                        const uint32_t full = __ballot_sync(0xffffffffu, nb != 0u);
+                        if (nb) {
+                            const uint32_t at = warp * 32 + __popc(full & (le_mask >> 1));
+                            part_a[at] = make_float4(d0[0], d0[1], d0[2], eps2);
+                            part_b[at] = make_uint4(__float_as_uint(inv), node0, prow | (bx << 16) | (by << 24),
+                                                    WEIGHTED ? __float_as_uint(wts ? __ldg(wts + (size_t) j * wstride) : 1.0f)
+                                                             : 0u);
+                        }
+                        __syncwarp();
+                        uint32_t before = warp * 32 - 1u;  // slots whose rows start before the current 32 items, less one
+                        for (uint32_t j0 = 0; j0 < wtotal; j0 += 32) {
+                            // bit b: a particle's first row is item j0 + b; the item's particle is the last one that has
+                            // started (no search: one reduction and a population count)
+                            const uint32_t heads =
+                                __reduce_or_sync(0xffffffffu, prow - j0 < 32u ? 1u << (prow - j0) : 0u);
+                            const uint32_t slot = before + __popc(heads & le_mask);
+                            before += __popc(heads);
+                            const uint32_t jj = j0 + lane;
+                            if (jj < wtotal) {
+                                const float4 PA = part_a[slot];
+                                const uint4 PB = part_b[slot];
+                                const uint32_t pby = PB.z >> 24, pbx = (PB.z >> 16) & 0xFFu;
+                                const uint32_t local = jj - (PB.z & 0xFFFFu);
+                                const uint32_t zl = (local * (PB.y >> 16)) >> 12;  // local / by: local < 256, by <= 16
+                                const uint32_t yl = local - zl * pby;
+                                const float dy = g.hhi[1] * (small_float(yl) + PA.y);
+                                const float dz = g.hhi[2] * (small_float(zl) + PA.z);
+                                const float dyz = __fmaf_rn(dy, dy, dz * dz);
+                                const float re2 = PA.w;
+                                if (dyz < re2) {
+                                    const float rinv = __uint_as_float(PB.x);
+                                    const uint32_t row = (PB.y & 0xFFFFu) + (zl * TY + yl) * TX;
+                                    const float pw = WEIGHTED ? __uint_as_float(PB.w) : 0.0f;
+                                    float xf = 0.0f;
+#pragma unroll(BUMP ? 4 : 2)
+                                    for (uint32_t xl = 0; xl < pbx; ++xl, xf += 1.0f) {
+                                        const float dx = g.hhi[0] * (xf + PA.x);
+                                        const float d2 = __fmaf_rn(dx, dx, dyz);
+                                        if (d2 < re2)
+                                            add_node<ACC>(smem, NN, row + xl, kernel_value<BUMP, ACC != ACC_DOUBLE>(d2, rinv, E45), pw,
+                                                          wscale, carry);
+                                    }
+                                }
+                            }
+                        }
+                        __syncwarp();
                     }
                 }
-    }
-    __syncthreads();
+            }
+    return seen;
+}
 
-    // ---- write the tile (x fastest, coalesced) and its statistics ----
-    // The density's tile sum is exact in integers: every output value is a multiple of 2^-32, and the
-    // integer and fractional parts of the rounded sums are added separately (each below 2^44 for a tile), so
-    // no node pays an FP64 conversion and add (the FP64 pipe of this part is 1/64 of the FP32 rate).
+// The 64-bit sums of nodes n .. n + 3, n a multiple of 4 (ACC_DOUBLE: their bits).
+template<int NN, int ACC>
+__device__ __forceinline__ void node_sums(const unsigned char* smem, int n, bool carry, unsigned long long q[4]) {
+    if (ACC == ACC_DOUBLE || (ACC == ACC_FIXED_W && carry)) {
+        const ulonglong2* p = reinterpret_cast<const ulonglong2*>(reinterpret_cast<const unsigned long long*>(smem) + n);
+        const ulonglong2 a = p[0], b = p[1];
+        q[0] = a.x;
+        q[1] = a.y;
+        q[2] = b.x;
+        q[3] = b.y;
+        return;
+    }
+    const uint4 lo = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint32_t*>(smem) + n);
+    const uint4 hi = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint32_t*>(smem) + NN + n);
+    if (ACC == ACC_FIXED_W) {  // signed high words
+        q[0] = (unsigned long long) ((long long) (int) hi.x * 65536) + lo.x;
+        q[1] = (unsigned long long) ((long long) (int) hi.y * 65536) + lo.y;
+        q[2] = (unsigned long long) ((long long) (int) hi.z * 65536) + lo.z;
+        q[3] = (unsigned long long) ((long long) (int) hi.w * 65536) + lo.w;
+        return;
+    }
+    const int sh = carry ? 32 : 16;
+    q[0] = ((unsigned long long) hi.x << sh) + lo.x;
+    q[1] = ((unsigned long long) hi.y << sh) + lo.y;
+    q[2] = ((unsigned long long) hi.z << sh) + lo.z;
+    q[3] = ((unsigned long long) hi.w << sh) + lo.w;
+}
+
+// Float bits as integers in the floats' order (no NaN), for integer warp reductions, and back.
+__device__ __forceinline__ int order_bits(float v) {
+    const int b = __float_as_int(v);
+    return b ^ ((b >> 31) & 0x7FFFFFFF);
+}
+__device__ __forceinline__ float unorder(int b) {
+    return __int_as_float(b ^ ((b >> 31) & 0x7FFFFFFF));
+}
+
+// Writes a tile (x fastest, coalesced) and its statistics. sums: the tile's slot of 64-bit sums, or null: the CTA's own.
+// The density's tile sum is exact in integers (no node pays an FP64 addition: the FP64 pipe of this part is 1/64 of the
+// FP32 rate).
+template<int TX, int TY, int TZ, int NT, int ACC>
+__device__ __forceinline__ void write_tile(const GridGeo& g, const int o3[3], GatherShared<TX, TY, TZ, NT>& sh,
+    const unsigned char* smem, const unsigned long long* sums, bool carry, float winv, float* __restrict__ grid, int ostride,
+    TileStats* __restrict__ ts_out) {
+    constexpr int NN = TX * TY * TZ;
+    const int t = threadIdx.x;
     double dsum = 0.0;
-    unsigned long long isum = 0ull, fsum = 0ull;
+    unsigned long long isum = 0ull, fsum = 0ull;  // whole and fractional parts (each below 2^44 for a tile)
     float vmin = INFINITY, vmax = -INFINITY;
-    for (int n = t; n < NN; n += NT) {
-        const int x = n % TX, y = (n / TX) % TY, z = n / (TX * TY);
-        if (x0 + x < g.s[0] && y0 + y < g.s[1] && z0 + z >= g.zlo && z0 + z < g.zhi) {
+    // four nodes along x per thread and round
+#pragma unroll 2
+    for (int n = 4 * t; n < NN; n += 4 * NT) {
+        const int x = o3[0] + n % TX, y = o3[1] + (n / TX) % TY, z = o3[2] + n / (TX * TY);
+        if (x >= g.s[0] || y >= g.s[1] || z < g.zlo || z >= g.zhi)
+            continue;
+        float* out = grid + (((size_t) (z - g.zlo) * g.s[1] + y) * g.s[0] + x) * (size_t) ostride;
+        unsigned long long q[4];
+        if (sums) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                q[e] = __ldcg(sums + n + e);
+        } else {
+            node_sums<NN, ACC>(smem, n, carry, q);
+        }
+        const int m = min(4, g.s[0] - x);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if (e >= m)
+                break;
             float v;
             if (ACC == ACC_EXACT) {
-                unsigned long long q;
-                v = fixed_to_float(acc_hi[n], acc_lo[n], q);
-                isum += q >> 32;
-                fsum += q & 0xFFFFFFFFull;
+                v = fixed_to_float(q[e]);
+                isum += q[e] >> 32;
+                fsum += q[e] & 0xFFFFFFFFull;
             } else {
-                v = ACC == ACC_FIXED_W ? __ll2float_rn((long long) acc64[n]) * winv : __double2float_rn(accd[n]);
+                v = ACC == ACC_FIXED_W ? __ll2float_rn((long long) q[e]) * winv
+                                       : __double2float_rn(__longlong_as_double((long long) q[e]));
                 dsum += (double) v;
             }
-            grid[(((size_t) (z0 + z - g.zlo) * g.s[1] + (y0 + y)) * g.s[0] + (x0 + x)) * (size_t) ostride] = v;
+            out[e * ostride] = v;
             vmin = fminf(vmin, v);
             vmax = fmaxf(vmax, v);
         }
     }
+    if (!ts_out)  // (uniform)
+        return;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         if (ACC == ACC_EXACT) {
@@ -768,24 +859,24 @@ __global__ void __launch_bounds__(NT, 1024 / NT) gather_fixed_kernel(GridGeo g, 
         } else {
             dsum += __shfl_xor_sync(0xffffffffu, dsum, o);
         }
-        vmin = fminf(vmin, __shfl_xor_sync(0xffffffffu, vmin, o));
-        vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
     }
+    vmin = unorder(__reduce_min_sync(0xffffffffu, order_bits(vmin)));
+    vmax = unorder(__reduce_max_sync(0xffffffffu, order_bits(vmax)));
     if ((t & 31) == 0) {
-        s_dsum[t >> 5] = dsum;
-        s_isum[t >> 5] = isum;
-        s_fsum[t >> 5] = fsum;
-        s_fmin[t >> 5] = vmin;
-        s_fmax[t >> 5] = vmax;
+        sh.dsum[t >> 5] = dsum;
+        sh.isum[t >> 5] = isum;
+        sh.fsum[t >> 5] = fsum;
+        sh.fmin[t >> 5] = vmin;
+        sh.fmax[t >> 5] = vmax;
     }
     __syncthreads();
     if (t == 0) {
         for (int w = 1; w < NT / 32; ++w) {
-            dsum += s_dsum[w];
-            isum += s_isum[w];
-            fsum += s_fsum[w];
-            vmin = fminf(vmin, s_fmin[w]);
-            vmax = fmaxf(vmax, s_fmax[w]);
+            dsum += sh.dsum[w];
+            isum += sh.isum[w];
+            fsum += sh.fsum[w];
+            vmin = fminf(vmin, sh.fmin[w]);
+            vmax = fmaxf(vmax, sh.fmax[w]);
         }
         if (ACC == ACC_EXACT)
             dsum = (double) isum + (double) fsum * 2.3283064365386963e-10;
@@ -793,7 +884,158 @@ __global__ void __launch_bounds__(NT, 1024 / NT) gather_fixed_kernel(GridGeo g, 
         ts.sum = dsum;
         ts.vmin = vmin;
         ts.vmax = vmax;
-        tiles[(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = ts;
+        *ts_out = ts;
+    }
+}
+
+// 2^31 / 2^ceil(log2 max|w|) of the frame's weights, and its inverse (ACC_FIXED_W)
+__device__ __forceinline__ void weight_scale(const FrameScalars* fs, float& wscale, float& winv) {
+    wscale = winv = 1.0f;
+    const float wmax = __uint_as_float(fs->wmax_bits);
+    if (wmax > 0.0f) {
+        int e;
+        frexpf(wmax, &e);  // wmax <= 2^e
+        e = max(e, -90);
+        wscale = ldexpf(1.0f, 31 - e);
+        winv = ldexpf(1.0f, e - 31);
+    }
+}
+
+template<int NN, int NT>
+__device__ __forceinline__ void clear_sums(unsigned char* smem) {
+    for (int n = threadIdx.x; n < NN / 2; n += NT)
+        reinterpret_cast<uint4*>(smem)[n] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+template<int TX, int TY, int TZ, int NT, int ACC, bool BUMP>
+__global__ void __launch_bounds__(NT, GATHER_RES / NT) gather_fixed_kernel(const __grid_constant__ GridGeo g,
+    const float4* __restrict__ rec_a, const int4* __restrict__ rec_b, const uint32_t* __restrict__ start,
+    const __grid_constant__ GatherPasses ps, TileStats* __restrict__ tiles, FrameScalars* __restrict__ fs, int rmax,
+    const GatherHeavy hv, uint32_t tiles_z) {
+    constexpr int NN = TX * TY * TZ;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ GatherShared<TX, TY, TZ, NT> sh;
+    const int t = threadIdx.x;
+    // tiles cover the slab [zlo, zhi) of the grid (z tile index offset by the slab's first tile)
+    const uint32_t pass = blockIdx.z / tiles_z, bz = blockIdx.z - pass * tiles_z;
+    const uint32_t tile = (bz * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+    const int o3[3] = {(int) blockIdx.x * TX, (int) blockIdx.y * TY, (int) (bz + g.zlo / TZ) * TZ};
+    clear_sums<NN, NT>(smem);
+    if (t < 3) {
+        const int T3[3] = {TX, TY, TZ};
+        tile_extent(g, fs, o3, T3, t, sh.ex);
+    }
+    float wscale = 1.0f, winv = 1.0f;
+    if (ACC == ACC_FIXED_W)
+        weight_scale(fs, wscale, winv);
+    __syncthreads();
+    bool carry = false;
+    if (sh.ex.ok) {
+        uint32_t seen = walk_tile<TX, TY, TZ, NT, ACC, BUMP>(g, rec_a, rec_b, start, fs, rmax, ps.w[pass], ps.wstride, wscale, o3,
+                                                       sh, smem, WALK_ALL, 0u, 0u, false, hv.limit);
+        if (seen == WALK_OVER) {
+            uint32_t slot = 0xFFFFFFFFu;
+            if (hv.cap > 0) {
+                seen = walk_tile<TX, TY, TZ, NT, ACC, BUMP>(g, rec_a, rec_b, start, fs, rmax, nullptr, 1, wscale, o3, sh, smem,
+                                                      WALK_COUNT, 0u, 0u, false, WALK_OVER - 1u);
+                if (t == 0) {
+                    sh.slot = slot;
+                    if (seen != WALK_OVER) {
+                        const uint32_t parts = (seen + hv.chunk - 1u) / hv.chunk;
+                        const unsigned long long at = atomicAdd(&fs->heavy, (1ull << 40) | parts);
+                        if ((uint32_t) (at >> 40) < hv.cap) {
+                            sh.slot = (uint32_t) (at >> 40);
+                            hv.tiles[sh.slot] = HeavyTile{tile, pass, (uint32_t) at, parts};
+                            hv.done[sh.slot] = 0u;
+                        }
+                    }
+                }
+                __syncthreads();
+                slot = sh.slot;
+            }
+            if (slot != 0xFFFFFFFFu) {
+                for (int n = t; n < NN; n += NT)
+                    hv.sums[(size_t) slot * NN + n] = 0ull;
+                return;
+            }
+            // no slot: this CTA walks the tile, however many records it has
+            carry = true;
+            clear_sums<NN, NT>(smem);
+            walk_tile<TX, TY, TZ, NT, ACC, BUMP>(g, rec_a, rec_b, start, fs, rmax, ps.w[pass], ps.wstride, wscale, o3, sh, smem,
+                                           WALK_ALL, 0u, 0u, true, WALK_OVER);
+        }
+    }
+    __syncthreads();
+    write_tile<TX, TY, TZ, NT, ACC>(g, o3, sh, smem, nullptr, carry, winv, ps.out[pass], ps.ostride[pass],
+                                    pass == 0 ? tiles + tile : nullptr);
+}
+
+// The queued parts of crowded tiles: returns at once when there are none.
+template<int TX, int TY, int TZ, int NT, int ACC, bool BUMP>
+__global__ void __launch_bounds__(NT, GATHER_RES / NT) gather_heavy_kernel(const __grid_constant__ GridGeo g,
+    const float4* __restrict__ rec_a, const int4* __restrict__ rec_b, const uint32_t* __restrict__ start,
+    const __grid_constant__ GatherPasses ps, TileStats* __restrict__ tiles, FrameScalars* __restrict__ fs, int rmax,
+    const GatherHeavy hv, uint32_t tiles_x, uint32_t tiles_y) {
+    constexpr int NN = TX * TY * TZ;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ GatherShared<TX, TY, TZ, NT> sh;
+    const int t = threadIdx.x;
+    const unsigned long long queued = fs->heavy;
+    const uint32_t items = (uint32_t) queued, ntiles = min((uint32_t) (queued >> 40), hv.cap);
+    if (items == 0u || ntiles == 0u)
+        return;
+    float wscale = 1.0f, winv = 1.0f;
+    if (ACC == ACC_FIXED_W)
+        weight_scale(fs, wscale, winv);
+    for (uint32_t it = blockIdx.x; it < items; it += gridDim.x) {
+        uint32_t lo = 0, hi = ntiles;  // the last tile whose first part is at or before `it`
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (hv.tiles[mid].first <= it)
+                lo = mid;
+            else
+                hi = mid;
+        }
+        const HeavyTile ht = hv.tiles[lo];
+        if (it < ht.first || it - ht.first >= ht.parts)
+            continue;  // parts of a tile that found the queue full
+        const uint32_t part = it - ht.first;
+        const uint32_t bx = ht.tile % tiles_x, by = (ht.tile / tiles_x) % tiles_y, bz = ht.tile / (tiles_x * tiles_y);
+        const int o3[3] = {(int) bx * TX, (int) by * TY, (int) (bz + g.zlo / TZ) * TZ};
+        __syncthreads();  // the previous item's sums and flags are read
+        clear_sums<NN, NT>(smem);
+        if (t < 3) {
+            const int T3[3] = {TX, TY, TZ};
+            tile_extent(g, fs, o3, T3, t, sh.ex);
+        }
+        __syncthreads();
+        walk_tile<TX, TY, TZ, NT, ACC, BUMP>(g, rec_a, rec_b, start, fs, rmax, ps.w[ht.pass], ps.wstride, wscale, o3, sh, smem,
+                                       WALK_PART, part * hv.chunk, part * hv.chunk + hv.chunk, false, WALK_OVER);
+        __syncthreads();
+        unsigned long long* sums = hv.sums + (size_t) lo * NN;
+        for (int n = 4 * t; n < NN; n += 4 * NT) {
+            unsigned long long q[4];
+            node_sums<NN, ACC>(smem, n, false, q);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if (q[e] == 0ull)
+                    continue;
+                if (ACC == ACC_DOUBLE)
+                    atomicAdd(reinterpret_cast<double*>(sums) + n + e, __longlong_as_double((long long) q[e]));
+                else
+                    atomicAdd(sums + n + e, q[e]);
+            }
+        }
+        __threadfence();  // this part's sums before its count
+        __syncthreads();
+        if (t == 0)
+            sh.slot = atomicAdd(hv.done + lo, 1u);
+        __syncthreads();
+        if (sh.slot == ht.parts - 1u) {  // every part has added its sums
+            __threadfence();
+            write_tile<TX, TY, TZ, NT, ACC>(g, o3, sh, smem, sums, false, winv, ps.out[ht.pass], ps.ostride[ht.pass],
+                                            ht.pass == 0 ? tiles + ht.tile : nullptr);
+        }
     }
 }
 
@@ -913,8 +1155,10 @@ __global__ void __launch_bounds__(256) normalize_kernel(float* __restrict__ grid
 }  // namespace
 
 size_t gather_smem_bytes(const GatherConfig& c) {
-    if (c.mode == GATHER_EXACT)
-        return (size_t) c.tx * c.ty * c.tz * sizeof(unsigned long long) + (size_t) (2 * c.rmax + 1) * sizeof(uint32_t);
+    if (c.mode == GATHER_EXACT) {  // 64-bit sums, 32 bytes per thread of staged particles, the row table
+        const size_t nt = c.tx == 32 ? 512 : 256;
+        return (size_t) c.tx * c.ty * c.tz * sizeof(unsigned long long) + nt * 32 + (size_t) (2 * c.rmax + 1) * sizeof(uint32_t);
+    }
     return (size_t) 2 * c.tx * c.ty * c.tz * sizeof(float) + (size_t) c.smax * (sizeof(float4) + sizeof(uint4)) +
            (size_t) (2 * c.rmax + 1) * sizeof(uint32_t);
 }
@@ -928,48 +1172,77 @@ uint32_t gather_tile_count(const GatherConfig& c, const GridGeo& g) {
     return ceil_div(g.s[0], c.tx) * ceil_div(g.s[1], c.ty) * gather_tiles_z(c, g);
 }
 
+GatherHeavy gather_heavy_plan(const GatherConfig& c, uint32_t n, int sms, size_t* bytes) {
+    GatherHeavy h{};
+    *bytes = 0;
+    h.chunk = std::max<uint32_t>(2048u, std::min<uint32_t>(SPLIT_MAX_RECORDS / 2, n / (uint32_t) (sms * 8)));
+    h.limit = 2 * h.chunk;
+    if (c.mode != GATHER_EXACT || n <= SPLIT_MAX_RECORDS) {
+        h.limit = SPLIT_MAX_RECORDS;
+        return h;
+    }
+    h.cap = (uint32_t) std::min<uint64_t>(2048, 4ull * n / h.limit + 16);
+    *bytes = (size_t) h.cap * ((size_t) c.tx * c.ty * c.tz * sizeof(unsigned long long) + sizeof(HeavyTile) + sizeof(uint32_t));
+    return h;
+}
+
 namespace {
-template<class K>
-cudaError_t launch_tiles(K kern, const GatherConfig& c, const GridGeo& g, int nt, size_t smem, cudaStream_t st,
-    const float4* rec_a, const int4* rec_b, const uint32_t* start, float* grid, TileStats* tiles, FrameScalars* fs,
-    const GatherWeights& w) {
+template<int TX, int TY, int TZ, int NT, int ACC, bool BUMP>
+cudaError_t launch_tiles(const GatherConfig& c, const GridGeo& g, size_t smem, cudaStream_t st, const float4* rec_a,
+    const int4* rec_b, const uint32_t* start, const GatherPasses& ps, TileStats* tiles, FrameScalars* fs, GatherHeavy hv,
+    void* hbuf, int sms) {
+    auto kern = gather_fixed_kernel<TX, TY, TZ, NT, ACC, BUMP>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
     if (e != cudaSuccess)
         return e;
-    dim3 grd(ceil_div(g.s[0], c.tx), ceil_div(g.s[1], c.ty), gather_tiles_z(c, g));
-    kern<<<grd, nt, smem, st>>>(g, rec_a, rec_b, start, grid, tiles, fs, c.rmax, w.w, w.wstride,
-                                w.ostride > 0 ? w.ostride : 1);
+    if (hv.cap) {
+        hv.sums = static_cast<unsigned long long*>(hbuf);
+        hv.tiles = reinterpret_cast<HeavyTile*>(hv.sums + (size_t) hv.cap * TX * TY * TZ);
+        hv.done = reinterpret_cast<uint32_t*>(hv.tiles + hv.cap);
+    }
+    const uint32_t gx = ceil_div(g.s[0], TX), gy = ceil_div(g.s[1], TY), gz = gather_tiles_z(c, g);
+    kern<<<dim3(gx, gy, gz * (uint32_t) ps.count), NT, smem, st>>>(g, rec_a, rec_b, start, ps, tiles, fs, c.rmax, hv, gz);
+    if (hv.cap) {
+        auto heavy = gather_heavy_kernel<TX, TY, TZ, NT, ACC, BUMP>;
+        if ((e = cudaFuncSetAttribute(heavy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) != cudaSuccess)
+            return e;
+        heavy<<<sms * (GATHER_RES / NT), NT, smem, st>>>(g, rec_a, rec_b, start, ps, tiles, fs, c.rmax, hv, gx, gy);
+    }
     return cudaGetLastError();
 }
 
-template<int W>
+template<int ACC, bool BUMP>
 cudaError_t launch_exact(const GatherConfig& c, const GridGeo& g, size_t smem, cudaStream_t st, const float4* rec_a,
-    const int4* rec_b, const uint32_t* start, float* grid, TileStats* tiles, FrameScalars* fs,
-    const GatherWeights& w) {
+    const int4* rec_b, const uint32_t* start, const GatherPasses& ps, TileStats* tiles, FrameScalars* fs,
+    const GatherHeavy& hv, void* hbuf, int sms) {
     if (c.tx == 16 && c.ty == 16 && c.tz == 16)
-        return launch_tiles(gather_fixed_kernel<16, 16, 16, 256, W>, c, g, 256, smem, st, rec_a, rec_b, start, grid,
-                            tiles, fs, w);
+        return launch_tiles<16, 16, 16, 256, ACC, BUMP>(c, g, smem, st, rec_a, rec_b, start, ps, tiles, fs, hv, hbuf, sms);
     if (c.tx == 16 && c.ty == 8 && c.tz == 8)
-        return launch_tiles(gather_fixed_kernel<16, 8, 8, 256, W>, c, g, 256, smem, st, rec_a, rec_b, start, grid,
-                            tiles, fs, w);
+        return launch_tiles<16, 8, 8, 256, ACC, BUMP>(c, g, smem, st, rec_a, rec_b, start, ps, tiles, fs, hv, hbuf, sms);
     if (c.tx == 32 && c.ty == 16 && c.tz == 8)
-        return launch_tiles(gather_fixed_kernel<32, 16, 8, 512, W>, c, g, 512, smem, st, rec_a, rec_b, start, grid,
-                            tiles, fs, w);
+        return launch_tiles<32, 16, 8, 512, ACC, BUMP>(c, g, smem, st, rec_a, rec_b, start, ps, tiles, fs, hv, hbuf, sms);
     return cudaErrorInvalidValue;
 }
 }  // namespace
 
 cudaError_t launch_gather(const GatherConfig& c, const GridGeo& g, const float4* rec_a, const int4* rec_b,
-    const uint32_t* start, float* grid, TileStats* tiles, FrameScalars* fs, cudaStream_t st, const GatherWeights& w) {
+    const uint32_t* start, const GatherPasses& ps, TileStats* tiles, FrameScalars* fs, const GatherHeavy& hv, void* hbuf,
+    int sms, cudaStream_t st) {
     const size_t smem = gather_smem_bytes(c);
     if (c.mode == GATHER_EXACT) {
-        if (w.mode == GatherWeights::DOUBLE)
-            return launch_exact<ACC_DOUBLE>(c, g, smem, st, rec_a, rec_b, start, grid, tiles, fs, w);
-        if (w.mode == GatherWeights::FIXED)
-            return launch_exact<ACC_FIXED_W>(c, g, smem, st, rec_a, rec_b, start, grid, tiles, fs, w);
-        return launch_exact<ACC_EXACT>(c, g, smem, st, rec_a, rec_b, start, grid, tiles, fs, w);
+        const bool bump = g.kernel == 0;
+        auto run = [&](auto acc) {
+            constexpr int ACC = decltype(acc)::value;
+            return bump ? launch_exact<ACC, true>(c, g, smem, st, rec_a, rec_b, start, ps, tiles, fs, hv, hbuf, sms)
+                        : launch_exact<ACC, false>(c, g, smem, st, rec_a, rec_b, start, ps, tiles, fs, hv, hbuf, sms);
+        };
+        if (ps.mode == GatherPasses::DOUBLE)
+            return run(std::integral_constant<int, ACC_DOUBLE>{});
+        if (ps.mode == GatherPasses::FIXED)
+            return run(std::integral_constant<int, ACC_FIXED_W>{});
+        return run(std::integral_constant<int, ACC_EXACT>{});
     }
-    if (w.mode != GatherWeights::DENSITY)
+    if (ps.mode != GatherPasses::DENSITY)
         return cudaErrorInvalidValue;  // the weighted aggregators use the particle-major gather
     if (c.tx != GATHER_TX || c.ty != GATHER_TY || c.tz != GATHER_TZ)
         return cudaErrorInvalidValue;
@@ -978,7 +1251,7 @@ cudaError_t launch_gather(const GatherConfig& c, const GridGeo& g, const float4*
     if (e != cudaSuccess)
         return e;
     dim3 grd(ceil_div(g.s[0], c.tx), ceil_div(g.s[1], c.ty), gather_tiles_z(c, g));
-    kern<<<grd, c.ty * c.tz, smem, st>>>(g, rec_a, rec_b, start, grid, tiles, fs, c.smax, c.rmax);
+    kern<<<grd, c.ty * c.tz, smem, st>>>(g, rec_a, rec_b, start, ps.out[0], tiles, fs, c.smax, c.rmax);
     return cudaGetLastError();
 }
 

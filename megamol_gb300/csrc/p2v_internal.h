@@ -80,16 +80,30 @@ struct GatherConfig {
     int rmax;              // row-table entries per plane chunk
 };
 
-// Accumulation and per-particle weights of one gather pass: DENSITY (exact fixed point), FIXED (the
-// intensity aggregator: weights w[j * wstride] in sorted order, signed fixed point), DOUBLE (the vector
-// aggregator: FP64 sums of weights w, or of the plain kernel values when w == nullptr). The output grid is
-// written with stride ostride (3 for one component of a vector volume).
-struct GatherWeights {
+// The gather's passes over the particles, in one launch: DENSITY (exact fixed point), FIXED (the intensity aggregator:
+// weights w[j * wstride] in sorted order, signed fixed point), DOUBLE (the vector aggregator: FP64 sums of weights w, or
+// of the plain kernel values where w == nullptr). A pass writes its grid `out` with stride ostride (3 for one component
+// of a vector volume); the tile statistics are the first pass'.
+struct GatherPasses {
     enum Mode { DENSITY = 0, FIXED = 1, DOUBLE = 2 };
     int mode = DENSITY;
-    const float* w = nullptr;
+    int count = 1;
     int wstride = 1;
-    int ostride = 1;
+    const float* w[4] = {};
+    float* out[4] = {};
+    int ostride[4] = {1, 1, 1, 1};
+};
+
+// The exact gather's crowded tiles: a tile with more than `limit` records is queued in parts of `chunk` records (cap
+// queue entries, each with a slot of 64-bit node sums and a count of its finished parts).
+struct HeavyTile {
+    uint32_t tile, pass, first, parts;
+};
+struct GatherHeavy {
+    unsigned long long* sums;
+    HeavyTile* tiles;
+    uint32_t* done;
+    uint32_t cap, chunk, limit;
 };
 
 // Per-particle weight source of one list for the intensity (nc = 1: first colour channel) or vector
@@ -129,9 +143,11 @@ cudaError_t launch_vector_grid(const uint32_t* order, const float* dens, const f
                                int sms, cudaStream_t st);
 
 size_t gather_smem_bytes(const GatherConfig& c);
+// The crowded-tile plan of a frame of n particles; bytes: the buffer launch_gather takes for it (0: none)
+GatherHeavy gather_heavy_plan(const GatherConfig& c, uint32_t n, int sms, size_t* bytes);
 cudaError_t launch_gather(const GatherConfig& c, const GridGeo& g, const float4* rec_a, const int4* rec_b,
-    const uint32_t* start, float* grid, TileStats* tiles, FrameScalars* fs, cudaStream_t st,
-    const GatherWeights& w = GatherWeights{});
+    const uint32_t* start, const GatherPasses& ps, TileStats* tiles, FrameScalars* fs, const GatherHeavy& hv, void* hbuf,
+    int sms, cudaStream_t st);
 uint32_t gather_tile_count(const GatherConfig& c, const GridGeo& g);
 // Reduce the tile statistics (fixed order, FP64 sum) and derive the normalisation of the grid.
 cudaError_t launch_finalize(const TileStats* tiles, uint32_t ntiles, FrameScalars* fs, int mass_normalize,

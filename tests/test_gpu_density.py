@@ -234,3 +234,42 @@ def test_particles_whose_support_misses_every_node(ctx, cyclic):
     assert np.array_equal(flagged.view(np.uint32), plain.view(np.uint32))
     v64 = oracle.density_f64(x, bbox, res, cyclic, 1.0, oracle.BUMP, NT)
     assert maxrel(flagged, v64) <= 1e-6
+
+
+def crowd(n, edge, spread, radius, seed):
+    """Half the particles in a Gaussian crowd at the box centre, half uniform; radii around `radius`."""
+    rng = np.random.default_rng(seed)
+    p = rng.uniform(0.0, edge, (n, 3))
+    p[::2] = edge / 2 + rng.normal(0.0, spread, ((n + 1) // 2, 3))
+    return np.column_stack([np.clip(p, 0.0, edge), rng.uniform(0.8, 1.2, n) * radius]).astype(np.float32)
+
+
+# n, box edge, crowd spread, radius, resolution: a tile one CTA may just walk alone and the next size, which queues its
+# parts; many parts; more crowded tiles than the queue holds; more records than one CTA's sums take, without a queue
+CROWDS = [(2 * 32_768, 24.0, 0.2, 0.9, 25), (2 * 32_768 + 2, 24.0, 0.2, 0.9, 25), (300_000, 48.0, 1.5, 0.9, 49),
+          (40_000, 64.0, 20.0, 8.0, 65), (20_000, 15.0, 3.0, 5.0, 16)]
+
+
+@pytest.mark.parametrize("kernel", [p2v.KERNEL_BUMP, p2v.KERNEL_GAUSS3])
+@pytest.mark.parametrize("n,edge,spread,radius,res", CROWDS)
+def test_crowded_tiles(ctx, n, edge, spread, radius, res, kernel):
+    """Tiles with tens of thousands of records: the FP64 bar, and the same bits for a shuffled frame. The 3-sigma
+    Gaussian's support is three times the bump's: a third of the radius."""
+    x = crowd(n, edge, spread, radius / (3 if kernel == p2v.KERNEL_GAUSS3 else 1), n)
+    bbox, r = (0, 0, 0, edge, edge, edge), (res, res, res)
+    vol, _ = run(ctx, [p2v.ParticleList(x)], bbox, r, kernel=kernel)
+    ref = oracle.density_f64(x, bbox, r, (1, 1, 1), 1.0, oracle.GAUSS3 if kernel else oracle.BUMP, NT)
+    assert maxrel(vol, ref) <= 1e-6, maxrel(vol, ref)
+    again, _ = run(ctx, [p2v.ParticleList(x[np.random.default_rng(1).permutation(n)])], bbox, r, kernel=kernel)
+    assert np.array_equal(vol, again)
+
+
+@pytest.mark.parametrize("tile", [(16, 8, 8), (32, 16, 8)])
+def test_crowded_tiles_of_other_shapes(ctx, tile):
+    x = crowd(300_000, 48.0, 1.5, 0.9, 9)
+    bbox, r = (0, 0, 0, 48.0, 48.0, 48.0), (49, 50, 47)
+    ctx.set_params(tile_x=tile[0], tile_y=tile[1], tile_z=tile[2])
+    vol, _ = run(ctx, [p2v.ParticleList(x)], bbox, r)
+    ctx.set_params(tile_x=0, tile_y=0, tile_z=0)
+    ref = oracle.density_f64(x, bbox, r, (1, 1, 1), 1.0, oracle.BUMP, NT)
+    assert maxrel(vol, ref) <= 1e-6, maxrel(vol, ref)
