@@ -510,64 +510,21 @@ __global__ void __launch_bounds__(256) sort_sanitize_kernel(uint32_t* __restrict
     }
 }
 
-// start[c] = first sorted position whose key is >= c, for c in [0, nbins]. Boundary i of the sorted keys
-// (between keys[i-1] and keys[i]) starts the cells (keys[i-1], keys[i]]. boundary_starts_kernel<G> writes
-// the start of every G-th cell there: out[b] = start[G b] for the b whose cell G b lies in that range; a run
-// of more than RUN (64 cells, 32 blocks) is queued in chunks of at most GAP_CHUNK for cell_gap_fill_kernel
-// (a sparse grid holds runs of millions of empty cells). Runs are disjoint and longer than RUN, so the
-// chunks number at most (nbins / G + 1) (1/GAP_CHUNK + 1/(RUN + 1)), below the nbins / 64 + 2 entries the
-// list holds. Dense frames (fewer than 8 cells per particle) take G = 1: the table directly. Sparse frames
-// take G = CELL_BLOCK, then cell_starts_kernel: every cell searches the keys of its block, which lie in
-// [out[b], out[b+1]) (up to n for the last block), and its thread stores start[c] (coalesced; per-boundary
-// threads would write gaps of tens of cells each, one scattered sector per store).
+// start[c] = first sorted position whose key is >= c, for c in [0, nbins]. Boundary i of the sorted keys (between
+// keys[i-1] and keys[i]) starts the run of cells (keys[i-1], keys[i]]. A warp takes 32 consecutive boundaries, scans the
+// lengths of their runs, and its lanes write the cells of all 32 runs together (consecutive lanes, consecutive cells:
+// coalesced however long the runs are; each lane finds the boundary owning its cell by a binary search over the scanned
+// lengths). A run of more than RUN_MAX cells (a sparse grid holds runs of millions of empty cells) is queued in chunks of
+// at most GAP_CHUNK for cell_gap_fill_kernel. Such runs are disjoint, so the chunks number at most (nbins + 1)
+// (1 / GAP_CHUNK + 1 / (RUN_MAX + 1)), below the nbins / 64 + 2 entries the list holds.
+// Bound by its stores: uniform 16M (338 M cells, runs of 21) 0.39 ms; a search per cell in a table of every 64th cell's
+// start, as sparse frames took before, 1.39 ms.
 constexpr uint32_t GAP_CHUNK = 8192;
-constexpr uint32_t CELL_BLOCK = 64;
+constexpr uint32_t RUN_MAX = 8192;
 
-template<uint32_t G>
 __global__ void __launch_bounds__(256) boundary_starts_kernel(const uint32_t* __restrict__ keys, uint32_t n,
     uint32_t nbins, uint32_t* __restrict__ out, uint4* __restrict__ gaps, uint32_t gap_cap,
     FrameScalars* __restrict__ fs, const FrameScalars* __restrict__ gate) {
-    constexpr uint32_t RUN = G == 1 ? 64u : 32u;
-    if (radix_skipped(gate))
-        return;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += gridDim.x * blockDim.x) {
-        const uint32_t lo = i == 0 ? 0u : keys[i - 1] + 1u;
-        uint32_t hi = i == n ? nbins : keys[i];
-        if (hi > nbins)
-            hi = nbins;
-        if (lo > hi)
-            continue;
-        const uint32_t b0 = (uint32_t) (((uint64_t) lo + G - 1) / G), b1 = hi / G;
-        if (b0 > b1)
-            continue;
-        if (b1 - b0 < RUN) {
-            for (uint32_t bb = b0; bb <= b1; ++bb)
-                out[bb] = i;
-        } else {
-            const uint32_t nch = (uint32_t) (((uint64_t) b1 - b0 + GAP_CHUNK) / GAP_CHUNK);
-            const uint32_t slot = atomicAdd(&fs->ngaps, nch);
-            for (uint32_t q = 0; q < nch; ++q) {
-                const uint64_t c0 = (uint64_t) b0 + (uint64_t) q * GAP_CHUNK;
-                const uint64_t c1 = std::min<uint64_t>(b1, c0 + GAP_CHUNK - 1);
-                if ((uint64_t) slot + q < gap_cap)
-                    gaps[slot + q] = make_uint4((uint32_t) c0, (uint32_t) c1, i, 0u);
-                else
-                    atomicOr(&fs->error, ERR_GAP_OVERFLOW);
-            }
-        }
-    }
-}
-
-// The dense table (G = 1) with coalesced stores: a warp takes 32 consecutive boundaries, scans the lengths of
-// their runs of up to RUN cells, and its lanes then write the cells of all 32 runs together (consecutive lanes,
-// consecutive cells; each lane finds the boundary owning its cell by a binary search over the scanned lengths).
-// Longer runs go to the gap list as in boundary_starts_kernel. Per-thread run loops stored one scattered
-// sector per cell and lane; the cells a boundary owns get longer when particles whose support holds no node
-// are sorted behind the others.
-__global__ void __launch_bounds__(256) boundary_starts_dense_kernel(const uint32_t* __restrict__ keys, uint32_t n,
-    uint32_t nbins, uint32_t* __restrict__ out, uint4* __restrict__ gaps, uint32_t gap_cap,
-    FrameScalars* __restrict__ fs, const FrameScalars* __restrict__ gate) {
-    constexpr uint32_t RUN = 64u;
     if (radix_skipped(gate))
         return;
     const uint32_t lane = lane_id();
@@ -583,7 +540,7 @@ __global__ void __launch_bounds__(256) boundary_starts_dense_kernel(const uint32
                 hi = nbins;
         }
         uint32_t len = lo <= hi ? hi - lo + 1u : 0u;
-        if (len > RUN) {
+        if (len > RUN_MAX) {
             const uint32_t i = (uint32_t) i64;
             const uint32_t nch = (uint32_t) (((uint64_t) len - 1 + GAP_CHUNK) / GAP_CHUNK);
             const uint32_t slot = atomicAdd(&fs->ngaps, nch);
@@ -624,26 +581,6 @@ __global__ void __launch_bounds__(256) boundary_starts_dense_kernel(const uint32
                 out[olo + (j - opre)] = (uint32_t) (base + ow);
         }
     }
-}
-
-__global__ void __launch_bounds__(256) cell_starts_kernel(const uint32_t* __restrict__ keys, uint32_t n,
-    uint32_t nbins, const uint32_t* __restrict__ bstart, uint32_t nblk, uint32_t* __restrict__ start,
-    const FrameScalars* __restrict__ gate) {
-    if (radix_skipped(gate))
-        return;
-    const uint64_t c = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x;
-    if (c > nbins)
-        return;
-    const uint32_t b = (uint32_t) (c / CELL_BLOCK);
-    uint32_t lo = bstart[b], hi = b + 1 < nblk ? bstart[b + 1] : n;
-    while (lo < hi) {
-        const uint32_t mid = lo + ((hi - lo) >> 1);
-        if ((uint64_t) keys[mid] < c)
-            lo = mid + 1;
-        else
-            hi = mid;
-    }
-    start[c] = lo;
 }
 
 __global__ void __launch_bounds__(256) cell_gap_fill_kernel(const uint4* __restrict__ gaps, uint32_t gap_cap,
@@ -1042,12 +979,8 @@ size_t bin_scan_words(uint32_t nbins) {
     return (size_t) ceil_div(nbins + 1, SCAN_TILE);
 }
 
-uint32_t cell_block_count(uint32_t nbins) {
-    return (uint32_t) (((uint64_t) nbins + CELL_BLOCK) / CELL_BLOCK);  // blocks of cells 0 .. nbins
-}
-
 cudaError_t launch_bin_sort(SortBuffers& b, uint32_t n, const GridGeo& g, uint32_t* counts, uint32_t* start,
-                            uint32_t* bstart, uint4* gaps, uint32_t gap_cap, FrameScalars* fs, int sms,
+                            uint4* gaps, uint32_t gap_cap, FrameScalars* fs, int sms,
                             cudaStream_t st) {
     const uint32_t nb = g.nbins + 1;
     cudaError_t e;
@@ -1080,18 +1013,8 @@ cudaError_t launch_bin_sort(SortBuffers& b, uint32_t n, const GridGeo& g, uint32
     const unsigned grid = (unsigned) std::max<uint32_t>(1u, std::min<uint32_t>(ceil_div(n + 1, 256), sms * 8));
     if (n > 0)
         sort_sanitize_kernel<<<grid, 256, 0, st>>>(b.keys[b.result], b.vals[b.result], n, g.nbins, b.err, gate);
-    if ((uint64_t) g.nbins < 8ull * n) {
-        boundary_starts_dense_kernel<<<grid, 256, 0, st>>>(b.keys[b.result], n, g.nbins, start, gaps, gap_cap, fs, gate);
-        cell_gap_fill_kernel<<<sms * 2, 256, 0, st>>>(gaps, gap_cap, start, fs, gate);
-    } else {
-        const uint32_t nblk = cell_block_count(g.nbins);
-        boundary_starts_kernel<CELL_BLOCK><<<grid, 256, 0, st>>>(b.keys[b.result], n, g.nbins, bstart, gaps, gap_cap,
-                                                                 fs, gate);
-        cell_gap_fill_kernel<<<sms * 2, 256, 0, st>>>(gaps, gap_cap, bstart, fs, gate);
-        cell_starts_kernel<<<(unsigned) (((uint64_t) g.nbins + 256) / 256), 256, 0, st>>>(b.keys[b.result], n,
-                                                                                          g.nbins, bstart, nblk, start,
-                                                                                          gate);
-    }
+    boundary_starts_kernel<<<grid, 256, 0, st>>>(b.keys[b.result], n, g.nbins, start, gaps, gap_cap, fs, gate);
+    cell_gap_fill_kernel<<<sms * 2, 256, 0, st>>>(gaps, gap_cap, start, fs, gate);
     count_valid_kernel<<<1, 1, 0, st>>>(start, g.nbins, fs);
     return cudaGetLastError();
 }

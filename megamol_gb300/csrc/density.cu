@@ -520,7 +520,6 @@ __device__ __forceinline__ uint32_t locate_record(const uint32_t* row_off, const
 // same result in any order. fs->heavy counts tiles (from bit 40) and parts; a full queue leaves the tile to its own CTA.
 template<int TX, int TY, int TZ, int NT>
 struct GatherShared {
-    static constexpr int NN = TX * TY * TZ;
     double dsum[NT / 32];
     unsigned long long isum[NT / 32], fsum[NT / 32];
     float fmin[NT / 32], fmax[NT / 32];

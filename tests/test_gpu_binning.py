@@ -166,3 +166,16 @@ def test_lookback_wait_runs_out_and_the_context_survives(ctx, with_ao):
     assert np.array_equal(before[0], after[0])
     assert np.array_equal(before[1], after[1], equal_nan=True)
     ctx.set_params(ao_mode=p2v.AO_NONE, ao_normals=p2v.NORMALS_LIST)
+
+
+@pytest.mark.parametrize("run", [64, 65, 8191, 8192, 8193])
+def test_runs_of_empty_cells_around_the_chunk_size(ctx, run):
+    """Two particles whose cells lie exactly `run` apart in the key order (162 cells per row): the longest run a warp
+    writes by itself, the shortest that is queued, and their neighbours."""
+    h = 100.0 / 159.0
+    x = np.full((2, 4), 0.5, np.float32)
+    x[0, :3] = (5.5 * h, 20.5 * h, 30.5 * h)
+    x[1, :3] = ((5.5 + run % 162) * h, (20.5 + run // 162) * h, 30.5 * h)
+    assert check(ctx, x, (0.0, 0.0, 0.0, 100.0, 100.0, 100.0), (160, 160, 160)) == 0
+    keys, _, _ = ctx.binning()
+    assert int(keys[1]) - int(keys[0]) == run
