@@ -25,32 +25,89 @@ namespace {
 // ---------------------------------------------------------------------------------------------
 // mip pyramid: level l+1 voxel = sum of the children 2g .. min(2g+1, N-1), divided by 8 always
 // ---------------------------------------------------------------------------------------------
-// One thread per voxel of the coarser level in 32-bit index arithmetic (an AO volume holds fewer than 2^31
-// texels, so every level above level 0 fewer than 2^28).
-// pairs: the finer level's rows have an even length and start 8-byte aligned, so the two children of a voxel
-// along x load as one float2 (the same values added in the same order as mip_voxel's loop: the same bits).
-__global__ void __launch_bounds__(256) mip_level_kernel(const float* __restrict__ src, int sx, int sy, int sz,
-    float* __restrict__ dst, int dx, int dy, int dz, float sat_scale, int quantize, int pairs) {
+// R8 levels (mip_voxel's integer rule): one thread per voxel of the coarser level in 32-bit index arithmetic (an AO
+// volume holds fewer than 2^31 texels, so every level above level 0 fewer than 2^28).
+__global__ void __launch_bounds__(256) mip_level_r8_kernel(const float* __restrict__ src, int sx, int sy, int sz,
+    float* __restrict__ dst, int dx, int dy, int dz, float sat_scale) {
     const uint32_t n = (uint32_t) dx * (uint32_t) dy * (uint32_t) dz;
     const uint32_t pxy = (uint32_t) dx * (uint32_t) dy;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t z = i / pxy, r = i - z * pxy;
         const uint32_t y = r / (uint32_t) dx, x = r - y * (uint32_t) dx;
-        if (pairs && !quantize) {
-            const int y1 = min(2 * (int) y + 1, sy - 1), z1 = min(2 * (int) z + 1, sz - 1);
-            float acc = 0.0f;
-            for (int zz = 2 * (int) z; zz <= z1; ++zz)
-                for (int yy = 2 * (int) y; yy <= y1; ++yy) {
-                    float2 v = __ldg(reinterpret_cast<const float2*>(src + ((int64_t) zz * sy + yy) * sx + 2 * x));
-                    if (sat_scale > 0.0f) {
-                        v.x = fminf(fmaxf(__fmul_rn(v.x, sat_scale), 0.0f), 1.0f);
-                        v.y = fminf(fmaxf(__fmul_rn(v.y, sat_scale), 0.0f), 1.0f);
+        dst[i] = mip_voxel<true>(src, sx, sy, sz, (int) x, (int) y, (int) z, sat_scale, 1);
+    }
+}
+
+// One level from the finer one, and with NORMALIZE the finer level's own min-max / mass normalisation in the same pass
+// (grid values are normalised in place, then averaged: the level is read once instead of twice).
+// A warp takes the 2 x 2 rows above one row of coarser voxels, 32 x at a time, whatever the row length and its alignment
+// are: four coalesced loads per lane, the odd lanes' values by shuffles, the children added in mip_voxel's order (the
+// same bits). Rows, planes and columns past the last coarser voxel (odd sizes) are only normalised.
+// Bound by HBM: mixed 64M (512^3) 0.183 ms with the normalisation, 1.2 GB at 6.6 TB/s (the two kernels took 0.165 +
+// 0.146); uniform 16M (695^3, rows of no alignment) 0.48 ms, 6.0 TB/s (0.42 + 0.45). Four segments in flight per warp
+// and 64 registers; two 0.50 ms, one at full occupancy 0.53, one segment per warp and round 0.59 (index arithmetic).
+constexpr int MIP_AHEAD = 4;
+
+template<bool NORMALIZE>
+__global__ void __launch_bounds__(256, 4) mip_rows_kernel(float* __restrict__ src, int sx, int sy, int sz,
+    float* __restrict__ dst, int dx, int dy, int dz, float sat_scale, const FrameScalars* __restrict__ fs,
+    int mass_normalize, int minmax_normalize) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t ny = ((uint32_t) sy + 1u) / 2u, nz = ((uint32_t) sz + 1u) / 2u, total = ny * nz;
+    float ms = 1.0f, off = 0.0f, sc = 1.0f;
+    if (NORMALIZE) {
+        ms = (float) fs->mass_scale;
+        off = fs->offset;
+        sc = fs->scale;
+    }
+    const uint32_t step = gridDim.x * (blockDim.x >> 5);
+    for (uint32_t q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); q < total; q += step) {
+        const uint32_t Z = q / ny, Y = q - Z * ny;
+        // (a level one voxel deep keeps one voxel: its missing neighbours are left out of the sum)
+        const bool y1 = 2 * Y + 1 < (uint32_t) sy, z1 = 2 * Z + 1 < (uint32_t) sz;
+        const bool has[4] = {true, y1, z1, y1 && z1};
+        float* row[4];
+        row[0] = src + ((size_t) (2 * Z) * sy + 2 * Y) * sx + lane;
+        row[1] = row[0] + sx;
+        row[2] = row[0] + (size_t) sy * sx;
+        row[3] = row[2] + sx;
+        float* out = Y < (uint32_t) dy && Z < (uint32_t) dz && (lane & 1) == 0 ? dst + ((size_t) Z * dy + Y) * dx : nullptr;
+        // every lane of the warp stays in the loop for its shuffles
+        for (int x0 = 0; x0 < sx; x0 += 32 * MIP_AHEAD) {
+            float v[MIP_AHEAD][4];
+#pragma unroll
+            for (int u = 0; u < MIP_AHEAD; ++u)
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    v[u][c] = has[c] && x0 + 32 * u + lane < sx ? row[c][x0 + 32 * u] : 0.0f;
+#pragma unroll
+            for (int u = 0; u < MIP_AHEAD; ++u) {
+                const int x = x0 + 32 * u + lane;
+                if (NORMALIZE) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        v[u][c] = normalize_one(v[u][c], ms, off, sc, mass_normalize, minmax_normalize);
+                        if (has[c] && x < sx)
+                            row[c][x0 + 32 * u] = v[u][c];
                     }
-                    acc = __fadd_rn(__fadd_rn(acc, v.x), v.y);
                 }
-            dst[i] = __fmul_rn(acc, 0.125f);
-        } else {
-            dst[i] = mip_voxel<true>(src, sx, sy, sz, (int) x, (int) y, (int) z, sat_scale, quantize);
+                const bool x1 = x + 1 < sx;
+                float acc = 0.0f;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    float a = v[u][c];
+                    if (sat_scale > 0.0f)
+                        a = fminf(fmaxf(__fmul_rn(a, sat_scale), 0.0f), 1.0f);
+                    const float b = __shfl_down_sync(0xffffffffu, a, 1);
+                    if (has[c]) {
+                        acc = __fadd_rn(acc, a);
+                        if (x1)
+                            acc = __fadd_rn(acc, b);
+                    }
+                }
+                if (out && (x >> 1) < dx)
+                    out[x >> 1] = __fmul_rn(acc, 0.125f);
+            }
         }
     }
 }
@@ -438,19 +495,35 @@ cudaError_t launch_brick_order(const BrickPlan& p, const GridGeo& g, const uint3
     return cudaGetLastError();
 }
 
+namespace {
+unsigned mip_rows_grid(const int sd[3], int sms) {
+    const uint64_t warps = (uint64_t) ((sd[1] + 1) / 2) * ((sd[2] + 1) / 2);
+    return (unsigned) std::max<uint64_t>(1, std::min<uint64_t>((warps + 7) / 8, (uint64_t) sms * 32));
+}
+}  // namespace
+
+cudaError_t launch_normalize_mip(float* grid, const int d0[3], const FrameScalars* fs, int mass_normalize,
+    int minmax_normalize, float sat_scale, float* level1, int sms, cudaStream_t st) {
+    mip_rows_kernel<true><<<mip_rows_grid(d0, sms), 256, 0, st>>>(grid, d0[0], d0[1], d0[2], level1, max(1, d0[0] / 2),
+        max(1, d0[1] / 2), max(1, d0[2] / 2), sat_scale, fs, mass_normalize, minmax_normalize);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_mip_levels(const float* l0, const int d0[3], float sat_scale, int quantize, int nlevels,
-    float* const* out, int (*dims)[3], int sms, cudaStream_t st) {
+    float* const* out, int first, int sms, cudaStream_t st) {
     const float* src = l0;
     int sd[3] = {d0[0], d0[1], d0[2]};
     for (int l = 1; l < nlevels; ++l) {
         int dd[3] = {max(1, sd[0] / 2), max(1, sd[1] / 2), max(1, sd[2] / 2)};
-        const int64_t nv = (int64_t) dd[0] * dd[1] * dd[2];
-        const unsigned grd = (unsigned) std::max<int64_t>(1, std::min<int64_t>((nv + 255) / 256, (int64_t) sms * 32));
-        const int pairs = (sd[0] % 2 == 0) && (reinterpret_cast<uintptr_t>(src) % 8 == 0);
-        mip_level_kernel<<<grd, 256, 0, st>>>(src, sd[0], sd[1], sd[2], out[l], dd[0], dd[1], dd[2],
-                                              l == 1 ? sat_scale : 0.0f, quantize, pairs);
-        for (int a = 0; a < 3; ++a)
-            dims[l][a] = dd[a];
+        const float sat = l == 1 ? sat_scale : 0.0f;
+        if (l >= first && quantize) {
+            const int64_t nv = (int64_t) dd[0] * dd[1] * dd[2];
+            const unsigned grd = (unsigned) std::max<int64_t>(1, std::min<int64_t>((nv + 255) / 256, (int64_t) sms * 32));
+            mip_level_r8_kernel<<<grd, 256, 0, st>>>(src, sd[0], sd[1], sd[2], out[l], dd[0], dd[1], dd[2], sat);
+        } else if (l >= first) {
+            mip_rows_kernel<false><<<mip_rows_grid(sd, sms), 256, 0, st>>>(const_cast<float*>(src), sd[0], sd[1], sd[2],
+                out[l], dd[0], dd[1], dd[2], sat, nullptr, 0, 0);
+        }
         src = out[l];
         for (int a = 0; a < 3; ++a)
             sd[a] = dd[a];

@@ -100,9 +100,13 @@ inline size_t batch_queue_words(uint32_t nseg) { return 2 + (size_t) nseg; }
 // zeroes the queue words and runs the queue with one resident block per free slot of every SM
 cudaError_t launch_batch_ao(const BatchQueueArgs& q, int sms, cudaStream_t st);
 
-// quantize = 1: the levels are R8 textures (texels k/255; out = ((sum k + 4) / 8) / 255)
+// Levels `first` .. nlevels - 1 of the pyramid over l0 (the ones below exist). quantize = 1: the levels are R8 textures
+// (texels k/255; out = ((sum k + 4) / 8) / 255)
 cudaError_t launch_mip_levels(const float* l0, const int d0[3], float sat_scale, int quantize, int nlevels,
-    float* const* out, int (*dims)[3], int sms, cudaStream_t st);
+    float* const* out, int first, int sms, cudaStream_t st);
+// the grid's normalisation (fs) and level 1 of its pyramid in one pass
+cudaError_t launch_normalize_mip(float* grid, const int d0[3], const FrameScalars* fs, int mass_normalize,
+    int minmax_normalize, float sat_scale, float* level1, int sms, cudaStream_t st);
 // acc: scratch of 4 (unorm8) or 8 bytes per voxel; vol: level 0 of the MDAO volume (x fastest)
 cudaError_t launch_mdao_volume(const MdaoParams& mp, const uint32_t* order, const float4* xyzr, uint32_t n,
     void* acc, float* vol, int sms, cudaStream_t st);

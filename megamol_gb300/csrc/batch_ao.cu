@@ -10,7 +10,7 @@
 // grid is resident. Each wait is bounded (a poll budget the host sets); when it runs out the block records
 // BATCH_ERR_TIMEOUT, every other block stops at its next ticket or wait, and the host reports P2V_ETIMEOUT.
 //
-// The items compute with the device functions of the per-frame kernels (mip_level_kernel, cone_blocks_kernel,
+// The items compute with the device functions of the per-frame kernels (mip_rows_kernel, cone_blocks_kernel,
 // gradient_normals_kernel): the same operations in the same order, so a frame's AO has the bits it has
 // from p2v_run_frame. Mip levels written by this launch are read with plain (coherent) loads; the density
 // grid, written before the launch, through the read-only path.

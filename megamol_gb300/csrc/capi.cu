@@ -76,6 +76,7 @@ struct Pipe {
     DevBuf cblocks;                        // corner blocks of the plain march's mip levels
     DevBuf bk0, bk1, xyzr_b, nrm_b, ord_b;  // the AO stages' brick order (ao_brick_order)
     bool xyzr_sorted = false;              // the binning of this frame wrote xyzr_s
+    bool mip1_done = false;                // this frame's normalisation built level 1 of the pyramid
     bool timing = false;                   // this frame records stage events
     bool aok = false;                      // EV_AOK0 / EV_AOK1 bracket this frame's main AO kernel
     uint32_t ao_fetches = 0;               // texture fetches per particle of the learned AO's inference
@@ -398,6 +399,9 @@ uint32_t record_bytes(int type) {
     default: return 0;
     }
 }
+
+int density_levels(const p2v_params& P, const int s[3]);
+size_t mip_layout(const int d0[3], int L, int d[MAX_LEVELS][3], size_t off[MAX_LEVELS]);
 
 }  // namespace
 
@@ -810,6 +814,7 @@ p2v_status p2v_ctx::enqueue_frame(Pipe& pp, const p2v_frame* fr, p2v_volume* vol
         P2V_CUDA_TRY(cudaEventRecord(ev[EV_DENSITY], st));
     const double voxel_volume = (double) g.hhi[0] * g.hhi[1] * g.hhi[2];
     const uint32_t* vg_order = nullptr;
+    pp.mip1_done = false;
     if (agg == 2) {
         VectorGridBufs vb{pp.vdens.as<float>(), pp.vdirs.as<float>(), pp.vkeys0.as<uint32_t>(),
                           pp.vvals0.as<uint32_t>()};
@@ -832,7 +837,19 @@ p2v_status p2v_ctx::enqueue_frame(Pipe& pp, const p2v_frame* fr, p2v_volume* vol
     } else if (!ext_grid) {
         P2V_CUDA_TRY(launch_finalize(tiles.as<TileStats>(), ntiles, fs, P.mass_normalize, P.normalize, 0.0, voxel_volume,
                                      st));
-        P2V_CUDA_TRY(launch_normalize_modes(dgrid, V, fs, P.mass_normalize, P.normalize, sms, st));
+        // a cone march over the grid: its pyramid's first level in the same pass
+        const int L = density_levels(P, g.s);
+        if ((P.ao_mode == P2V_AO_CONE || P.ao_mode == P2V_AO_LEARNED) && P.ao_volume == P2V_AOVOL_DENSITY && !slot &&
+            L > 1 && (P.mass_normalize || P.normalize)) {
+            int d[MAX_LEVELS][3];
+            size_t off[MAX_LEVELS];
+            P2V_CUDA_TRY(pp.mips.ensure(sizeof(float) * (mip_layout(g.s, L, d, off) + 1)));
+            P2V_CUDA_TRY(launch_normalize_mip(dgrid, g.s, fs, P.mass_normalize, P.normalize, P.ao_volume_scale,
+                                              pp.mips.as<float>() + off[1], sms, st));
+            pp.mip1_done = true;
+        } else {
+            P2V_CUDA_TRY(launch_normalize_modes(dgrid, V, fs, P.mass_normalize, P.normalize, sms, st));
+        }
     }
     if (timed)
         P2V_CUDA_TRY(cudaEventRecord(ev[EV_NORM], st));
@@ -1020,6 +1037,30 @@ void mdao_dims(const float clip[6], int vol_size, int dims[3], float& shortest, 
     max_lod = std::ceil(std::log2(static_cast<float>(vol_size))) - 1.0f;
 }
 
+namespace {
+// Mip levels of a density grid's pyramid (p2v_params.ao_levels; 0: down to the longest edge's last halving).
+int density_levels(const p2v_params& P, const int s[3]) {
+    const int smax = std::max(s[0], std::max(s[1], s[2]));
+    const int L = P.ao_levels > 0 ? P.ao_levels : (int) std::ceil(std::log2((double) smax));
+    return std::max(1, std::min(L, MAX_LEVELS));
+}
+
+// Sizes and offsets (in floats) of the levels 1 .. L - 1 over a level 0 of size d0, each on a 128-byte boundary; returns
+// the floats they take.
+size_t mip_layout(const int d0[3], int L, int d[MAX_LEVELS][3], size_t off[MAX_LEVELS]) {
+    size_t need = 0;
+    for (int a = 0; a < 3; ++a)
+        d[0][a] = d0[a];
+    for (int l = 1; l < L; ++l) {
+        for (int a = 0; a < 3; ++a)
+            d[l][a] = std::max(1, d[l - 1][a] / 2);
+        off[l] = need;
+        need += ((size_t) d[l][0] * d[l][1] * d[l][2] + 31) & ~size_t(31);
+    }
+    return need;
+}
+}  // namespace
+
 p2v_status p2v_ctx::build_cone(Pipe& pp, const p2v_frame* fr, const GridGeo& g, const float* dgrid,
                                const float bb[6], uint32_t n, const uint32_t* order, ConeParams& cp, cudaStream_t st,
                                BatchSlot* slot) {
@@ -1081,10 +1122,8 @@ p2v_status p2v_ctx::build_cone(Pipe& pp, const p2v_frame* fr, const GridGeo& g, 
     } else {
         for (int a = 0; a < 3; ++a)
             d0[a] = g.s[a];
-        const int smax = std::max(g.s[0], std::max(g.s[1], g.s[2]));
         shortest = (float) std::min(g.s[0], std::min(g.s[1], g.s[2]));
-        L = P.ao_levels > 0 ? P.ao_levels : (int) std::ceil(std::log2((double) smax));
-        L = std::max(1, std::min(L, MAX_LEVELS));
+        L = density_levels(P, d0);
         max_lod = (float) (L - 1);
         // the density grid is node-centred: as a texture it spans [min - h/2, max + h/2]
         for (int a = 0; a < 3; ++a) {
@@ -1107,28 +1146,19 @@ p2v_status p2v_ctx::build_cone(Pipe& pp, const p2v_frame* fr, const GridGeo& g, 
     // the samplers address texels with 32-bit offsets
     if ((uint64_t) d0[0] * d0[1] * d0[2] >= (1ull << 31))
         return fail(P2V_EUNSUPPORTED, "AO volume %dx%dx%d exceeds 2^31 texels", d0[0], d0[1], d0[2]);
-    // level 0 is the density grid (saturated on the fly) or the MDAO volume; levels 1.. are built here
-    // each level starts on a 128-byte boundary
-    size_t need = 0;
+    // level 0 is the density grid (saturated on the fly) or the MDAO volume; levels 1.. are built here (level 1 of a
+    // density grid with its normalisation, earlier)
     int d[MAX_LEVELS][3];
-    for (int a = 0; a < 3; ++a)
-        d[0][a] = d0[a];
-    for (int l = 1; l < L; ++l) {
-        for (int a = 0; a < 3; ++a)
-            d[l][a] = std::max(1, d[l - 1][a] / 2);
-        need += ((size_t) d[l][0] * d[l][1] * d[l][2] + 31) & ~size_t(31);
-    }
+    size_t off[MAX_LEVELS];
+    const size_t need = mip_layout(d0, L, d, off);
     P2V_CUDA_TRY(mips.ensure(sizeof(float) * (need + 1)));
     float* lvp[MAX_LEVELS];
     lvp[0] = const_cast<float*>(level0);
-    size_t off = 0;
-    for (int l = 1; l < L; ++l) {
-        lvp[l] = mips.as<float>() + off;
-        off += ((size_t) d[l][0] * d[l][1] * d[l][2] + 31) & ~size_t(31);
-    }
-    int dims[MAX_LEVELS][3];
+    for (int l = 1; l < L; ++l)
+        lvp[l] = mips.as<float>() + off[l];
     if (!slot)  // a batch frame's levels are built by the batch AO launch
-        P2V_CUDA_TRY(launch_mip_levels(level0, d0, cp.sat, mdao && P.mdao_unorm8 ? 1 : 0, L, lvp, dims, sms, st));
+        P2V_CUDA_TRY(launch_mip_levels(level0, d0, cp.sat, mdao && P.mdao_unorm8 ? 1 : 0, L, lvp,
+                                       !mdao && pp.mip1_done ? 2 : 1, sms, st));
     for (int l = 0; l < L; ++l) {
         cp.lv[l].v = lvp[l];
         for (int a = 0; a < 3; ++a) {

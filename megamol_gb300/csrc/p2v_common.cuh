@@ -54,6 +54,16 @@ struct FrameScalars {
     double mass_scale;
 };
 
+// A grid value's normalisation (FrameScalars' constants).
+__device__ __forceinline__ float normalize_one(float v, float ms, float off, float sc, int mass_normalize,
+                                               int minmax_normalize) {
+    if (mass_normalize)
+        v = v * ms;
+    if (minmax_normalize)
+        v = (v - off) * sc;
+    return v;
+}
+
 // Per-CTA partial statistics of the density tiles.
 struct TileStats {
     double sum;

@@ -237,3 +237,32 @@ def test_block_march_has_the_bits_of_the_texel_march(ctx, n, res, over):
     a, _, _ = run_ao(ctx, f, nrm, ao_march=p2v.AO_MARCH_THREAD, **kw)
     b, _, _ = run_ao(ctx, f, nrm, ao_march=p2v.AO_MARCH_WARP, **kw)
     assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("res", [(2, 2, 2), (3, 2, 5), (31, 33, 32), (64, 7, 9), (65, 66, 67), (130, 5, 129)])
+@pytest.mark.parametrize("norm", [dict(normalize=1), dict(normalize=0, mass_normalize=1), dict(normalize=0)])
+def test_mip_levels_of_odd_sizes(ctx, res, norm):
+    """Grid and pyramid with the first level built by the normalisation pass (and without one), over row lengths around
+    a warp's 32: level l + 1 is the FP32 sum of the children, x fastest, times 1/8, and the grid is the one a frame
+    without AO gives, bit for bit."""
+    f = frame(n=5_000, seed=80)
+    f.res = res
+    L = p2v.ParticleList(f.xyzr, p2v.VERTDATA_FLOAT_XYZR, normals=synth.random_normals(f.n, 81))
+    ao, vol, _ = run_ao(ctx, f, synth.random_normals(f.n, 81), ao_mode=p2v.AO_CONE, ao_levels=4, ao_volume_scale=0.7, **norm)
+    # fmax / fmin: the saturation takes a NaN (the grid of a constant density after min-max normalisation) to 0
+    lv = np.fmin(np.fmax(vol * np.float32(0.7), np.float32(0)), np.float32(1))
+    for l in range(1, 4):
+        d = [max(1, s // 2) for s in lv.shape]
+        acc = np.zeros(d, np.float32)
+        for z in range(2):
+            for y in range(2):
+                for x in range(2):
+                    c = lv[z:, y:, x:][::2, ::2, ::2][:d[0], :d[1], :d[2]]
+                    if min(c.shape) > 0:  # (an axis of one voxel has no second child)
+                        acc = acc + c
+        lv = acc * np.float32(0.125)
+        assert np.array_equal(ctx.ao_volume(l), lv), l
+    ctx.set_params(ao_mode=p2v.AO_NONE)
+    plain = np.empty_like(vol.ravel())
+    ctx.run_frame([L], f.bbox, plain)
+    assert np.array_equal(plain.reshape(vol.shape), vol, equal_nan=True)
