@@ -78,55 +78,87 @@ __device__ __forceinline__ bool support_misses_nodes(const float q[3], float r, 
 // frame-wide maxima and counts cost one atomic per block rather than per 256 particles. empty_flag (a power of
 // two above every cell key, or 0): added to the key of a particle whose support holds no node, so that the
 // sort puts those particles after every other (in cell order) and the cell start table, which the density
-// gather walks, leaves them out.
+// gather walks, leaves them out. counts (nullable; the counting sort): particles per key, keys in [0, nbins] (nbins: the
+// invalid particles); rank then receives each particle's arrival rank in its cell, its slot there until the cells are put
+// in index order (no pass over the keys for it).
+constexpr int PACK_AHEAD = 2;  // (4: mixed 64M 0.43 against 0.39 ms)
+
 template<class T, int NC, bool ALIGNED>
 __global__ void __launch_bounds__(256) pack_keys_kernel(ListDesc L, GridGeo g, float4* __restrict__ xyzr,
-    uint32_t* __restrict__ keys, uint32_t* __restrict__ idx, FrameScalars* __restrict__ fs, uint32_t empty_flag) {
+    uint32_t* __restrict__ keys, uint32_t* __restrict__ counts, uint32_t* __restrict__ rank,
+    FrameScalars* __restrict__ fs, uint32_t empty_flag) {
     __shared__ int32_t s_cmin[3][8], s_cmax[3][8];
     __shared__ uint32_t s_rmax[8], s_drop[8];
     int32_t cell[3] = {INT32_MAX, INT32_MAX, INT32_MAX};
     int32_t cellhi[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
     uint32_t rbits = 0u, drop = 0u;
     const uint64_t step = (uint64_t) gridDim.x * blockDim.x;
-    for (uint64_t i = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; i < L.count; i += step) {
-        const uint8_t* rec = L.data + i * L.stride;
-        const float x = load_comp<T, ALIGNED>(rec);
-        const float y = load_comp<T, ALIGNED>(rec + sizeof(T));
-        const float z = load_comp<T, ALIGNED>(rec + 2 * sizeof(T));
-        const float r = NC == 4 ? load_comp<T, ALIGNED>(rec + 3 * sizeof(T)) : L.global_radius;
-        const float p[3] = {x, y, z};
-        bool valid = isfinite(x) && isfinite(y) && isfinite(z) && isfinite(r) && r > 0.0f;
-        uint32_t bin[3];
-        int32_t c[3];
-        float qa[3];
+    // PACK_AHEAD particles per round: their loads, and the counting additions whose old values are the ranks, are in
+    // flight together
+    for (uint64_t i0 = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; i0 < L.count; i0 += PACK_AHEAD * step) {
+        float4 p[PACK_AHEAD];
+        uint32_t key[PACK_AHEAD];
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const float q = (p[a] - g.minf[a]) / g.hf[a];
-            qa[a] = q;
-            valid = valid && fabsf(q) < 1073741824.0f;
-            c[a] = clamp_cell(q);
-            const int32_t b = c[a] < -1 ? -1 : (c[a] > g.s[a] ? g.s[a] : c[a]);
-            bin[a] = static_cast<uint32_t>(b + 1);
+        for (int u = 0; u < PACK_AHEAD; ++u) {
+            const uint64_t i = i0 + u * step;
+            p[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (i < L.count) {
+                const uint8_t* rec = L.data + i * L.stride;
+                p[u].x = load_comp<T, ALIGNED>(rec);
+                p[u].y = load_comp<T, ALIGNED>(rec + sizeof(T));
+                p[u].z = load_comp<T, ALIGNED>(rec + 2 * sizeof(T));
+                p[u].w = NC == 4 ? load_comp<T, ALIGNED>(rec + 3 * sizeof(T)) : L.global_radius;
+            }
         }
-        uint32_t key = g.nbins;
-        if (valid) {
-            key = (bin[2] * g.nb[1] + bin[1]) * g.nb[0] + bin[0];
+#pragma unroll
+        for (int u = 0; u < PACK_AHEAD; ++u) {
+            const uint64_t i = i0 + u * step;
+            if (i >= L.count)
+                break;
+            const float r = p[u].w;
+            const float pc[3] = {p[u].x, p[u].y, p[u].z};
+            bool valid = isfinite(pc[0]) && isfinite(pc[1]) && isfinite(pc[2]) && isfinite(r) && r > 0.0f;
+            uint32_t bin[3];
+            int32_t c[3];
+            float qa[3];
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
-                cell[a] = min(cell[a], c[a]);
-                cellhi[a] = max(cellhi[a], c[a]);
+                const float q = (pc[a] - g.minf[a]) / g.hf[a];
+                qa[a] = q;
+                valid = valid && fabsf(q) < 1073741824.0f;
+                c[a] = clamp_cell(q);
+                const int32_t b = c[a] < -1 ? -1 : (c[a] > g.s[a] ? g.s[a] : c[a]);
+                bin[a] = static_cast<uint32_t>(b + 1);
             }
-            rbits = max(rbits, __float_as_uint(r));
-            if (empty_flag && support_misses_nodes(qa, r, g))
-                key |= empty_flag;
-        } else {
-            ++drop;
+            key[u] = g.nbins;
+            if (valid) {
+                key[u] = (bin[2] * g.nb[1] + bin[1]) * g.nb[0] + bin[0];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    cell[a] = min(cell[a], c[a]);
+                    cellhi[a] = max(cellhi[a], c[a]);
+                }
+                rbits = max(rbits, __float_as_uint(r));
+                if (empty_flag && support_misses_nodes(qa, r, g))
+                    key[u] |= empty_flag;
+            } else {
+                ++drop;
+            }
+            const uint64_t o = L.offset + i;
+            xyzr[o] = p[u];
+            keys[o] = key[u];
         }
-        const uint64_t o = L.offset + i;
-        xyzr[o] = make_float4(x, y, z, r);
-        keys[o] = key;
-        if (idx)
-            idx[o] = static_cast<uint32_t>(o);
+        if (counts) {
+            uint32_t rk[PACK_AHEAD];
+#pragma unroll
+            for (int u = 0; u < PACK_AHEAD; ++u)
+                if (i0 + u * step < L.count)
+                    rk[u] = atomicAdd(counts + key[u], 1u);
+#pragma unroll
+            for (int u = 0; u < PACK_AHEAD; ++u)
+                if (i0 + u * step < L.count)
+                    rank[L.offset + i0 + u * step] = rk[u];
+        }
     }
     // block reduction: one atomic per block and quantity
 #pragma unroll
@@ -184,7 +216,7 @@ constexpr int SORT_TILE = SORT_THREADS * SORT_ITEMS;  // 4096 keys per tile
 constexpr int MAX_RADIX = 512;
 constexpr int MAX_PASSES = 5;
 constexpr int HIST_WORDS = MAX_PASSES * MAX_RADIX;    // digit histograms, pass p at p * MAX_RADIX
-// after the histograms: one tile counter per radix pass
+// after the histograms: one tile counter per radix pass, and the count of finished histogram blocks
 constexpr int LOOKBACK_WINDOW = 8;  // predecessor tiles a look-back round reads at once (4: 3.55, 16: 3.49 ms)
 constexpr uint32_t FLAG_AGG = 1u << 30;
 constexpr uint32_t FLAG_PRE = 2u << 30;
@@ -227,15 +259,22 @@ __device__ __forceinline__ bool radix_skipped(const FrameScalars* gate) {
     return gate != nullptr && gate->bin_maxcount <= BIN_CELL_MAX;
 }
 
-__global__ void __launch_bounds__(256) radix_hist_kernel(const uint32_t* __restrict__ keys, uint32_t n, SortPlan pl,
-    uint32_t* __restrict__ hist, const FrameScalars* __restrict__ gate) {
-    if (radix_skipped(gate))
+// Digit histograms of every pass over the keys, and (the block that finishes last) their exclusive scans in place: the
+// digits' first destinations. Also clears the passes' look-back words. The first nblk blocks (of 256 threads) take part;
+// `done` counts the finished ones (zero before).
+__device__ __forceinline__ void radix_hist(const uint32_t* __restrict__ keys, uint32_t n, const SortPlan& pl,
+                                           uint32_t* __restrict__ hist, uint32_t* __restrict__ done,
+                                           uint32_t* __restrict__ status, uint64_t status_words, uint32_t nblk) {
+    if (blockIdx.x >= nblk)
         return;
     __shared__ uint32_t sh[HIST_WORDS];
+    __shared__ uint32_t s_last, s_sum[8];
     for (int i = threadIdx.x; i < HIST_WORDS; i += blockDim.x)
         sh[i] = 0;
+    for (uint64_t i = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; i < status_words / 4; i += (uint64_t) nblk * blockDim.x)
+        reinterpret_cast<uint4*>(status)[i] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += nblk * blockDim.x) {
         const uint32_t k = keys[j];
         for (int p = 0; p < pl.passes; ++p)
             atomicAdd(&sh[p * MAX_RADIX + ((k >> pl.shift[p]) & ((1u << pl.bits[p]) - 1u))], 1u);
@@ -244,27 +283,40 @@ __global__ void __launch_bounds__(256) radix_hist_kernel(const uint32_t* __restr
     for (int i = threadIdx.x; i < pl.passes * MAX_RADIX; i += blockDim.x)
         if (sh[i])
             atomicAdd(&hist[i], sh[i]);
-}
-
-// Exclusive scan of each pass' digit histogram (one block of MAX_RADIX threads).
-__global__ void __launch_bounds__(MAX_RADIX) radix_scan_kernel(uint32_t* hist, int passes,
-                                                                const FrameScalars* __restrict__ gate) {
-    if (radix_skipped(gate))
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0)
+        s_last = atomicAdd(done, 1u) == nblk - 1u ? 1u : 0u;
+    __syncthreads();
+    if (!s_last)
         return;
-    __shared__ uint32_t s[MAX_RADIX];
-    for (int p = 0; p < passes; ++p) {
-        const uint32_t v = hist[p * MAX_RADIX + threadIdx.x];
-        s[threadIdx.x] = v;
-        __syncthreads();
-        for (int o = 1; o < MAX_RADIX; o <<= 1) {
-            const uint32_t t = threadIdx.x >= (unsigned) o ? s[threadIdx.x - o] : 0u;
-            __syncthreads();
-            s[threadIdx.x] += t;
-            __syncthreads();
+    __threadfence();
+    const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
+    for (int p = 0; p < pl.passes; ++p) {
+        uint32_t* h = hist + p * MAX_RADIX + 2 * threadIdx.x;  // two digits per thread
+        const uint32_t a = __ldcg(h), b = __ldcg(h + 1);
+        uint32_t incl = a + b;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= (uint32_t) o)
+                incl += t;
         }
-        hist[p * MAX_RADIX + threadIdx.x] = s[threadIdx.x] - v;
+        if (lane == 31)
+            s_sum[w] = incl;
+        __syncthreads();
+        uint32_t pre = incl - a - b;
+        for (uint32_t k = 0; k < w; ++k)
+            pre += s_sum[k];
+        h[0] = pre;
+        h[1] = pre + a;
         __syncthreads();
     }
+}
+
+__global__ void __launch_bounds__(256) radix_hist_kernel(const uint32_t* __restrict__ keys, uint32_t n, SortPlan pl,
+    uint32_t* __restrict__ hist, uint32_t* __restrict__ done, uint32_t* __restrict__ status, uint64_t status_words) {
+    radix_hist(keys, n, pl, hist, done, status, status_words, gridDim.x);
 }
 
 __device__ __forceinline__ uint32_t ld_volatile(const uint32_t* p) {
@@ -282,7 +334,7 @@ __device__ __forceinline__ void st_volatile(uint32_t* p, uint32_t v) {
 // The look-back waits are bounded (wait_polls polls of a predecessor that has published nothing). A wait
 // that runs out records ERR_LOOKBACK_TIMEOUT; every other wait then stops at its next poll and later passes
 // return at once. A tile that gave up adds only the counts it saw, so its destinations stay at or below the
-// true ones (inside the output); sort_sanitize_kernel then replaces the unfinished output by a valid one.
+// true ones (inside the output); boundary_starts_kernel then replaces the unfinished output by a valid one.
 template<bool GATHER, int BITS>
 __global__ void __launch_bounds__(SORT_THREADS, 3) onesweep_kernel(const uint32_t* __restrict__ keys_in,
     const uint32_t* __restrict__ vals_in, uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, uint32_t n,
@@ -497,19 +549,6 @@ __global__ void __launch_bounds__(SORT_THREADS, 3) onesweep_kernel(const uint32_
     }
 }
 
-// After a radix sort whose look-back gave up: every particle gets the invalid key nbins and the identity
-// order, a valid sorted state (an empty grid), so that no later stage indexes with unfinished output. The
-// frame reports P2V_ETIMEOUT.
-__global__ void __launch_bounds__(256) sort_sanitize_kernel(uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
-    uint32_t n, uint32_t nbins, const uint32_t* __restrict__ err, const FrameScalars* __restrict__ gate) {
-    if (radix_skipped(gate) || !(ld_volatile(err) & ERR_LOOKBACK_TIMEOUT))
-        return;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        keys[i] = nbins;
-        vals[i] = i;
-    }
-}
-
 // start[c] = first sorted position whose key is >= c, for c in [0, nbins]. Boundary i of the sorted keys (between
 // keys[i-1] and keys[i]) starts the run of cells (keys[i-1], keys[i]]. A warp takes 32 consecutive boundaries, scans the
 // lengths of their runs, and its lanes write the cells of all 32 runs together (consecutive lanes, consecutive cells:
@@ -517,16 +556,20 @@ __global__ void __launch_bounds__(256) sort_sanitize_kernel(uint32_t* __restrict
 // lengths). A run of more than RUN_MAX cells (a sparse grid holds runs of millions of empty cells) is queued in chunks of
 // at most GAP_CHUNK for cell_gap_fill_kernel. Such runs are disjoint, so the chunks number at most (nbins + 1)
 // (1 / GAP_CHUNK + 1 / (RUN_MAX + 1)), below the nbins / 64 + 2 entries the list holds.
+// After a radix sort whose look-back gave up (err), every particle gets the invalid key nbins and the identity order, a
+// valid sorted state (an empty grid), so that no later stage indexes with unfinished output; the frame reports
+// P2V_ETIMEOUT.
 // Bound by its stores: uniform 16M (338 M cells, runs of 21) 0.39 ms; a search per cell in a table of every 64th cell's
 // start, as sparse frames took before, 1.39 ms.
 constexpr uint32_t GAP_CHUNK = 8192;
 constexpr uint32_t RUN_MAX = 8192;
 
-__global__ void __launch_bounds__(256) boundary_starts_kernel(const uint32_t* __restrict__ keys, uint32_t n,
-    uint32_t nbins, uint32_t* __restrict__ out, uint4* __restrict__ gaps, uint32_t gap_cap,
+__global__ void __launch_bounds__(256) boundary_starts_kernel(uint32_t* __restrict__ keys,
+    uint32_t* __restrict__ vals, uint32_t n, uint32_t nbins, uint32_t* __restrict__ out, uint4* __restrict__ gaps, uint32_t gap_cap,
     FrameScalars* __restrict__ fs, const FrameScalars* __restrict__ gate) {
     if (radix_skipped(gate))
         return;
+    const bool failed = (ld_volatile(&fs->error) & ERR_LOOKBACK_TIMEOUT) != 0u;
     const uint32_t lane = lane_id();
     const uint64_t wstride = (uint64_t) gridDim.x * blockDim.x;
     for (uint64_t base = (uint64_t) blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base <= n; base += wstride) {
@@ -534,10 +577,17 @@ __global__ void __launch_bounds__(256) boundary_starts_kernel(const uint32_t* __
         uint32_t lo = 1u, hi = 0u;  // empty run
         if (i64 <= n) {
             const uint32_t i = (uint32_t) i64;
-            lo = i == 0 ? 0u : keys[i - 1] + 1u;
-            hi = i == n ? nbins : keys[i];
-            if (hi > nbins)
+            if (!failed) {
+                lo = i == 0 ? 0u : keys[i - 1] + 1u;
+                hi = i == n ? nbins : min(keys[i], nbins);
+            } else {
+                lo = i == 0 ? 0u : nbins + 1u;
                 hi = nbins;
+                if (i < n) {
+                    keys[i] = nbins;
+                    vals[i] = i;
+                }
+            }
         }
         uint32_t len = lo <= hi ? hi - lo + 1u : 0u;
         if (len > RUN_MAX) {
@@ -596,14 +646,6 @@ __global__ void __launch_bounds__(256) cell_gap_fill_kernel(const uint4* __restr
 }
 
 // ---- counting sort by cell ----
-// counts[key] = particles per key, keys in [0, nbins] (nbins: the invalid particles); rank[i] = the
-// particle's arrival rank in its cell (its slot there until order_bins_kernel fixes the order)
-__global__ void __launch_bounds__(256) count_bins_kernel(const uint32_t* __restrict__ keys, uint32_t n,
-                                                         uint32_t* __restrict__ counts, uint32_t* __restrict__ rank) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        rank[i] = atomicAdd(counts + keys[i], 1u);
-}
-
 constexpr int SCAN_THREADS = 256, SCAN_ITEMS = 16, SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
 // 16 consecutive counts of thread `tid` in tile `tile` (zeros past nb); true when all 16 exist
@@ -627,7 +669,8 @@ __device__ __forceinline__ bool load_counts(const uint32_t* __restrict__ counts,
     return full;
 }
 
-// Scan of the cell counts in three steps (tile sums, their scan, tile scans): no cross-tile waiting.
+// Scan of the cell counts in two steps (tile sums; tile scans, each block adding up the sums before its tile): no
+// cross-tile waiting.
 // Step 1: the sum of every tile of SCAN_TILE counts, and the largest count (fs->bin_maxcount).
 __global__ void __launch_bounds__(SCAN_THREADS) bin_tile_sums_kernel(const uint32_t* __restrict__ counts, uint32_t nb,
     uint32_t* __restrict__ tsum, FrameScalars* __restrict__ fs) {
@@ -662,56 +705,21 @@ __global__ void __launch_bounds__(SCAN_THREADS) bin_tile_sums_kernel(const uint3
     }
 }
 
-// Step 2: exclusive scan of the tile sums in place (one block).
-__global__ void __launch_bounds__(1024) bin_tile_scan_kernel(uint32_t* __restrict__ tsum, uint32_t ntiles) {
-    __shared__ uint32_t s_warp[32];
-    __shared__ uint32_t s_carry;
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    if (tid == 0)
-        s_carry = 0;
-    __syncthreads();
-    for (uint32_t base = 0; base < ntiles; base += 1024) {
-        const uint32_t i = base + tid;
-        const uint32_t x = i < ntiles ? tsum[i] : 0u;
-        uint32_t incl = x;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o)
-                incl += t;
-        }
-        if (lane == 31)
-            s_warp[w] = incl;
-        __syncthreads();
-        if (w == 0) {
-            uint32_t ws = s_warp[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t t = __shfl_up_sync(0xffffffffu, ws, o);
-                if (lane >= o)
-                    ws += t;
-            }
-            s_warp[lane] = ws;  // inclusive over warps
-        }
-        __syncthreads();
-        const uint32_t carry = s_carry;
-        const uint32_t excl = carry + (w > 0 ? s_warp[w - 1] : 0u) + incl - x;
-        if (i < ntiles)
-            tsum[i] = excl;
-        __syncthreads();
-        if (tid == 0)
-            s_carry = carry + s_warp[31];
-        __syncthreads();
-    }
-}
-
-// Step 3: start[c] = tile prefix + the scan inside the tile, for c in [0, nb); cells holding two or more
+// Step 2: start[c] = the sums of the tiles before + the scan inside the tile, for c in [0, nb); cells holding two or more
 // particles are appended to `multi` (their order inside the cell is fixed by order_bins_kernel).
 __global__ void __launch_bounds__(SCAN_THREADS) bin_starts_kernel(const uint32_t* __restrict__ counts, uint32_t nb,
     const uint32_t* __restrict__ tsum, uint32_t* __restrict__ start, uint32_t* __restrict__ multi,
     FrameScalars* __restrict__ fs) {
-    __shared__ uint32_t s_warp[SCAN_THREADS / 32];
+    __shared__ uint32_t s_warp[SCAN_THREADS / 32], s_before[SCAN_THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    uint32_t before = 0;
+    for (uint32_t k = tid; k < blockIdx.x; k += SCAN_THREADS)
+        before += tsum[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        before += __shfl_xor_sync(0xffffffffu, before, o);
+    if (lane == 0)
+        s_before[w] = before;
     const uint64_t b0 = (uint64_t) blockIdx.x * SCAN_TILE + (uint64_t) tid * SCAN_ITEMS;
     uint32_t v[SCAN_ITEMS];
     const bool full = load_counts(counts, nb, b0, v);
@@ -743,7 +751,9 @@ __global__ void __launch_bounds__(SCAN_THREADS) bin_starts_kernel(const uint32_t
     uint32_t wpre = 0;
     for (int k = 0; k < w; ++k)
         wpre += s_warp[k];
-    uint32_t run = tsum[blockIdx.x] + wpre + incl - sum;
+    uint32_t run = wpre + incl - sum;
+    for (int k = 0; k < SCAN_THREADS / 32; ++k)
+        run += s_before[k];
 #pragma unroll
     for (int e = 0; e < SCAN_ITEMS; ++e) {
         if (v[e] >= 2u)
@@ -788,13 +798,18 @@ __global__ void __launch_bounds__(256) scatter_bins_kernel(const uint32_t* __res
 }
 
 // Every cell with two or more particles (the list `multi`) puts them in index order (an insertion sort of
-// at most BIN_CELL_MAX entries) and rewrites their values and records: the result is the stable sort by key.
-__global__ void __launch_bounds__(256) order_bins_kernel(uint32_t n, uint32_t nbins, const uint32_t* __restrict__ multi,
+// at most BIN_CELL_MAX entries) and rewrites their values and records: the result is the stable sort by key. A frame with
+// a fuller cell goes to the radix sort instead, and takes its histograms here.
+__global__ void __launch_bounds__(256) order_bins_kernel(const uint32_t* __restrict__ keys, SortPlan pl,
+    uint32_t* __restrict__ hist, uint32_t* __restrict__ done, uint32_t* __restrict__ status, uint64_t status_words,
+    uint32_t hist_blocks, uint32_t n, uint32_t nbins, const uint32_t* __restrict__ multi,
     uint32_t* __restrict__ vals, const uint32_t* __restrict__ start, const float4* __restrict__ xyzr,
     float4* __restrict__ rec_a, int4* __restrict__ rec_b, float4* __restrict__ xyzr_out, GridGeo geo,
     const FrameScalars* __restrict__ fs) {
-    if (fs->bin_maxcount > BIN_CELL_MAX)
+    if (fs->bin_maxcount > BIN_CELL_MAX) {
+        radix_hist(keys, n, pl, hist, done, status, status_words, hist_blocks);
         return;
+    }
     const uint32_t nm = fs->bin_nmulti;
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nm; q += gridDim.x * blockDim.x) {
         const uint32_t k = multi[q];
@@ -836,6 +851,26 @@ __global__ void __launch_bounds__(256) keys_from_starts_kernel(const uint32_t* _
     }
 }
 
+// The frame's first kernel: its scalars, the counting sort's cell counts (a multiple of four words) and the radix sort's
+// histograms and counters.
+__global__ void __launch_bounds__(256) init_frame_kernel(FrameScalars* fs, uint4* __restrict__ counts, uint64_t ncounts4,
+                                                         uint32_t* __restrict__ hist, uint32_t hist_words) {
+    const uint64_t t = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x, step = (uint64_t) gridDim.x * blockDim.x;
+    for (uint64_t i = t; i < ncounts4; i += step)
+        counts[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (uint64_t i = t; i < hist_words; i += step)
+        hist[i] = 0u;
+    if (t == 0) {
+        FrameScalars z{};
+        for (int a = 0; a < 3; ++a) {
+            z.cmin[a] = INT32_MAX;
+            z.cmax[a] = INT32_MIN;
+        }
+        z.dmin_bits = 0x7f7fffffu;  // FLT_MAX, as the vector aggregator's minDens starts
+        *fs = z;
+    }
+}
+
 __global__ void count_valid_kernel(const uint32_t* __restrict__ start, uint32_t nbins, FrameScalars* fs) {
     fs->n_valid = start[nbins];
 }
@@ -845,8 +880,8 @@ __global__ void count_valid_kernel(const uint32_t* __restrict__ start, uint32_t 
 // ---------------------------------------------------------------------------------------------
 // host launchers
 // ---------------------------------------------------------------------------------------------
-cudaError_t launch_pack_keys(const ListDesc& L, const GridGeo& g, float4* xyzr, uint32_t* keys, uint32_t* idx,
-    FrameScalars* fs, uint32_t empty_flag, cudaStream_t st) {
+cudaError_t launch_pack_keys(const ListDesc& L, const GridGeo& g, float4* xyzr, uint32_t* keys, uint32_t* counts,
+    uint32_t* rank, FrameScalars* fs, uint32_t empty_flag, cudaStream_t st) {
     if (L.count == 0)
         return cudaSuccess;
     const dim3 block(256);
@@ -857,30 +892,30 @@ cudaError_t launch_pack_keys(const ListDesc& L, const GridGeo& g, float4* xyzr, 
     case 1: {  // FLOAT_XYZ
         bool al = (addr % 4 == 0) && (L.stride % 4 == 0);
         if (al)
-            pack_keys_kernel<float, 3, true><<<grid, block, 0, st>>>(L, g, xyzr, keys, idx, fs, empty_flag);
+            pack_keys_kernel<float, 3, true><<<grid, block, 0, st>>>(L, g, xyzr, keys, counts, rank, fs, empty_flag);
         else
-            pack_keys_kernel<float, 3, false><<<grid, block, 0, st>>>(L, g, xyzr, keys, idx, fs, empty_flag);
+            pack_keys_kernel<float, 3, false><<<grid, block, 0, st>>>(L, g, xyzr, keys, counts, rank, fs, empty_flag);
     } break;
     case 2: {  // FLOAT_XYZR
         bool al = (addr % 4 == 0) && (L.stride % 4 == 0);
         if (al)
-            pack_keys_kernel<float, 4, true><<<grid, block, 0, st>>>(L, g, xyzr, keys, idx, fs, empty_flag);
+            pack_keys_kernel<float, 4, true><<<grid, block, 0, st>>>(L, g, xyzr, keys, counts, rank, fs, empty_flag);
         else
-            pack_keys_kernel<float, 4, false><<<grid, block, 0, st>>>(L, g, xyzr, keys, idx, fs, empty_flag);
+            pack_keys_kernel<float, 4, false><<<grid, block, 0, st>>>(L, g, xyzr, keys, counts, rank, fs, empty_flag);
     } break;
     case 3: {  // SHORT_XYZ
         bool al = (addr % 2 == 0) && (L.stride % 2 == 0);
         if (al)
-            pack_keys_kernel<uint16_t, 3, true><<<grid, block, 0, st>>>(L, g, xyzr, keys, idx, fs, empty_flag);
+            pack_keys_kernel<uint16_t, 3, true><<<grid, block, 0, st>>>(L, g, xyzr, keys, counts, rank, fs, empty_flag);
         else
-            pack_keys_kernel<uint16_t, 3, false><<<grid, block, 0, st>>>(L, g, xyzr, keys, idx, fs, empty_flag);
+            pack_keys_kernel<uint16_t, 3, false><<<grid, block, 0, st>>>(L, g, xyzr, keys, counts, rank, fs, empty_flag);
     } break;
     case 4: {  // DOUBLE_XYZ
         bool al = (addr % 8 == 0) && (L.stride % 8 == 0);
         if (al)
-            pack_keys_kernel<double, 3, true><<<grid, block, 0, st>>>(L, g, xyzr, keys, idx, fs, empty_flag);
+            pack_keys_kernel<double, 3, true><<<grid, block, 0, st>>>(L, g, xyzr, keys, counts, rank, fs, empty_flag);
         else
-            pack_keys_kernel<double, 3, false><<<grid, block, 0, st>>>(L, g, xyzr, keys, idx, fs, empty_flag);
+            pack_keys_kernel<double, 3, false><<<grid, block, 0, st>>>(L, g, xyzr, keys, counts, rank, fs, empty_flag);
     } break;
     default:
         return cudaErrorInvalidValue;
@@ -888,8 +923,17 @@ cudaError_t launch_pack_keys(const ListDesc& L, const GridGeo& g, float4* xyzr, 
     return cudaGetLastError();
 }
 
-size_t sort_status_words(uint32_t n) {
-    return (size_t) ceil_div(n, SORT_TILE) * MAX_RADIX;
+namespace {
+size_t status_words_of(const SortPlan& pl, uint32_t n) {  // every pass has its own look-back words
+    size_t w = 0;
+    for (int p = 0; p < pl.passes; ++p)
+        w += (size_t) ceil_div(n, SORT_TILE) << pl.bits[p];
+    return w;
+}
+}  // namespace
+
+size_t sort_status_words(uint32_t n, uint32_t max_key) {
+    return std::max(status_words_of(sort_plan(max_key), n), status_words_of(sort_plan(max_key, true), n));
 }
 
 size_t sort_hist_words() {
@@ -912,7 +956,7 @@ uint32_t sort_empty_flag(uint32_t max_key) {
 
 template<bool GATHER, int BITS>
 cudaError_t launch_onesweep_bits(uint32_t tiles, SortBuffers& b, int cur, uint32_t n, int shift, const uint32_t* offs,
-                                 uint32_t* counter, cudaStream_t st, const FrameScalars* gate) {
+                                 uint32_t* counter, uint32_t* status, cudaStream_t st, const FrameScalars* gate) {
     constexpr int RADIX = 1 << BITS;
     const int smem = (int) sizeof(uint32_t) * (2 * SORT_TILE + SORT_WARPS * RADIX + 2 * RADIX);
     const cudaError_t e = cudaFuncSetAttribute(onesweep_kernel<GATHER, BITS>,
@@ -921,7 +965,7 @@ cudaError_t launch_onesweep_bits(uint32_t tiles, SortBuffers& b, int cur, uint32
         return e;
     onesweep_kernel<GATHER, BITS><<<tiles, SORT_THREADS, smem, st>>>(b.keys[cur],
         (cur == 0 && b.implicit_vals0 && b.first_pass) ? nullptr : b.vals[cur], b.keys[cur ^ 1],
-        b.vals[cur ^ 1], n, shift, offs, counter, b.status, b.err, GATHER ? b.xyzr_in : nullptr,
+        b.vals[cur ^ 1], n, shift, offs, counter, status, b.err, GATHER ? b.xyzr_in : nullptr,
         GATHER ? b.rec_a : nullptr, GATHER ? b.rec_b : nullptr, GATHER ? b.xyzr_out : nullptr, b.geo, gate,
         b.wait_polls ? b.wait_polls : SPIN_LIMIT, b.first_pass ? b.hold_tile : -1);
     return cudaSuccess;
@@ -929,42 +973,62 @@ cudaError_t launch_onesweep_bits(uint32_t tiles, SortBuffers& b, int cur, uint32
 
 template<bool GATHER>
 cudaError_t launch_onesweep(int bits, uint32_t tiles, SortBuffers& b, int cur, uint32_t n, int shift,
-                            const uint32_t* offs, uint32_t* counter, cudaStream_t st, const FrameScalars* gate) {
-    return bits == 9 ? launch_onesweep_bits<GATHER, 9>(tiles, b, cur, n, shift, offs, counter, st, gate)
-                     : launch_onesweep_bits<GATHER, 8>(tiles, b, cur, n, shift, offs, counter, st, gate);
+                            const uint32_t* offs, uint32_t* counter, uint32_t* status, cudaStream_t st,
+                            const FrameScalars* gate) {
+    return bits == 9 ? launch_onesweep_bits<GATHER, 9>(tiles, b, cur, n, shift, offs, counter, status, st, gate)
+                     : launch_onesweep_bits<GATHER, 8>(tiles, b, cur, n, shift, offs, counter, status, st, gate);
 }
 
-cudaError_t launch_sort(SortBuffers& b, uint32_t n, uint32_t max_key, int sms, cudaStream_t st, const FrameScalars* gate,
-                        bool odd) {
-    const SortPlan pl = sort_plan(max_key, odd);
+namespace {
+unsigned hist_grid(uint32_t n, int sms) {
+    return (unsigned) std::max<uint32_t>(1u, std::min<uint32_t>(ceil_div(n, 256 * 8), (uint32_t) sms * 4));
+}
+
+// the radix passes, after their histograms
+cudaError_t launch_passes(SortBuffers& b, const SortPlan& pl, uint32_t n, cudaStream_t st, const FrameScalars* gate) {
     const uint32_t tiles = ceil_div(n, SORT_TILE);
-    cudaError_t e = cudaMemsetAsync(b.hist, 0, sizeof(uint32_t) * HIST_WORDS + sizeof(uint32_t) * MAX_PASSES, st);
-    if (e != cudaSuccess)
-        return e;
-    b.result = pl.passes & 1;
-    if (n == 0)
-        return cudaSuccess;
-    const unsigned hgrid = (unsigned) std::min<uint32_t>(ceil_div(n, 256 * 8), (uint32_t) sms * 4);
-    radix_hist_kernel<<<hgrid ? hgrid : 1, 256, 0, st>>>(b.keys[0], n, pl, b.hist, gate);
-    radix_scan_kernel<<<1, MAX_RADIX, 0, st>>>(b.hist, pl.passes, gate);
+    uint32_t* status = b.status;
     int cur = 0;
     for (int p = 0; p < pl.passes; ++p) {
         b.first_pass = p == 0;
-        e = cudaMemsetAsync(b.status, 0, sizeof(uint32_t) * (size_t) tiles * ((size_t) 1 << pl.bits[p]), st);
-        if (e != cudaSuccess)
-            return e;
         uint32_t* counter = b.hist + HIST_WORDS + p;
-        const bool last = p == pl.passes - 1;
-        if (last && b.xyzr_in != nullptr)
-            e = launch_onesweep<true>(pl.bits[p], tiles, b, cur, n, pl.shift[p], b.hist + p * MAX_RADIX, counter, st,
-                                      gate);
-        else
-            e = launch_onesweep<false>(pl.bits[p], tiles, b, cur, n, pl.shift[p], b.hist + p * MAX_RADIX, counter, st,
-                                       gate);
+        const uint32_t* offs = b.hist + p * MAX_RADIX;
+        const cudaError_t e =
+            p == pl.passes - 1 && b.xyzr_in != nullptr
+                ? launch_onesweep<true>(pl.bits[p], tiles, b, cur, n, pl.shift[p], offs, counter, status, st, gate)
+                : launch_onesweep<false>(pl.bits[p], tiles, b, cur, n, pl.shift[p], offs, counter, status, st, gate);
         if (e != cudaSuccess)
             return e;
+        status += (size_t) tiles << pl.bits[p];
         cur ^= 1;
     }
+    return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t launch_sort(SortBuffers& b, uint32_t n, uint32_t max_key, int sms, cudaStream_t st) {
+    const SortPlan pl = sort_plan(max_key);
+    b.result = pl.passes & 1;
+    if (n == 0)
+        return cudaSuccess;
+    const cudaError_t e = cudaMemsetAsync(b.hist, 0, sizeof(uint32_t) * sort_hist_words(), st);
+    if (e != cudaSuccess)
+        return e;
+    radix_hist_kernel<<<hist_grid(n, sms), 256, 0, st>>>(b.keys[0], n, pl, b.hist, b.hist + HIST_WORDS + MAX_PASSES,
+                                                         b.status, status_words_of(pl, n));
+    return launch_passes(b, pl, n, st, nullptr);
+}
+
+cudaError_t launch_init_frame(FrameScalars* fs, uint32_t* counts, uint32_t nbins, uint32_t* hist, int sms,
+                              cudaStream_t st) {
+    const uint64_t c4 = counts ? ((uint64_t) nbins + 4) / 4 : 0;
+    const unsigned grid = (unsigned) std::max<uint64_t>(4, std::min<uint64_t>((c4 + 255) / 256, (uint64_t) sms * 8));
+    init_frame_kernel<<<grid, 256, 0, st>>>(fs, reinterpret_cast<uint4*>(counts), c4, hist, (uint32_t) sort_hist_words());
+    return cudaGetLastError();
+}
+
+cudaError_t launch_count_valid(const uint32_t* start, uint32_t nbins, FrameScalars* fs, cudaStream_t st) {
+    count_valid_kernel<<<1, 1, 0, st>>>(start, nbins, fs);
     return cudaGetLastError();
 }
 
@@ -983,39 +1047,40 @@ cudaError_t launch_bin_sort(SortBuffers& b, uint32_t n, const GridGeo& g, uint32
                             uint4* gaps, uint32_t gap_cap, FrameScalars* fs, int sms,
                             cudaStream_t st) {
     const uint32_t nb = g.nbins + 1;
-    cudaError_t e;
     const bool counting = counts != nullptr && n > 0;
-    if (counting) {
-        // counting sort by cell: histogram, scan (= the cell starts), scatter, per-cell index order
-        const uint32_t ntiles = (uint32_t) bin_scan_words(g.nbins);
-        if ((e = cudaMemsetAsync(counts, 0, sizeof(uint32_t) * nb, st)) != cudaSuccess)
-            return e;
-        const unsigned pgrid = (unsigned) std::max<uint32_t>(1u, std::min<uint32_t>(ceil_div(n, 256), (uint32_t) sms * 16));
-        // ranks in vals[0]: the gated radix sort then takes the identity as its first pass' values
-        b.implicit_vals0 = true;
-        count_bins_kernel<<<pgrid, 256, 0, st>>>(b.keys[0], n, counts, b.vals[0]);
-        // tile sums in the status buffer; the multi-particle cell list in keys[1] (the counting sort writes no
-        // sorted keys there)
-        bin_tile_sums_kernel<<<ntiles, SCAN_THREADS, 0, st>>>(counts, nb, b.status, fs);
-        bin_tile_scan_kernel<<<1, 1024, 0, st>>>(b.status, ntiles);
-        bin_starts_kernel<<<ntiles, SCAN_THREADS, 0, st>>>(counts, nb, b.status, start, b.keys[1], fs);
-        scatter_bins_kernel<<<pgrid, 256, 0, st>>>(b.keys[0], b.vals[0], b.xyzr_in, n, start, b.vals[1], b.rec_a,
-                                                   b.rec_b, b.xyzr_out, b.geo, fs);
-        order_bins_kernel<<<pgrid, 256, 0, st>>>(n, g.nbins, b.keys[1], b.vals[1], start, b.xyzr_in, b.rec_a, b.rec_b,
-                                                 b.xyzr_out, b.geo, fs);
-    }
     // the radix path: alone, or as the fallback (gated) when a cell holds more than BIN_CELL_MAX particles;
     // with the counting sort its pass count is odd so both leave the sorted keys in buffer 1
     const FrameScalars* gate = counting ? fs : nullptr;
     const uint32_t max_key = b.empty_flag ? (b.empty_flag | (b.empty_flag - 1u)) : g.nbins;
-    if ((e = launch_sort(b, n, max_key, sms, st, gate, counting)) != cudaSuccess)
-        return e;
+    const SortPlan pl = sort_plan(max_key, counting);
+    b.result = pl.passes & 1;
+    uint32_t* done = b.hist + HIST_WORDS + MAX_PASSES;
+    const uint64_t sw = status_words_of(pl, n);
+    if (counting) {
+        // counting sort by cell (counts and arrival ranks from the packing): scan (= the cell starts), scatter, per-cell
+        // index order. Tile sums in the status buffer; the multi-particle cell list in keys[1] (the counting sort writes no
+        // sorted keys there); ranks in vals[0], the gated radix sort takes the identity as its first pass' values
+        const uint32_t ntiles = (uint32_t) bin_scan_words(g.nbins);
+        const unsigned pgrid = (unsigned) std::max<uint32_t>(1u, std::min<uint32_t>(ceil_div(n, 256), (uint32_t) sms * 16));
+        b.implicit_vals0 = true;
+        bin_tile_sums_kernel<<<ntiles, SCAN_THREADS, 0, st>>>(counts, nb, b.status, fs);
+        bin_starts_kernel<<<ntiles, SCAN_THREADS, 0, st>>>(counts, nb, b.status, start, b.keys[1], fs);
+        scatter_bins_kernel<<<pgrid, 256, 0, st>>>(b.keys[0], b.vals[0], b.xyzr_in, n, start, b.vals[1], b.rec_a,
+                                                   b.rec_b, b.xyzr_out, b.geo, fs);
+        order_bins_kernel<<<pgrid, 256, 0, st>>>(b.keys[0], pl, b.hist, done, b.status, sw,
+                                                 std::min(pgrid, hist_grid(n, sms)), n, g.nbins, b.keys[1], b.vals[1], start, b.xyzr_in, b.rec_a, b.rec_b, b.xyzr_out, b.geo, fs);
+    } else if (n > 0) {
+        radix_hist_kernel<<<hist_grid(n, sms), 256, 0, st>>>(b.keys[0], n, pl, b.hist, done, b.status, sw);
+    }
+    if (n > 0) {
+        const cudaError_t e = launch_passes(b, pl, n, st, gate);
+        if (e != cudaSuccess)
+            return e;
+    }
     const unsigned grid = (unsigned) std::max<uint32_t>(1u, std::min<uint32_t>(ceil_div(n + 1, 256), sms * 8));
-    if (n > 0)
-        sort_sanitize_kernel<<<grid, 256, 0, st>>>(b.keys[b.result], b.vals[b.result], n, g.nbins, b.err, gate);
-    boundary_starts_kernel<<<grid, 256, 0, st>>>(b.keys[b.result], n, g.nbins, start, gaps, gap_cap, fs, gate);
+    boundary_starts_kernel<<<grid, 256, 0, st>>>(b.keys[b.result], b.vals[b.result], n, g.nbins, start, gaps, gap_cap, fs,
+                                                 gate);
     cell_gap_fill_kernel<<<sms * 2, 256, 0, st>>>(gaps, gap_cap, start, fs, gate);
-    count_valid_kernel<<<1, 1, 0, st>>>(start, g.nbins, fs);
     return cudaGetLastError();
 }
 

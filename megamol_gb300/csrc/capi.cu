@@ -186,16 +186,6 @@ struct FrameJob {
     uint32_t ao_fetches = 0;
 };
 
-__global__ void init_scalars_kernel(FrameScalars* fs) {
-    FrameScalars z{};
-    for (int a = 0; a < 3; ++a) {
-        z.cmin[a] = INT32_MAX;
-        z.cmax[a] = INT32_MIN;
-    }
-    z.dmin_bits = 0x7f7fffffu;  // FLT_MAX, as the vector aggregator's minDens starts
-    *fs = z;
-}
-
 }  // namespace
 
 struct p2v_ctx {
@@ -540,12 +530,13 @@ p2v_status p2v_ctx::enqueue_frame(Pipe& pp, const p2v_frame* fr, p2v_volume* vol
     const bool counting = n > 0 && (uint64_t) g.nbins + 1 <= 64ull * n &&
                           4ull * ((uint64_t) g.nbins + 1) <= COUNTING_TABLE_MAX_BYTES;
     if (counting)
-        P2V_CUDA_TRY(pp.bcount.ensure(4 * ((size_t) g.nbins + 1)));
+        P2V_CUDA_TRY(pp.bcount.ensure(4 * ((size_t) g.nbins + 4)));
     // the radix path sorts particles whose support holds no node after all others (a key bit above the cells),
     // so the density gather never visits them; the AO stages' brick order reads the cell table for every
     // particle and keeps plain cell keys
     const uint32_t empty_flag = (!counting && P.ao_brick_order == 0) ? sort_empty_flag(g.nbins) : 0u;
-    P2V_CUDA_TRY(status.ensure(4 * (std::max(sort_status_words(n), bin_scan_words(g.nbins)) + 256)));
+    const uint32_t max_key = empty_flag ? (empty_flag | (empty_flag - 1u)) : g.nbins;
+    P2V_CUDA_TRY(status.ensure(4 * (std::max(sort_status_words(n, max_key), bin_scan_words(g.nbins)) + 256)));
     P2V_CUDA_TRY(hist.ensure(4 * sort_hist_words()));
     P2V_CUDA_TRY(cstart.ensure(4 * ((size_t) g.nbins + 1)));
     P2V_CUDA_TRY(gaps.ensure(sizeof(uint4) * gap_cap));
@@ -581,13 +572,14 @@ p2v_status p2v_ctx::enqueue_frame(Pipe& pp, const p2v_frame* fr, p2v_volume* vol
         P2V_CUDA_TRY(pp.vkeys1.ensure(sizeof(uint32_t) * V));
         P2V_CUDA_TRY(pp.vvals0.ensure(sizeof(uint32_t) * V));
         P2V_CUDA_TRY(pp.vvals1.ensure(sizeof(uint32_t) * V));
-        P2V_CUDA_TRY(status.ensure(4 * (sort_status_words((uint32_t) V) + 256)));
+        P2V_CUDA_TRY(status.ensure(4 * (sort_status_words((uint32_t) V, 0xFFFFFFFFu) + 256)));
     }
 
     FrameScalars* fs = scal.as<FrameScalars>();
     if (timed)
         P2V_CUDA_TRY(cudaEventRecord(ev[EV_START], st));
-    init_scalars_kernel<<<1, 1, 0, st>>>(fs);
+    uint32_t* counts = counting ? pp.bcount.as<uint32_t>() : nullptr;
+    P2V_CUDA_TRY(launch_init_frame(fs, counts, g.nbins, hist.as<uint32_t>(), sms, st));
 
     // ---- upload + pack + keys ----
     uint64_t raw_need = 0;
@@ -634,7 +626,8 @@ p2v_status p2v_ctx::enqueue_frame(Pipe& pp, const p2v_frame* fr, p2v_volume* vol
                 raw_off += (bytes + 15) & ~uint64_t(15);
             }
         }
-        P2V_CUDA_TRY(launch_pack_keys(d, g, xyzr.as<float4>(), keys0.as<uint32_t>(), nullptr, fs, empty_flag, st));
+        P2V_CUDA_TRY(launch_pack_keys(d, g, xyzr.as<float4>(), keys0.as<uint32_t>(), counts, vals0.as<uint32_t>(), fs,
+                                      empty_flag, st));
         off += L.count;
     }
     if (timed)
@@ -755,7 +748,7 @@ p2v_status p2v_ctx::enqueue_frame(Pipe& pp, const p2v_frame* fr, p2v_volume* vol
         return fail(P2V_EINVAL, "sort_wait_polls must be >= 0");
     sb.wait_polls = (uint32_t) P.sort_wait_polls;
     sb.hold_tile = P.test_hold_sort ? 1 : -1;
-    P2V_CUDA_TRY(launch_bin_sort(sb, n, g, counting ? pp.bcount.as<uint32_t>() : nullptr, cstart.as<uint32_t>(),
+    P2V_CUDA_TRY(launch_bin_sort(sb, n, g, counts, cstart.as<uint32_t>(),
                                  gaps.as<uint4>(), gap_cap, fs, sms, st));
     const uint32_t* skeys = sb.keys[sb.result];
     if (slot) {
@@ -778,6 +771,7 @@ p2v_status p2v_ctx::enqueue_frame(Pipe& pp, const p2v_frame* fr, p2v_volume* vol
         P2V_CUDA_TRY(cudaMemcpyAsync(dgrid, ext_grid, sizeof(float) * V,
                                      ext_grid_mem == P2V_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                                      st));
+        P2V_CUDA_TRY(launch_count_valid(cstart.as<uint32_t>(), g.nbins, fs, st));
     } else {
         // aggregator 0: the density; 1: the intensity-weighted sums; 2: three direction-weighted passes into
         // the interleaved vector volume and the plain kernel sums (the weights) into wsum

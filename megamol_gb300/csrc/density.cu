@@ -101,6 +101,8 @@ __global__ void __launch_bounds__(TY* TZ, 2) gather_kernel(GridGeo g, const floa
     const int t = threadIdx.x;
     const int ty = t % TY;
     const int tz = t / TY;
+    if (blockIdx.x + blockIdx.y + blockIdx.z == 0 && t == 0)
+        fs->n_valid = start[g.nbins];
     // tiles cover the slab [zlo, zhi) of the grid (z tile index offset by the slab's first tile)
     const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, z0 = (blockIdx.z + g.zlo / TZ) * TZ;
     const bool row_in = (y0 + ty < g.s[1]) && (z0 + tz >= g.zlo) && (z0 + tz < g.zhi);
@@ -915,6 +917,8 @@ __global__ void __launch_bounds__(NT, GATHER_RES / NT) gather_fixed_kernel(const
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ GatherShared<TX, TY, TZ, NT> sh;
     const int t = threadIdx.x;
+    if (blockIdx.x + blockIdx.y + blockIdx.z == 0 && t == 0)
+        fs->n_valid = start[g.nbins];
     // tiles cover the slab [zlo, zhi) of the grid (z tile index offset by the slab's first tile)
     const uint32_t pass = blockIdx.z / tiles_z, bz = blockIdx.z - pass * tiles_z;
     const uint32_t tile = (bz * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;

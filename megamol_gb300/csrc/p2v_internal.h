@@ -43,27 +43,30 @@ struct SortBuffers {
     int32_t hold_tile = -1;   // test hook: this tile of the first pass never publishes its counts (-1 none)
 };
 
-// idx (optional) receives the identity order of the packed particles. empty_flag: 0, or the bit that
-// sort_empty_flag returns, added to the keys of particles whose support holds no grid node.
-cudaError_t launch_pack_keys(const ListDesc& L, const GridGeo& g, float4* xyzr, uint32_t* keys, uint32_t* idx,
-    FrameScalars* fs, uint32_t empty_flag, cudaStream_t st);
+// The frame's first kernel: initial scalars, zero cell counts (nullable; room for nbins + 4 words) and histograms.
+cudaError_t launch_init_frame(FrameScalars* fs, uint32_t* counts, uint32_t nbins, uint32_t* hist, int sms,
+    cudaStream_t st);
+// counts, rank (the counting sort, else null): particles per key and each particle's arrival rank. empty_flag: 0, or the
+// bit that sort_empty_flag returns, added to the keys of particles whose support holds no grid node.
+cudaError_t launch_pack_keys(const ListDesc& L, const GridGeo& g, float4* xyzr, uint32_t* keys, uint32_t* counts,
+    uint32_t* rank, FrameScalars* fs, uint32_t empty_flag, cudaStream_t st);
+// fs->n_valid = start[nbins] (the gathers do it themselves)
+cudaError_t launch_count_valid(const uint32_t* start, uint32_t nbins, FrameScalars* fs, cudaStream_t st);
 // The power of two above every cell key (max_key) that marks particles whose support holds no node, or 0 when
 // the extra key bit would cost the radix sort a pass.
 uint32_t sort_empty_flag(uint32_t max_key);
-size_t sort_status_words(uint32_t n);
+size_t sort_status_words(uint32_t n, uint32_t max_key);
 size_t sort_hist_words();
 int sort_passes(uint32_t max_key);
-// Stable LSD radix sort of keys[0] / vals[0]; b.result names the buffers holding the output. With a gate
-// every kernel returns at once unless the gate's counting sort overflowed; odd: an odd pass count.
-cudaError_t launch_sort(SortBuffers& b, uint32_t n, uint32_t max_key, int sms, cudaStream_t st,
-    const FrameScalars* gate = nullptr, bool odd = false);
+// Stable LSD radix sort of keys[0] / vals[0]; b.result names the buffers holding the output.
+cudaError_t launch_sort(SortBuffers& b, uint32_t n, uint32_t max_key, int sms, cudaStream_t st);
 // keys[j] for sorted positions j from the cell start table (the counting sort writes no sorted keys).
 cudaError_t launch_keys_from_starts(const uint32_t* start, uint32_t nbins, uint32_t n, uint32_t* keys, int sms,
     cudaStream_t st);
 // Words of the status buffer the counting sort's scan needs for nbins + 1 cells.
 size_t bin_scan_words(uint32_t nbins);
-// The particle binning: the stable sort of the bin keys (keys[0], vals[0] from launch_pack_keys) with the
-// gather records, and the cell start table (nbins + 1 entries). counts (nbins + 1 words) selects the
+// The particle binning (after launch_init_frame and launch_pack_keys): the stable sort of the bin keys (keys[0]) with the
+// gather records, and the cell start table (nbins + 1 entries). counts (from the packing, ranks in vals[0]) selects the
 // counting sort by cell, whose per-cell ordering handles cells of up to 32 particles; a fuller cell sends
 // the frame through the radix sort on the device. counts == nullptr: the radix sort alone.
 cudaError_t launch_bin_sort(SortBuffers& b, uint32_t n, const GridGeo& g, uint32_t* counts, uint32_t* start,
