@@ -225,8 +225,9 @@ struct p2v_ctx {
     // p2v_run_ao_on_grid: the density grid the AO stage reads instead of this frame's own (null: none)
     const float* ext_grid = nullptr;
     int ext_grid_mem = P2V_MEM_HOST;
-    DevBuf mlp_P, mlp_m, mlp_v, mlp_g, mlp_part, mlp_ploss, mlp_loss, mlp_w1h, mlp_w2h, mlp_lo, mlp_hi, mlp_idx,
-        mlp_y;
+    DevBuf mlp_P, mlp_m, mlp_v, mlp_g, mlp_part, mlp_ploss, mlp_w1h, mlp_w2h, mlp_lo, mlp_hi, mlp_idx, mlp_y;
+    DevBuf mlp_gx;                       // p2v_mlp_gradients' pairs
+    float* mlp_gh = nullptr;             // its pinned result (gradient and loss)
     DevBuf tX, tT;                       // collected training pairs
     uint64_t t_pairs = 0, t_cap = 0;
     std::vector<uint32_t> t_valid;       // indices of pairs with features
@@ -1752,8 +1753,7 @@ p2v_status p2v_ctx::mlp_alloc() {
     P2V_CUDA_TRY(mlp_P.ensure(sizeof(float) * MLP_NPARAM));
     P2V_CUDA_TRY(mlp_m.ensure(sizeof(float) * MLP_NPARAM));
     P2V_CUDA_TRY(mlp_v.ensure(sizeof(float) * MLP_NPARAM));
-    P2V_CUDA_TRY(mlp_g.ensure(sizeof(float) * MLP_NPARAM));
-    P2V_CUDA_TRY(mlp_loss.ensure(sizeof(float) * 4));
+    P2V_CUDA_TRY(mlp_g.ensure(sizeof(float) * (MLP_NPARAM + 1)));  // and the loss
     P2V_CUDA_TRY(mlp_w1h.ensure(sizeof(__nv_bfloat16) * MLP_H * MLP_KP));
     P2V_CUDA_TRY(mlp_w2h.ensure(sizeof(__nv_bfloat16) * MLP_H * MLP_H));
     P2V_CUDA_TRY(mlp_lo.ensure(sizeof(float) * MLP_IN));
@@ -1917,7 +1917,9 @@ void p2v_destroy(p2v_ctx* c) {
         cudaFreeHost(c->b_segs_h);
     if (c->b_err_h)
         cudaFreeHost(c->b_err_h);
-    for (DevBuf* b : {&c->mlp_P, &c->mlp_m, &c->mlp_v, &c->mlp_g, &c->mlp_part, &c->mlp_ploss, &c->mlp_loss,
+    if (c->mlp_gh)
+        cudaFreeHost(c->mlp_gh);
+    for (DevBuf* b : {&c->mlp_P, &c->mlp_m, &c->mlp_v, &c->mlp_g, &c->mlp_part, &c->mlp_ploss, &c->mlp_gx,
                       &c->mlp_w1h, &c->mlp_w2h, &c->mlp_lo, &c->mlp_hi, &c->mlp_idx, &c->mlp_y, &c->tX, &c->tT})
         b->release();
     if (c->own_stream)
@@ -2343,7 +2345,7 @@ p2v_status p2v_mlp_train(p2v_ctx* c, const p2v_train_params* tp, p2v_train_repor
     c->mlp_init_params(tp->seed, (float) std::log(mean / (1.0 - mean)));
 
     const int batch = tp->batch;
-    const int nblk = (batch + 31) / 32;
+    const int nblk = mlp_train_blocks(batch);
     if (c->mlp_idx.ensure(sizeof(uint32_t) * (train.size() + val.size() + 8)) != cudaSuccess ||
         c->mlp_part.ensure(sizeof(float) * (size_t) nblk * MLP_NPARAM) != cudaSuccess ||
         c->mlp_ploss.ensure(sizeof(float) * nblk) != cudaSuccess ||
@@ -2367,8 +2369,7 @@ p2v_status p2v_mlp_train(p2v_ctx* c, const p2v_train_params* tp, p2v_train_repor
         for (size_t b0 = 0; b0 < train.size(); b0 += (size_t) batch) {
             const int nb = (int) std::min<size_t>((size_t) batch, train.size() - b0);
             e = launch_mlp_train_step(c->mlp_P.as<float>(), c->tX.as<float>(), c->tT.as<float>(), d_idx + b0, nb,
-                                      c->mlp_part.as<float>(), c->mlp_ploss.as<float>(), c->mlp_g.as<float>(),
-                                      c->mlp_loss.as<float>(), st);
+                                      c->mlp_part.as<float>(), c->mlp_ploss.as<float>(), c->mlp_g.as<float>(), st);
             if (e == cudaSuccess)
                 e = launch_mlp_adam(c->mlp_P.as<float>(), c->mlp_g.as<float>(), c->mlp_m.as<float>(),
                                     c->mlp_v.as<float>(), lr, tp->beta1, tp->beta2, tp->eps, ++c->mlp_step, st);
@@ -2379,7 +2380,7 @@ p2v_status p2v_mlp_train(p2v_ctx* c, const p2v_train_params* tp, p2v_train_repor
         lr *= tp->lr_decay;
     }
     float last_loss = 0.0f;
-    cudaMemcpyAsync(&last_loss, c->mlp_loss.ptr, sizeof(float), cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(&last_loss, c->mlp_g.as<float>() + MLP_NPARAM, sizeof(float), cudaMemcpyDeviceToHost, st);
     const size_t last_nb = train.size() % (size_t) batch ? train.size() % (size_t) batch : (size_t) batch;
     float val_rmse = 0.0f, val_max = 0.0f;
     if (!val.empty()) {
@@ -2452,37 +2453,30 @@ p2v_status p2v_mlp_gradients(p2v_ctx* c, const float* x, const float* t, uint32_
     if (!c || !x || !t || !grad || n == 0 || !c->mlp_P.ptr)
         return P2V_EINVAL;
     cudaSetDevice(c->device);
-    const int nblk = (int) ((n + 31) / 32);
-    DevBuf dx, dt, di;
-    if (dx.ensure(sizeof(float) * (size_t) n * MLP_IN) != cudaSuccess || dt.ensure(sizeof(float) * n) != cudaSuccess ||
-        di.ensure(sizeof(uint32_t) * n) != cudaSuccess ||
-        c->mlp_part.ensure(sizeof(float) * (size_t) nblk * MLP_NPARAM) != cudaSuccess ||
-        c->mlp_ploss.ensure(sizeof(float) * nblk) != cudaSuccess) {
-        dx.release();
-        dt.release();
-        di.release();
+    // the pairs (features, then targets) and the result's pinned copy stay with the context, for the next call
+    const size_t xf = (size_t) n * MLP_IN;
+    if (c->mlp_gx.ensure(sizeof(float) * (xf + n)) != cudaSuccess ||
+        c->mlp_part.ensure(sizeof(float) * (size_t) mlp_train_blocks((int) n) * MLP_NPARAM) != cudaSuccess ||
+        c->mlp_ploss.ensure(sizeof(float) * mlp_train_blocks((int) n)) != cudaSuccess ||
+        (!c->mlp_gh && cudaMallocHost(&c->mlp_gh, sizeof(float) * (MLP_NPARAM + 1)) != cudaSuccess))
         return c->fail(P2V_ENOMEM, "gradient buffers");
-    }
-    std::vector<uint32_t> idx(n);
-    std::iota(idx.begin(), idx.end(), 0u);
-    cudaMemcpy(dx.ptr, x, sizeof(float) * (size_t) n * MLP_IN, cudaMemcpyHostToDevice);
-    cudaMemcpy(dt.ptr, t, sizeof(float) * n, cudaMemcpyHostToDevice);
-    cudaMemcpy(di.ptr, idx.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice);
-    cudaError_t e = launch_mlp_train_step(c->mlp_P.as<float>(), dx.as<float>(), dt.as<float>(), di.as<uint32_t>(),
-                                          (int) n, c->mlp_part.as<float>(), c->mlp_ploss.as<float>(),
-                                          c->mlp_g.as<float>(), c->mlp_loss.as<float>(), nullptr);
-    float l = 0.0f;
+    float* dx = c->mlp_gx.as<float>();
+    cudaStream_t st = c->own_stream;
+    cudaError_t e = cudaMemcpyAsync(dx, x, sizeof(float) * xf, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess)
-        e = cudaMemcpy(grad, c->mlp_g.ptr, sizeof(float) * MLP_NPARAM, cudaMemcpyDeviceToHost);
+        e = cudaMemcpyAsync(dx + xf, t, sizeof(float) * n, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess)
-        e = cudaMemcpy(&l, c->mlp_loss.ptr, sizeof(float), cudaMemcpyDeviceToHost);
-    dx.release();
-    dt.release();
-    di.release();
+        e = launch_mlp_train_step(c->mlp_P.as<float>(), dx, dx + xf, nullptr, (int) n, c->mlp_part.as<float>(),
+                                  c->mlp_ploss.as<float>(), c->mlp_g.as<float>(), st);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(c->mlp_gh, c->mlp_g.ptr, sizeof(float) * (MLP_NPARAM + 1), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess)
+        e = cudaStreamSynchronize(st);
     if (e != cudaSuccess)
         return c->fail(P2V_ECUDA, "gradients: %s", cudaGetErrorString(e));
+    std::memcpy(grad, c->mlp_gh, sizeof(float) * MLP_NPARAM);
     if (loss)
-        *loss = l / (float) n;
+        *loss = c->mlp_gh[MLP_NPARAM] / (float) n;
     return P2V_OK;
 }
 

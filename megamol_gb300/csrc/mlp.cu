@@ -166,147 +166,228 @@ __global__ void __launch_bounds__(128) mlp_collect_kernel(const ConeParams cp, c
 // ---------------------------------------------------------------------------------------------
 // training: forward + backward of TS samples per CTA, FP32; per-CTA gradient partials
 // ---------------------------------------------------------------------------------------------
-constexpr int TS = 32;
+// Bound by latency (2048 samples are 0.1 GFLOP): 16 samples per CTA fill the SMs at the default batch, and every product
+// runs on register tiles (4 samples per thread in the forward and backward passes, 4 x 4 parameters in the gradients),
+// its operands as 16-byte shared-memory reads of rows that are stored in the order they are read in. 2048 samples: 22 us;
+// 32 samples per CTA with two scalar shared-memory reads per multiply-add took 36.
+constexpr int TS = 16;
 constexpr int TT = 256;
+constexpr int XP = 64;            // padded feature count (zeros past MLP_IN)
+constexpr int WP = MLP_H + 1;     // row pitch of the transposed weights (conflict-free transposing stores)
 
-__global__ void __launch_bounds__(TT) mlp_train_kernel(const float* __restrict__ P, const float* __restrict__ X,
-    const float* __restrict__ T, const uint32_t* __restrict__ idx, int nbatch, float inv_batch,
-    float* __restrict__ partial, float* __restrict__ partial_loss) {
-    extern __shared__ __align__(16) float sh[];
-    float* W1 = sh;                          // [H][IN]
-    float* W2 = W1 + MLP_H * MLP_IN;         // [H][H]
-    float* Xs = W2 + MLP_H * MLP_H;          // [TS][IN]
-    float* A1 = Xs + TS * MLP_IN;            // [TS][H]
-    float* H1 = A1 + TS * MLP_H;
-    float* A2 = H1 + TS * MLP_H;
-    float* H2 = A2 + TS * MLP_H;
-    float* D2 = H2 + TS * MLP_H;             // dL/dA2
-    float* D1 = D2 + TS * MLP_H;             // dL/dA1
-    float* dz = D1 + TS * MLP_H;             // [TS]
-    const float* b1 = P + OFF_B1;
-    const float* b2 = P + OFF_B2;
-    const float* w3 = P + OFF_W3;
-    const int t = threadIdx.x;
-    const int s0 = blockIdx.x * TS;
-    const int ns = min(TS, nbatch - s0);
-    for (int k = t; k < MLP_H * MLP_IN; k += TT)
-        W1[k] = P[OFF_W1 + k];
-    for (int k = t; k < MLP_H * MLP_H; k += TT)
-        W2[k] = P[OFF_W2 + k];
-    for (int k = t; k < TS * MLP_IN; k += TT) {
-        const int s = k / MLP_IN, i = k % MLP_IN;
-        Xs[k] = s < ns ? X[(size_t) idx[s0 + s] * MLP_IN + i] : 0.0f;
-    }
-    __syncthreads();
-    for (int o = t; o < TS * MLP_H; o += TT) {
-        const int s = o / MLP_H, j = o % MLP_H;
-        float a = b1[j];
-        for (int i = 0; i < MLP_IN; ++i)
-            a = fmaf(W1[j * MLP_IN + i], Xs[s * MLP_IN + i], a);
-        A1[o] = a;
-        H1[o] = silu(a);
-    }
-    __syncthreads();
-    for (int o = t; o < TS * MLP_H; o += TT) {
-        const int s = o / MLP_H, j = o % MLP_H;
-        float a = b2[j];
-        for (int i = 0; i < MLP_H; ++i)
-            a = fmaf(W2[j * MLP_H + i], H1[s * MLP_H + i], a);
-        A2[o] = a;
-        H2[o] = silu(a);
-    }
-    __syncthreads();
-    if (t < TS) {
-        float l = 0.0f, d = 0.0f;
-        if (t < ns) {
-            float z = P[OFF_B3];
-            for (int j = 0; j < MLP_H; ++j)
-                z = fmaf(w3[j], H2[t * MLP_H + j], z);
-            const float y = sigmoidf_(z);
-            const float e = y - T[idx[s0 + t]];
-            l = e * e;
-            d = 2.0f * e * inv_batch * y * (1.0f - y);
-        }
-        dz[t] = d;
-        // loss partial of this CTA (fixed-order warp reduction)
-        for (int off = 16; off > 0; off >>= 1)
-            l += __shfl_xor_sync(0xffffffffu, l, off);
-        if (t == 0)
-            partial_loss[blockIdx.x] = l;
-    }
-    __syncthreads();
-    float* G = partial + (size_t) blockIdx.x * MLP_NPARAM;
-    for (int o = t; o < TS * MLP_H; o += TT) {
-        const int s = o / MLP_H, j = o % MLP_H;
-        const float a = A2[o];
-        const float sg = sigmoidf_(a);
-        D2[o] = dz[s] * w3[j] * sg * (1.0f + a * (1.0f - sg));
-    }
-    if (t < MLP_H) {
-        float g = 0.0f;
-        for (int s = 0; s < TS; ++s)
-            g = fmaf(dz[s], H2[s * MLP_H + t], g);
-        G[OFF_W3 + t] = g;
-    } else if (t == MLP_H) {
-        float g = 0.0f;
-        for (int s = 0; s < TS; ++s)
-            g += dz[s];
-        G[OFF_B3] = g;
-    }
-    __syncthreads();
-    for (int o = t; o < MLP_H * MLP_H; o += TT) {
-        const int j = o / MLP_H, i = o % MLP_H;
-        float g = 0.0f;
-        for (int s = 0; s < TS; ++s)
-            g = fmaf(D2[s * MLP_H + j], H1[s * MLP_H + i], g);
-        G[OFF_W2 + o] = g;
-    }
-    if (t < MLP_H) {
-        float g = 0.0f;
-        for (int s = 0; s < TS; ++s)
-            g += D2[s * MLP_H + t];
-        G[OFF_B2 + t] = g;
-    }
-    for (int o = t; o < TS * MLP_H; o += TT) {
-        const int s = o / MLP_H, i = o % MLP_H;
-        float g = 0.0f;
-        for (int j = 0; j < MLP_H; ++j)
-            g = fmaf(D2[s * MLP_H + j], W2[j * MLP_H + i], g);
-        const float a = A1[o];
-        const float sg = sigmoidf_(a);
-        D1[o] = g * sg * (1.0f + a * (1.0f - sg));
-    }
-    __syncthreads();
-    for (int o = t; o < MLP_H * MLP_IN; o += TT) {
-        const int j = o / MLP_IN, i = o % MLP_IN;
-        float g = 0.0f;
-        for (int s = 0; s < TS; ++s)
-            g = fmaf(D1[s * MLP_H + j], Xs[s * MLP_IN + i], g);
-        G[OFF_W1 + o] = g;
-    }
-    if (t < MLP_H) {
-        float g = 0.0f;
-        for (int s = 0; s < TS; ++s)
-            g += D1[s * MLP_H + t];
-        G[OFF_B1 + t] = g;
+struct TrainShared {  // every array 16-byte aligned
+    alignas(16) float w1t[MLP_IN * WP];     // W1^T: [feature][neuron]
+    alignas(16) float w2t[MLP_H * WP];      // W2^T: [input][neuron]
+    alignas(16) float w2[MLP_H * MLP_H];    // [neuron][input]
+    alignas(16) float x[TS * XP];           // features by sample
+    alignas(16) float xt[MLP_IN * TS];      // and by feature
+    alignas(16) float h1[TS * MLP_H];       // first layer's activations by sample
+    alignas(16) float h1t[MLP_H * TS];      // and by neuron
+    alignas(16) float a1[MLP_H * TS];       // its pre-activations by neuron
+    alignas(16) float d2[TS * MLP_H];       // dL/dA2 by sample
+    alignas(16) float d2t[MLP_H * TS];      // and by neuron
+    alignas(16) float d1[TS * MLP_H];       // dL/dA1
+    alignas(16) float h2[TS * MLP_H];
+    alignas(16) float zp[2 * TS];           // halves of the last layer's sums
+    float dz[TS], loss[TS];
+};
+
+__device__ __forceinline__ void fma4(float (&acc)[4], float w, const float4 v) {
+    acc[0] = fmaf(w, v.x, acc[0]);
+    acc[1] = fmaf(w, v.y, acc[1]);
+    acc[2] = fmaf(w, v.z, acc[2]);
+    acc[3] = fmaf(w, v.w, acc[3]);
+}
+
+// sum over the CTA's samples of da[s][j0 + r] db[s][i0 + c], a 4 x 4 tile of a weight gradient
+template<int PB>
+__device__ __forceinline__ void grad_tile(const float* da, const float* db, int j0, int i0, float (&g)[4][4]) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            g[r][c] = 0.0f;
+#pragma unroll
+    for (int s = 0; s < TS; ++s) {
+        const float4 a = *reinterpret_cast<const float4*>(da + s * MLP_H + j0);
+        const float4 b = *reinterpret_cast<const float4*>(db + s * PB + i0);
+        fma4(g[0], a.x, b);
+        fma4(g[1], a.y, b);
+        fma4(g[2], a.z, b);
+        fma4(g[3], a.w, b);
     }
 }
 
-// gradient = sum of the CTA partials in CTA order (deterministic)
-__global__ void __launch_bounds__(256) mlp_reduce_kernel(const float* __restrict__ partial, int nblk,
-    const float* __restrict__ partial_loss, float* __restrict__ grad, float* __restrict__ loss) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < MLP_NPARAM) {
-        float g = 0.0f;
-        for (int b = 0; b < nblk; ++b)
-            g += partial[(size_t) b * MLP_NPARAM + p];
-        grad[p] = g;
+__device__ __forceinline__ void put(float* p, float v, bool add) {
+    *p = add ? *p + v : v;
+}
+
+// idx: the batch's pairs (null: the first nbatch rows)
+__global__ void __launch_bounds__(TT) mlp_train_kernel(const float* __restrict__ P, const float* __restrict__ X,
+    const float* __restrict__ T, const uint32_t* __restrict__ idx, int nbatch, float inv_batch,
+    float* __restrict__ partial, float* __restrict__ partial_loss) {
+    extern __shared__ __align__(16) unsigned char train_smem[];
+    TrainShared& S = *reinterpret_cast<TrainShared*>(train_smem);
+    const int t = threadIdx.x;
+    for (int k = t; k < MLP_H * MLP_IN; k += TT)
+        S.w1t[(k % MLP_IN) * WP + k / MLP_IN] = P[OFF_W1 + k];
+    for (int k = t; k < MLP_H * MLP_H; k += TT) {
+        const float v = P[OFF_W2 + k];
+        S.w2[k] = v;
+        S.w2t[(k % MLP_H) * WP + k / MLP_H] = v;
     }
-    if (p == 0) {
-        float l = 0.0f;
-        for (int b = 0; b < nblk; ++b)
-            l += partial_loss[b];
-        *loss = l;
+    // thread t: neuron (or input) j of the four samples sq .. sq + 3
+    const int j = t % MLP_H, sq = 4 * (t / MLP_H);
+    const float b1 = P[OFF_B1 + j], b2 = P[OFF_B2 + j], w3 = P[OFF_W3 + j], b3 = P[OFF_B3];
+    float* G = partial + (size_t) blockIdx.x * MLP_NPARAM;
+    float loss_sum = 0.0f;
+    // groups of TS samples; the CTA's partials are written by its first and added to by the others
+    for (int s0 = blockIdx.x * TS; s0 < nbatch; s0 += gridDim.x * TS) {
+        const bool more = s0 != (int) blockIdx.x * TS;
+        const int ns = min(TS, nbatch - s0);
+        __syncthreads();  // the previous group's arrays are read
+        for (int k = t; k < TS * XP; k += TT) {
+            const int s = k / XP, i = k % XP;
+            float v = 0.0f;
+            if (s < ns && i < MLP_IN)
+                v = X[(size_t) (idx ? idx[s0 + s] : (uint32_t) (s0 + s)) * MLP_IN + i];
+            S.x[k] = v;
+            if (i < MLP_IN)
+                S.xt[i * TS + s] = v;
+        }
+        float acc[4];
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            acc[e] = b1;
+#pragma unroll 6
+        for (int i = 0; i < MLP_IN; ++i)
+            fma4(acc, S.w1t[i * WP + j], *reinterpret_cast<const float4*>(S.xt + i * TS + sq));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float h = silu(acc[e]);
+            S.a1[j * TS + sq + e] = acc[e];
+            S.h1[(sq + e) * MLP_H + j] = h;
+            S.h1t[j * TS + sq + e] = h;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            acc[e] = b2;
+#pragma unroll 8
+        for (int i = 0; i < MLP_H; ++i)
+            fma4(acc, S.w2t[i * WP + j], *reinterpret_cast<const float4*>(S.h1t + i * TS + sq));
+        // the last layer's sum over j: a warp holds half the neurons of four samples
+        float z[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float h = silu(acc[e]);
+            S.h2[(sq + e) * MLP_H + j] = h;
+            z[e] = w3 * h;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                z[e] += __shfl_xor_sync(0xffffffffu, z[e], o);
+        if (t % 32 == 0)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                S.zp[(t / 32) * 4 + e] = z[e];  // [sample quad][half][e]
+        __syncthreads();
+        if (t < TS) {
+            float l = 0.0f, d = 0.0f;
+            if (t < ns) {
+                const int q = t / 4, e = t % 4;
+                const float y = sigmoidf_(b3 + (S.zp[8 * q + e] + S.zp[8 * q + 4 + e]));
+                const float err = y - T[idx ? idx[s0 + t] : (uint32_t) (s0 + t)];
+                l = err * err;
+                d = 2.0f * err * inv_batch * y * (1.0f - y);
+            }
+            S.dz[t] = d;
+            S.loss[t] = l;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float a = acc[e], sg = sigmoidf_(a);
+            const float d = S.dz[sq + e] * w3 * sg * (1.0f + a * (1.0f - sg));
+            S.d2[(sq + e) * MLP_H + j] = d;
+            S.d2t[j * TS + sq + e] = d;
+        }
+        if (t == 0) {
+            float l = 0.0f, g = 0.0f;
+            for (int s = 0; s < TS; ++s) {
+                l += S.loss[s];
+                g += S.dz[s];
+            }
+            loss_sum += l;
+            put(G + OFF_B3, g, more);
+        }
+        __syncthreads();
+        // dL/dA1 of input j
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            acc[e] = 0.0f;
+#pragma unroll 8
+        for (int i = 0; i < MLP_H; ++i)
+            fma4(acc, S.w2[i * MLP_H + j], *reinterpret_cast<const float4*>(S.d2t + i * TS + sq));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float a = S.a1[j * TS + sq + e], sg = sigmoidf_(a);
+            S.d1[(sq + e) * MLP_H + j] = acc[e] * sg * (1.0f + a * (1.0f - sg));
+        }
+        const int j0 = 4 * (t / 16), i0 = 4 * (t % 16);
+        float g[4][4];
+        grad_tile<MLP_H>(S.d2, S.h1, j0, i0, g);
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                put(G + OFF_W2 + (j0 + r) * MLP_H + i0 + c, g[r][c], more);
+        __syncthreads();
+        grad_tile<XP>(S.d1, S.x, j0, i0, g);
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (i0 + c < MLP_IN)
+                    put(G + OFF_W1 + (j0 + r) * MLP_IN + i0 + c, g[r][c], more);
+        if (t < 3 * MLP_H) {  // the biases' gradients and the last layer's weights'
+            const int k = t % MLP_H, what = t / MLP_H;
+            float v = 0.0f;
+#pragma unroll
+            for (int s = 0; s < TS; ++s)
+                v = what == 0 ? v + S.d1[s * MLP_H + k] : what == 1 ? v + S.d2[s * MLP_H + k]
+                                                                  : fmaf(S.dz[s], S.h2[s * MLP_H + k], v);
+            put(G + (what == 0 ? OFF_B1 : what == 1 ? OFF_B2 : OFF_W3) + k, v, more);
+        }
+    }
+    if (t == 0)
+        partial_loss[blockIdx.x] = loss_sum;
+}
+
+// gradient = sum of the CTA partials in a fixed order (deterministic): a block takes 32 parameters, its 8 warps an
+// eighth of the partials each, added up in warp order. The loss follows the gradient (grad[MLP_NPARAM]).
+__global__ void __launch_bounds__(256) mlp_reduce_kernel(const float* __restrict__ partial, int nblk,
+    const float* __restrict__ partial_loss, float* __restrict__ grad) {
+    __shared__ float s_g[8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int p = blockIdx.x * 32 + lane;
+    const int per = (nblk + 7) / 8, b0 = min(w * per, nblk), b1 = min(b0 + per, nblk);
+    const bool is_loss = p == MLP_NPARAM;
+    float g = 0.0f;
+    if (p <= MLP_NPARAM) {
+#pragma unroll 8
+        for (int b = b0; b < b1; ++b)
+            g += is_loss ? partial_loss[b] : partial[(size_t) b * MLP_NPARAM + p];
+    }
+    s_g[w][lane] = g;
+    __syncthreads();
+    if (w == 0 && p <= MLP_NPARAM) {
+        for (int k = 1; k < 8; ++k)
+            g += s_g[k][lane];
+        grad[p] = g;
     }
 }
 
@@ -802,8 +883,8 @@ __global__ void __launch_bounds__(tc::THREADS, tc::CTAS) mlp_infer_tc_kernel(con
 
 }  // namespace
 
-size_t mlp_train_smem_bytes() {
-    return sizeof(float) * (MLP_H * MLP_IN + MLP_H * MLP_H + TS * MLP_IN + 6 * TS * MLP_H + TS);
+int mlp_train_blocks(int nbatch) {
+    return std::min((nbatch + TS - 1) / TS, 304);  // two CTAs (83 KB of shared memory each) on each of 152 SMs
 }
 
 cudaError_t FeatureTex::ensure(const int dims[3]) {
@@ -871,14 +952,14 @@ cudaError_t launch_mlp_collect(const ConeParams& cp, const uint32_t* order, cons
 }
 
 cudaError_t launch_mlp_train_step(const float* P, const float* X, const float* T, const uint32_t* idx, int nbatch,
-    float* partial, float* partial_loss, float* grad, float* loss, cudaStream_t st) {
-    const int nblk = (nbatch + TS - 1) / TS;
-    const size_t smem = mlp_train_smem_bytes();
-    cudaError_t e = cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    float* partial, float* partial_loss, float* grad, cudaStream_t st) {
+    const int nblk = mlp_train_blocks(nbatch);
+    constexpr int smem = (int) sizeof(TrainShared);
+    cudaError_t e = cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess)
         return e;
     mlp_train_kernel<<<nblk, TT, smem, st>>>(P, X, T, idx, nbatch, 1.0f / (float) nbatch, partial, partial_loss);
-    mlp_reduce_kernel<<<ceil_div(MLP_NPARAM, 256), 256, 0, st>>>(partial, nblk, partial_loss, grad, loss);
+    mlp_reduce_kernel<<<(MLP_NPARAM + 32) / 32, 256, 0, st>>>(partial, nblk, partial_loss, grad);
     return cudaGetLastError();
 }
 

@@ -75,12 +75,15 @@ struct FeatureTex {
 // copy level L (level-0 saturation `sat` applied when > 0) into the texture
 cudaError_t launch_fill_feature_tex(const ConeLevel& L, float sat, const FeatureTex& t, cudaStream_t st);
 
-size_t mlp_train_smem_bytes();
+// CTAs (gradient partials of MLP_NPARAM floats, loss partials) of a batch
+int mlp_train_blocks(int nbatch);
 // xyzr, nrm in sorted order (sel holds sorted positions), ao in input order (order: sorted position -> index)
 cudaError_t launch_mlp_collect(const ConeParams& cp, const uint32_t* order, const uint32_t* sel, uint32_t nsel,
     const float4* xyzr, const float4* nrm, const float* ao, float* X, float* T, uint32_t* kept, cudaStream_t st);
+// the gradient of the batch's mean squared error (rows idx, null: the first nbatch), and after it the summed loss:
+// grad has MLP_NPARAM + 1 floats
 cudaError_t launch_mlp_train_step(const float* P, const float* X, const float* T, const uint32_t* idx, int nbatch,
-    float* partial, float* partial_loss, float* grad, float* loss, cudaStream_t st);
+    float* partial, float* partial_loss, float* grad, cudaStream_t st);
 cudaError_t launch_mlp_adam(float* P, const float* g, float* m, float* v, float lr, float b1, float b2, float eps,
     int step, cudaStream_t st);
 cudaError_t launch_mlp_forward_f32(const float* P, const float* X, const uint32_t* idx, uint32_t n, float* y,
