@@ -44,6 +44,7 @@ __device__ __forceinline__ float intensity_of(const uint8_t* rec, int ctype, flo
 template<int NC>
 __global__ void __launch_bounds__(256) pack_weights_kernel(WeightSource src, float* __restrict__ w,
                                                            FrameScalars* __restrict__ fs) {
+    chain_begin();
     __shared__ uint32_t s_max[8];
     uint32_t mbits = 0u;
     const uint64_t step = (uint64_t) gridDim.x * blockDim.x;
@@ -82,6 +83,7 @@ __global__ void __launch_bounds__(256) pack_weights_kernel(WeightSource src, flo
 __global__ void __launch_bounds__(256) permute_weights_kernel(const uint32_t* __restrict__ order,
                                                               const float* __restrict__ win, float* __restrict__ wout,
                                                               uint32_t n, int nc) {
+    chain_begin();
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
         const uint32_t o = order[j];
         for (int c = 0; c < nc; ++c)
@@ -96,6 +98,7 @@ __global__ void __launch_bounds__(256) permute_weights_kernel(const uint32_t* __
 __global__ void __launch_bounds__(256) vector_finish_kernel(float* __restrict__ vol3, const float* __restrict__ wsum,
                                                             int64_t V, FrameScalars* __restrict__ fs,
                                                             VectorGridBufs vg) {
+    chain_begin();
     __shared__ uint32_t s_lo[8], s_hi[8], s_nz[8];
     uint32_t lo = 0x7f7fffffu, hi = 0u, nz = 0u;
     for (int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < V; i += (int64_t) gridDim.x * blockDim.x) {
@@ -196,6 +199,7 @@ __global__ void __launch_bounds__(256) vector_grid_kernel(const uint32_t* __rest
 // ParticlesToDensity.cpp:669-682 with the densities' range: every component maps by (a - min) * (1 /
 // (max - min)) when normalising; the published range is the densities'.
 __global__ void vector_range_kernel(FrameScalars* fs, int minmax_normalize) {
+    chain_begin();
     const float mn = __uint_as_float(fs->dmin_bits), mx = __uint_as_float(fs->dmax_bits);
     fs->vmin = mn;
     fs->vmax = mx;
@@ -220,9 +224,9 @@ cudaError_t launch_pack_weights(const WeightSource& src, int nc, float* w, Frame
         return cudaSuccess;
     const unsigned grd = (unsigned) std::max<uint64_t>(1, std::min<uint64_t>((src.count + 1023) / 1024, (uint64_t) sms * 8));
     if (nc == 1)
-        pack_weights_kernel<1><<<grd, 256, 0, st>>>(src, w, fs);
+        chain(pack_weights_kernel<1>, grd, 256, 0, st, src, w, fs);
     else
-        pack_weights_kernel<3><<<grd, 256, 0, st>>>(src, w, fs);
+        chain(pack_weights_kernel<3>, grd, 256, 0, st, src, w, fs);
     return cudaGetLastError();
 }
 
@@ -231,15 +235,15 @@ cudaError_t launch_permute_weights(const uint32_t* order, const float* win, floa
     if (n == 0)
         return cudaSuccess;
     const unsigned grd = (unsigned) std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(n, 256), (uint32_t) sms * 16));
-    permute_weights_kernel<<<grd, 256, 0, st>>>(order, win, wout, n, nc);
+    chain(permute_weights_kernel, grd, 256, 0, st, order, win, wout, n, nc);
     return cudaGetLastError();
 }
 
 cudaError_t launch_vector_finish(float* vol3, const float* wsum, int64_t V, FrameScalars* fs, int minmax_normalize,
                                  int sms, cudaStream_t st, const VectorGridBufs* vg) {
     const unsigned grd = (unsigned) std::max<int64_t>(1, std::min<int64_t>((V + 255) / 256, (int64_t) sms * 16));
-    vector_finish_kernel<<<grd, 256, 0, st>>>(vol3, wsum, V, fs, vg ? *vg : VectorGridBufs{});
-    vector_range_kernel<<<1, 1, 0, st>>>(fs, minmax_normalize);
+    chain(vector_finish_kernel, grd, 256, 0, st, vol3, wsum, V, fs, vg ? *vg : VectorGridBufs{});
+    chain(vector_range_kernel, 1, 1, 0, st, fs, minmax_normalize);
     return cudaGetLastError();
 }
 

@@ -29,6 +29,7 @@ namespace {
 // volume holds fewer than 2^31 texels, so every level above level 0 fewer than 2^28).
 __global__ void __launch_bounds__(256) mip_level_r8_kernel(const float* __restrict__ src, int sx, int sy, int sz,
     float* __restrict__ dst, int dx, int dy, int dz, float sat_scale) {
+    chain_begin();
     const uint32_t n = (uint32_t) dx * (uint32_t) dy * (uint32_t) dz;
     const uint32_t pxy = (uint32_t) dx * (uint32_t) dy;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -52,6 +53,7 @@ template<bool NORMALIZE>
 __global__ void __launch_bounds__(256, 4) mip_rows_kernel(float* __restrict__ src, int sx, int sy, int sz,
     float* __restrict__ dst, int dx, int dy, int dz, float sat_scale, const FrameScalars* __restrict__ fs,
     int mass_normalize, int minmax_normalize) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const uint32_t ny = ((uint32_t) sy + 1u) / 2u, nz = ((uint32_t) sz + 1u) / 2u, total = ny * nz;
     float ms = 1.0f, off = 0.0f, sc = 1.0f;
@@ -122,6 +124,7 @@ __global__ void __launch_bounds__(256, 4) mip_rows_kernel(float* __restrict__ sr
 __global__ void __launch_bounds__(32 * MAX_CONES) cone_ao_list_kernel(const ConeParams cp,
     const uint32_t* __restrict__ list, const float4* __restrict__ xyzr, const float4* __restrict__ nrm, uint32_t n,
     const uint32_t* __restrict__ n_dev, const uint32_t* __restrict__ out_order, float* __restrict__ ao) {
+    chain_begin();
     __shared__ float s_acc[MAX_CONES];
     const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
     if (n_dev)
@@ -172,6 +175,7 @@ __global__ void __launch_bounds__(32 * MAX_CONES) cone_ao_list_kernel(const Cone
 __global__ void __launch_bounds__(256) sort_particles_kernel(const uint32_t* __restrict__ order, uint32_t n,
     const float4* __restrict__ xyzr, const float4* __restrict__ nrm, float4* __restrict__ xyzr_s,
     float4* __restrict__ nrm_s) {
+    chain_begin();
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
         const uint32_t o = order[j];
         if (xyzr)  // null: the binning's last pass wrote the sorted positions already
@@ -183,6 +187,7 @@ __global__ void __launch_bounds__(256) sort_particles_kernel(const uint32_t* __r
 // Unit normals down the density gradient (P2V_NORMALS_GRADIENT), one thread per particle.
 __global__ void __launch_bounds__(256) gradient_normals_kernel(const GridGeo geo, const float* __restrict__ grid,
     const float4* __restrict__ xyzr, uint32_t n, float4* __restrict__ nrm) {
+    chain_begin();
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n)
         return;
@@ -195,6 +200,7 @@ __global__ void __launch_bounds__(256) gradient_normals_kernel(const GridGeo geo
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) aosphere_deposit_kernel(const AOSphereParams ap, const float4* __restrict__ xyzr,
     uint32_t n, unsigned long long* __restrict__ acc) {
+    chain_begin();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
@@ -240,6 +246,7 @@ __global__ void __launch_bounds__(256) aosphere_deposit_kernel(const AOSpherePar
 
 __global__ void __launch_bounds__(256) fixed_to_float_kernel(const unsigned long long* __restrict__ acc, int64_t n,
     float* __restrict__ out) {
+    chain_begin();
     for (int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < n; i += (int64_t) gridDim.x * blockDim.x)
         out[i] = (float) ((double) acc[i] * 2.3283064365386963e-10);
 }
@@ -247,6 +254,7 @@ __global__ void __launch_bounds__(256) fixed_to_float_kernel(const unsigned long
 __global__ void __launch_bounds__(128) aosphere_ao_kernel(const AOSphereParams ap, const float* __restrict__ tex,
     const uint32_t* __restrict__ order, const float4* __restrict__ xyzr, const float4* __restrict__ nrm, uint32_t n,
     int mode, float* __restrict__ ao) {
+    chain_begin();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
@@ -290,6 +298,7 @@ __global__ void __launch_bounds__(128) aosphere_ao_kernel(const AOSphereParams a
 
 __global__ void __launch_bounds__(256) pack_normals_kernel(const uint8_t* __restrict__ src, uint32_t stride,
     uint64_t count, uint64_t offset, float4* __restrict__ nrm, int aligned) {
+    chain_begin();
     const uint64_t i = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x;
     if (i >= count)
         return;
@@ -338,6 +347,7 @@ constexpr int BSCAN_THREADS = 256, BSCAN_ITEMS = 16, BSCAN_TILE = BSCAN_THREADS 
 // segment counts, and the sum of every tile of BSCAN_TILE segments
 __global__ void __launch_bounds__(BSCAN_THREADS) brick_counts_kernel(const uint32_t* __restrict__ start, BrickGeo bg,
     uint32_t nseg, uint32_t* __restrict__ cnt, uint32_t* __restrict__ tsum) {
+    chain_begin();
     __shared__ uint32_t s_sum[BSCAN_THREADS / 32];
     uint32_t sum = 0;
     for (int e = 0; e < BSCAN_ITEMS; ++e) {
@@ -365,6 +375,7 @@ __global__ void __launch_bounds__(BSCAN_THREADS) brick_counts_kernel(const uint3
 
 // exclusive scan of the tile sums in place (one block)
 __global__ void __launch_bounds__(1024) brick_tile_scan_kernel(uint32_t* __restrict__ tsum, uint32_t ntiles) {
+    chain_begin();
     __shared__ uint32_t s_warp[32];
     __shared__ uint32_t s_carry;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -408,6 +419,7 @@ __global__ void __launch_bounds__(1024) brick_tile_scan_kernel(uint32_t* __restr
 // the segments' brick-order offsets in place of their counts: the tile's prefix + the scan inside the tile
 __global__ void __launch_bounds__(BSCAN_THREADS) brick_offsets_kernel(uint32_t nseg, uint32_t* __restrict__ cnt,
                                                                       const uint32_t* __restrict__ tsum) {
+    chain_begin();
     __shared__ uint32_t s_warp[BSCAN_THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     // this thread's segments: BSCAN_ITEMS consecutive ones, so that the in-tile scan is a thread-local run
@@ -446,6 +458,7 @@ __global__ void __launch_bounds__(256) brick_scatter_kernel(const uint32_t* __re
     const int4* __restrict__ rec_b, BrickGeo bg, uint32_t nbins, uint32_t n, const uint32_t* __restrict__ off,
     int3 s3, const float4* __restrict__ xyzr, const float4* __restrict__ nrm, const uint32_t* __restrict__ order,
     float4* __restrict__ xyzr_b, float4* __restrict__ nrm_b, uint32_t* __restrict__ order_b) {
+    chain_begin();
     const uint32_t nvalid = start[nbins];
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
         uint32_t d = j;
@@ -486,11 +499,11 @@ cudaError_t launch_brick_order(const BrickPlan& p, const GridGeo& g, const uint3
         return cudaSuccess;
     BrickGeo bg{p.nb[0], p.nb[1], p.nb[2], (p.nb[0] + 15) / 16, (p.nb[1] + 3) / 4};
     const uint32_t nseg = (uint32_t) p.nseg, ntiles = (uint32_t) p.ntiles;
-    brick_counts_kernel<<<ntiles, BSCAN_THREADS, 0, st>>>(start, bg, nseg, cnt, tsum);
-    brick_tile_scan_kernel<<<1, 1024, 0, st>>>(tsum, ntiles);
-    brick_offsets_kernel<<<ntiles, BSCAN_THREADS, 0, st>>>(nseg, cnt, tsum);
+    chain(brick_counts_kernel, ntiles, BSCAN_THREADS, 0, st, start, bg, nseg, cnt, tsum);
+    chain(brick_tile_scan_kernel, 1, 1024, 0, st, tsum, ntiles);
+    chain(brick_offsets_kernel, ntiles, BSCAN_THREADS, 0, st, nseg, cnt, tsum);
     const unsigned grd = (unsigned) std::max<uint32_t>(1u, std::min<uint32_t>(ceil_div(n, 256), (uint32_t) sms * 16));
-    brick_scatter_kernel<<<grd, 256, 0, st>>>(start, rec_b, bg, g.nbins, n, cnt, make_int3(g.s[0], g.s[1], g.s[2]),
+    chain(brick_scatter_kernel, grd, 256, 0, st, start, rec_b, bg, g.nbins, n, cnt, make_int3(g.s[0], g.s[1], g.s[2]),
                                               xyzr, nrm, order, xyzr_b, nrm_b, order_b);
     return cudaGetLastError();
 }
@@ -504,7 +517,7 @@ unsigned mip_rows_grid(const int sd[3], int sms) {
 
 cudaError_t launch_normalize_mip(float* grid, const int d0[3], const FrameScalars* fs, int mass_normalize,
     int minmax_normalize, float sat_scale, float* level1, int sms, cudaStream_t st) {
-    mip_rows_kernel<true><<<mip_rows_grid(d0, sms), 256, 0, st>>>(grid, d0[0], d0[1], d0[2], level1, max(1, d0[0] / 2),
+    chain(mip_rows_kernel<true>, mip_rows_grid(d0, sms), 256, 0, st, grid, d0[0], d0[1], d0[2], level1, max(1, d0[0] / 2),
         max(1, d0[1] / 2), max(1, d0[2] / 2), sat_scale, fs, mass_normalize, minmax_normalize);
     return cudaGetLastError();
 }
@@ -519,9 +532,9 @@ cudaError_t launch_mip_levels(const float* l0, const int d0[3], float sat_scale,
         if (l >= first && quantize) {
             const int64_t nv = (int64_t) dd[0] * dd[1] * dd[2];
             const unsigned grd = (unsigned) std::max<int64_t>(1, std::min<int64_t>((nv + 255) / 256, (int64_t) sms * 32));
-            mip_level_r8_kernel<<<grd, 256, 0, st>>>(src, sd[0], sd[1], sd[2], out[l], dd[0], dd[1], dd[2], sat);
+            chain(mip_level_r8_kernel, grd, 256, 0, st, src, sd[0], sd[1], sd[2], out[l], dd[0], dd[1], dd[2], sat);
         } else if (l >= first) {
-            mip_rows_kernel<false><<<mip_rows_grid(sd, sms), 256, 0, st>>>(const_cast<float*>(src), sd[0], sd[1], sd[2],
+            chain(mip_rows_kernel<false>, mip_rows_grid(sd, sms), 256, 0, st, const_cast<float*>(src), sd[0], sd[1], sd[2],
                 out[l], dd[0], dd[1], dd[2], sat, nullptr, 0, 0);
         }
         src = out[l];
@@ -537,7 +550,7 @@ cudaError_t launch_cone_ao_warp(const ConeParams& cp, const float4* xyzr, const 
         return cudaSuccess;
     const int threads = 32 * cp.ncones;
     const unsigned grd = (unsigned) std::min<uint64_t>(n, (uint64_t) sms * std::max(1, 2048 / threads));
-    cone_ao_list_kernel<<<grd, threads, 0, st>>>(cp, nullptr, xyzr, nrm, n, nullptr, out_order, ao);
+    chain(cone_ao_list_kernel, grd, threads, 0, st, cp, nullptr, xyzr, nrm, n, nullptr, out_order, ao);
     return cudaGetLastError();
 }
 
@@ -547,7 +560,7 @@ cudaError_t launch_cone_ao_list(const ConeParams& cp, const uint32_t* list, cons
         return cudaSuccess;
     // one block of ncones warps per particle, a bounded grid
     const unsigned grd = (unsigned) std::min<uint32_t>(n, 4096u);
-    cone_ao_list_kernel<<<grd, 32 * cp.ncones, 0, st>>>(cp, list, xyzr, nrm, n, n_dev, out_order, ao);
+    chain(cone_ao_list_kernel, grd, 32 * cp.ncones, 0, st, cp, list, xyzr, nrm, n, n_dev, out_order, ao);
     return cudaGetLastError();
 }
 
@@ -558,11 +571,11 @@ cudaError_t launch_aosphere(const AOSphereParams& ap, const float4* xyzr, uint32
     if (e != cudaSuccess)
         return e;
     if (n > 0)
-        aosphere_deposit_kernel<<<ceil_div(n, 256), 256, 0, st>>>(ap, xyzr, n, acc);
+        chain(aosphere_deposit_kernel, ceil_div(n, 256), 256, 0, st, ap, xyzr, n, acc);
     const unsigned grd = (unsigned) std::max<int64_t>(1, std::min<int64_t>((nv + 255) / 256, (int64_t) sms * 16));
-    fixed_to_float_kernel<<<grd, 256, 0, st>>>(acc, nv, tex);
+    chain(fixed_to_float_kernel, grd, 256, 0, st, acc, nv, tex);
     if (n > 0)
-        aosphere_ao_kernel<<<ceil_div(n, 128), 128, 0, st>>>(ap, tex, order, xyzr, nrm, n, mode, ao);
+        chain(aosphere_ao_kernel, ceil_div(n, 128), 128, 0, st, ap, tex, order, xyzr, nrm, n, mode, ao);
     return cudaGetLastError();
 }
 
@@ -571,7 +584,7 @@ cudaError_t launch_sort_particles(const uint32_t* order, uint32_t n, const float
     if (n == 0)
         return cudaSuccess;
     const unsigned grd = (unsigned) std::max<uint32_t>(1u, std::min<uint32_t>(ceil_div(n, 256), (uint32_t) sms * 16));
-    sort_particles_kernel<<<grd, 256, 0, st>>>(order, n, xyzr, nrm, xyzr_s, nrm_s);
+    chain(sort_particles_kernel, grd, 256, 0, st, order, n, xyzr, nrm, xyzr_s, nrm_s);
     return cudaGetLastError();
 }
 
@@ -579,7 +592,7 @@ cudaError_t launch_gradient_normals(const GridGeo& geo, const float* grid, const
                                     cudaStream_t st) {
     if (n == 0)
         return cudaSuccess;
-    gradient_normals_kernel<<<ceil_div(n, 256), 256, 0, st>>>(geo, grid, xyzr, n, nrm);
+    chain(gradient_normals_kernel, ceil_div(n, 256), 256, 0, st, geo, grid, xyzr, n, nrm);
     return cudaGetLastError();
 }
 
@@ -588,7 +601,7 @@ cudaError_t launch_pack_normals(const void* src, uint32_t stride, uint64_t count
     if (count == 0)
         return cudaSuccess;
     const int aligned = (reinterpret_cast<uintptr_t>(src) % 4 == 0) && (stride % 4 == 0);
-    pack_normals_kernel<<<(unsigned) ((count + 255) / 256), 256, 0, st>>>(static_cast<const uint8_t*>(src), stride,
+    chain(pack_normals_kernel, (unsigned) ((count + 255) / 256), 256, 0, st, static_cast<const uint8_t*>(src), stride,
                                                                          count, offset, nrm, aligned);
     return cudaGetLastError();
 }

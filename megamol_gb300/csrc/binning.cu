@@ -87,6 +87,7 @@ template<class T, int NC, bool ALIGNED>
 __global__ void __launch_bounds__(256) pack_keys_kernel(ListDesc L, GridGeo g, float4* __restrict__ xyzr,
     uint32_t* __restrict__ keys, uint32_t* __restrict__ counts, uint32_t* __restrict__ rank,
     FrameScalars* __restrict__ fs, uint32_t empty_flag) {
+    chain_begin();
     __shared__ int32_t s_cmin[3][8], s_cmax[3][8];
     __shared__ uint32_t s_rmax[8], s_drop[8];
     int32_t cell[3] = {INT32_MAX, INT32_MAX, INT32_MAX};
@@ -316,6 +317,7 @@ __device__ __forceinline__ void radix_hist(const uint32_t* __restrict__ keys, ui
 
 __global__ void __launch_bounds__(256) radix_hist_kernel(const uint32_t* __restrict__ keys, uint32_t n, SortPlan pl,
     uint32_t* __restrict__ hist, uint32_t* __restrict__ done, uint32_t* __restrict__ status, uint64_t status_words) {
+    chain_begin();
     radix_hist(keys, n, pl, hist, done, status, status_words, gridDim.x);
 }
 
@@ -342,6 +344,7 @@ __global__ void __launch_bounds__(SORT_THREADS, 3) onesweep_kernel(const uint32_
     uint32_t* __restrict__ status, uint32_t* __restrict__ err, const float4* __restrict__ xyzr_in,
     float4* __restrict__ rec_a, int4* __restrict__ rec_b, float4* __restrict__ xyzr_out, GridGeo geo,
     const FrameScalars* __restrict__ gate, uint32_t wait_polls, int32_t hold_tile) {
+    chain_begin();
     if (radix_skipped(gate) || (ld_volatile(err) & ERR_LOOKBACK_TIMEOUT))
         return;
     constexpr int RADIX = 1 << BITS;
@@ -567,6 +570,7 @@ constexpr uint32_t RUN_MAX = 8192;
 __global__ void __launch_bounds__(256) boundary_starts_kernel(uint32_t* __restrict__ keys,
     uint32_t* __restrict__ vals, uint32_t n, uint32_t nbins, uint32_t* __restrict__ out, uint4* __restrict__ gaps, uint32_t gap_cap,
     FrameScalars* __restrict__ fs, const FrameScalars* __restrict__ gate) {
+    chain_begin();
     if (radix_skipped(gate))
         return;
     const bool failed = (ld_volatile(&fs->error) & ERR_LOOKBACK_TIMEOUT) != 0u;
@@ -635,6 +639,7 @@ __global__ void __launch_bounds__(256) boundary_starts_kernel(uint32_t* __restri
 
 __global__ void __launch_bounds__(256) cell_gap_fill_kernel(const uint4* __restrict__ gaps, uint32_t gap_cap,
     uint32_t* __restrict__ start, const FrameScalars* __restrict__ fs, const FrameScalars* __restrict__ gate) {
+    chain_begin();
     if (radix_skipped(gate))
         return;
     const uint32_t ng = min(fs->ngaps, gap_cap);
@@ -674,6 +679,7 @@ __device__ __forceinline__ bool load_counts(const uint32_t* __restrict__ counts,
 // Step 1: the sum of every tile of SCAN_TILE counts, and the largest count (fs->bin_maxcount).
 __global__ void __launch_bounds__(SCAN_THREADS) bin_tile_sums_kernel(const uint32_t* __restrict__ counts, uint32_t nb,
     uint32_t* __restrict__ tsum, FrameScalars* __restrict__ fs) {
+    chain_begin();
     __shared__ uint32_t s_sum[SCAN_THREADS / 32], s_max[SCAN_THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     uint32_t v[SCAN_ITEMS];
@@ -710,6 +716,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) bin_tile_sums_kernel(const uint3
 __global__ void __launch_bounds__(SCAN_THREADS) bin_starts_kernel(const uint32_t* __restrict__ counts, uint32_t nb,
     const uint32_t* __restrict__ tsum, uint32_t* __restrict__ start, uint32_t* __restrict__ multi,
     FrameScalars* __restrict__ fs) {
+    chain_begin();
     __shared__ uint32_t s_warp[SCAN_THREADS / 32], s_before[SCAN_THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     uint32_t before = 0;
@@ -781,6 +788,7 @@ __global__ void __launch_bounds__(256) scatter_bins_kernel(const uint32_t* __res
     const uint32_t* __restrict__ rank, const float4* __restrict__ xyzr, uint32_t n,
     const uint32_t* __restrict__ start, uint32_t* __restrict__ vals_out, float4* __restrict__ rec_a,
     int4* __restrict__ rec_b, float4* __restrict__ xyzr_out, GridGeo geo, const FrameScalars* __restrict__ fs) {
+    chain_begin();
     if (fs->bin_maxcount > BIN_CELL_MAX)
         return;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -806,6 +814,7 @@ __global__ void __launch_bounds__(256) order_bins_kernel(const uint32_t* __restr
     uint32_t* __restrict__ vals, const uint32_t* __restrict__ start, const float4* __restrict__ xyzr,
     float4* __restrict__ rec_a, int4* __restrict__ rec_b, float4* __restrict__ xyzr_out, GridGeo geo,
     const FrameScalars* __restrict__ fs) {
+    chain_begin();
     if (fs->bin_maxcount > BIN_CELL_MAX) {
         radix_hist(keys, n, pl, hist, done, status, status_words, hist_blocks);
         return;
@@ -855,6 +864,7 @@ __global__ void __launch_bounds__(256) keys_from_starts_kernel(const uint32_t* _
 // histograms and counters.
 __global__ void __launch_bounds__(256) init_frame_kernel(FrameScalars* fs, uint4* __restrict__ counts, uint64_t ncounts4,
                                                          uint32_t* __restrict__ hist, uint32_t hist_words) {
+    chain_begin();
     const uint64_t t = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x, step = (uint64_t) gridDim.x * blockDim.x;
     for (uint64_t i = t; i < ncounts4; i += step)
         counts[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -872,6 +882,7 @@ __global__ void __launch_bounds__(256) init_frame_kernel(FrameScalars* fs, uint4
 }
 
 __global__ void count_valid_kernel(const uint32_t* __restrict__ start, uint32_t nbins, FrameScalars* fs) {
+    chain_begin();
     fs->n_valid = start[nbins];
 }
 
@@ -892,30 +903,30 @@ cudaError_t launch_pack_keys(const ListDesc& L, const GridGeo& g, float4* xyzr, 
     case 1: {  // FLOAT_XYZ
         bool al = (addr % 4 == 0) && (L.stride % 4 == 0);
         if (al)
-            pack_keys_kernel<float, 3, true><<<grid, block, 0, st>>>(L, g, xyzr, keys, counts, rank, fs, empty_flag);
+            chain(pack_keys_kernel<float, 3, true>, grid, block, 0, st, L, g, xyzr, keys, counts, rank, fs, empty_flag);
         else
-            pack_keys_kernel<float, 3, false><<<grid, block, 0, st>>>(L, g, xyzr, keys, counts, rank, fs, empty_flag);
+            chain(pack_keys_kernel<float, 3, false>, grid, block, 0, st, L, g, xyzr, keys, counts, rank, fs, empty_flag);
     } break;
     case 2: {  // FLOAT_XYZR
         bool al = (addr % 4 == 0) && (L.stride % 4 == 0);
         if (al)
-            pack_keys_kernel<float, 4, true><<<grid, block, 0, st>>>(L, g, xyzr, keys, counts, rank, fs, empty_flag);
+            chain(pack_keys_kernel<float, 4, true>, grid, block, 0, st, L, g, xyzr, keys, counts, rank, fs, empty_flag);
         else
-            pack_keys_kernel<float, 4, false><<<grid, block, 0, st>>>(L, g, xyzr, keys, counts, rank, fs, empty_flag);
+            chain(pack_keys_kernel<float, 4, false>, grid, block, 0, st, L, g, xyzr, keys, counts, rank, fs, empty_flag);
     } break;
     case 3: {  // SHORT_XYZ
         bool al = (addr % 2 == 0) && (L.stride % 2 == 0);
         if (al)
-            pack_keys_kernel<uint16_t, 3, true><<<grid, block, 0, st>>>(L, g, xyzr, keys, counts, rank, fs, empty_flag);
+            chain(pack_keys_kernel<uint16_t, 3, true>, grid, block, 0, st, L, g, xyzr, keys, counts, rank, fs, empty_flag);
         else
-            pack_keys_kernel<uint16_t, 3, false><<<grid, block, 0, st>>>(L, g, xyzr, keys, counts, rank, fs, empty_flag);
+            chain(pack_keys_kernel<uint16_t, 3, false>, grid, block, 0, st, L, g, xyzr, keys, counts, rank, fs, empty_flag);
     } break;
     case 4: {  // DOUBLE_XYZ
         bool al = (addr % 8 == 0) && (L.stride % 8 == 0);
         if (al)
-            pack_keys_kernel<double, 3, true><<<grid, block, 0, st>>>(L, g, xyzr, keys, counts, rank, fs, empty_flag);
+            chain(pack_keys_kernel<double, 3, true>, grid, block, 0, st, L, g, xyzr, keys, counts, rank, fs, empty_flag);
         else
-            pack_keys_kernel<double, 3, false><<<grid, block, 0, st>>>(L, g, xyzr, keys, counts, rank, fs, empty_flag);
+            chain(pack_keys_kernel<double, 3, false>, grid, block, 0, st, L, g, xyzr, keys, counts, rank, fs, empty_flag);
     } break;
     default:
         return cudaErrorInvalidValue;
@@ -963,7 +974,7 @@ cudaError_t launch_onesweep_bits(uint32_t tiles, SortBuffers& b, int cur, uint32
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess)
         return e;
-    onesweep_kernel<GATHER, BITS><<<tiles, SORT_THREADS, smem, st>>>(b.keys[cur],
+    chain(onesweep_kernel<GATHER, BITS>, tiles, SORT_THREADS, smem, st, b.keys[cur],
         (cur == 0 && b.implicit_vals0 && b.first_pass) ? nullptr : b.vals[cur], b.keys[cur ^ 1],
         b.vals[cur ^ 1], n, shift, offs, counter, status, b.err, GATHER ? b.xyzr_in : nullptr,
         GATHER ? b.rec_a : nullptr, GATHER ? b.rec_b : nullptr, GATHER ? b.xyzr_out : nullptr, b.geo, gate,
@@ -1014,7 +1025,7 @@ cudaError_t launch_sort(SortBuffers& b, uint32_t n, uint32_t max_key, int sms, c
     const cudaError_t e = cudaMemsetAsync(b.hist, 0, sizeof(uint32_t) * sort_hist_words(), st);
     if (e != cudaSuccess)
         return e;
-    radix_hist_kernel<<<hist_grid(n, sms), 256, 0, st>>>(b.keys[0], n, pl, b.hist, b.hist + HIST_WORDS + MAX_PASSES,
+    chain(radix_hist_kernel, hist_grid(n, sms), 256, 0, st, b.keys[0], n, pl, b.hist, b.hist + HIST_WORDS + MAX_PASSES,
                                                          b.status, status_words_of(pl, n));
     return launch_passes(b, pl, n, st, nullptr);
 }
@@ -1023,12 +1034,12 @@ cudaError_t launch_init_frame(FrameScalars* fs, uint32_t* counts, uint32_t nbins
                               cudaStream_t st) {
     const uint64_t c4 = counts ? ((uint64_t) nbins + 4) / 4 : 0;
     const unsigned grid = (unsigned) std::max<uint64_t>(4, std::min<uint64_t>((c4 + 255) / 256, (uint64_t) sms * 8));
-    init_frame_kernel<<<grid, 256, 0, st>>>(fs, reinterpret_cast<uint4*>(counts), c4, hist, (uint32_t) sort_hist_words());
+    chain(init_frame_kernel, grid, 256, 0, st, fs, reinterpret_cast<uint4*>(counts), c4, hist, (uint32_t) sort_hist_words());
     return cudaGetLastError();
 }
 
 cudaError_t launch_count_valid(const uint32_t* start, uint32_t nbins, FrameScalars* fs, cudaStream_t st) {
-    count_valid_kernel<<<1, 1, 0, st>>>(start, nbins, fs);
+    chain(count_valid_kernel, 1, 1, 0, st, start, nbins, fs);
     return cudaGetLastError();
 }
 
@@ -1063,14 +1074,14 @@ cudaError_t launch_bin_sort(SortBuffers& b, uint32_t n, const GridGeo& g, uint32
         const uint32_t ntiles = (uint32_t) bin_scan_words(g.nbins);
         const unsigned pgrid = (unsigned) std::max<uint32_t>(1u, std::min<uint32_t>(ceil_div(n, 256), (uint32_t) sms * 16));
         b.implicit_vals0 = true;
-        bin_tile_sums_kernel<<<ntiles, SCAN_THREADS, 0, st>>>(counts, nb, b.status, fs);
-        bin_starts_kernel<<<ntiles, SCAN_THREADS, 0, st>>>(counts, nb, b.status, start, b.keys[1], fs);
-        scatter_bins_kernel<<<pgrid, 256, 0, st>>>(b.keys[0], b.vals[0], b.xyzr_in, n, start, b.vals[1], b.rec_a,
+        chain(bin_tile_sums_kernel, ntiles, SCAN_THREADS, 0, st, counts, nb, b.status, fs);
+        chain(bin_starts_kernel, ntiles, SCAN_THREADS, 0, st, counts, nb, b.status, start, b.keys[1], fs);
+        chain(scatter_bins_kernel, pgrid, 256, 0, st, b.keys[0], b.vals[0], b.xyzr_in, n, start, b.vals[1], b.rec_a,
                                                    b.rec_b, b.xyzr_out, b.geo, fs);
-        order_bins_kernel<<<pgrid, 256, 0, st>>>(b.keys[0], pl, b.hist, done, b.status, sw,
+        chain(order_bins_kernel, pgrid, 256, 0, st, b.keys[0], pl, b.hist, done, b.status, sw,
                                                  std::min(pgrid, hist_grid(n, sms)), n, g.nbins, b.keys[1], b.vals[1], start, b.xyzr_in, b.rec_a, b.rec_b, b.xyzr_out, b.geo, fs);
     } else if (n > 0) {
-        radix_hist_kernel<<<hist_grid(n, sms), 256, 0, st>>>(b.keys[0], n, pl, b.hist, done, b.status, sw);
+        chain(radix_hist_kernel, hist_grid(n, sms), 256, 0, st, b.keys[0], n, pl, b.hist, done, b.status, sw);
     }
     if (n > 0) {
         const cudaError_t e = launch_passes(b, pl, n, st, gate);
@@ -1078,9 +1089,9 @@ cudaError_t launch_bin_sort(SortBuffers& b, uint32_t n, const GridGeo& g, uint32
             return e;
     }
     const unsigned grid = (unsigned) std::max<uint32_t>(1u, std::min<uint32_t>(ceil_div(n + 1, 256), sms * 8));
-    boundary_starts_kernel<<<grid, 256, 0, st>>>(b.keys[b.result], b.vals[b.result], n, g.nbins, start, gaps, gap_cap, fs,
+    chain(boundary_starts_kernel, grid, 256, 0, st, b.keys[b.result], b.vals[b.result], n, g.nbins, start, gaps, gap_cap, fs,
                                                  gate);
-    cell_gap_fill_kernel<<<sms * 2, 256, 0, st>>>(gaps, gap_cap, start, fs, gate);
+    chain(cell_gap_fill_kernel, sms * 2, 256, 0, st, gaps, gap_cap, start, fs, gate);
     return cudaGetLastError();
 }
 

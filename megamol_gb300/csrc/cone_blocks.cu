@@ -34,6 +34,7 @@ __device__ __forceinline__ void store_block(float* p, const float v[8]) {
 __global__ void __launch_bounds__(256) corner_blocks_kernel(const __grid_constant__ ConeParams cp,
                                                             const __grid_constant__ ConeBlocks cb,
                                                             float* __restrict__ blocks) {
+    chain_begin();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cb.nblocks; i += gridDim.x * blockDim.x) {
         float v[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
         int l = -1;
@@ -93,6 +94,7 @@ template<bool SPLIT>
 __global__ void __launch_bounds__(MARCH_THREADS, 12) cone_blocks_kernel(const __grid_constant__ ConeParams cp,
     const __grid_constant__ ConeBlocks cb, const float4* __restrict__ xyzr, const float4* __restrict__ nrm, uint32_t n,
     const uint32_t* __restrict__ out_order, float* __restrict__ ao) {
+    chain_begin();
     __shared__ float s_acc[SPLIT ? MARCH_THREADS : 1];
     const uint32_t t = threadIdx.x, nc = (uint32_t) cp.ncones;
     uint32_t i, c = 0;
@@ -212,13 +214,13 @@ cudaError_t launch_cone_blocks(const ConeParams& cp, ConeBlocks cb, float* block
         return cudaSuccess;
     cb.blocks = blocks;
     const unsigned bgrid = (unsigned) std::min<uint32_t>(ceil_div(cb.nblocks, 256), (uint32_t) sms * 32);
-    corner_blocks_kernel<<<bgrid, 256, 0, st>>>(cp, cb, blocks);
+    chain(corner_blocks_kernel, bgrid, 256, 0, st, cp, cb, blocks);
     // fewer particles than the SMs hold threads: one thread per (particle, cone)
     if ((uint64_t) n < (uint64_t) sms * 2048) {
         const uint32_t per = (uint32_t) MARCH_THREADS / (uint32_t) cp.ncones;
-        cone_blocks_kernel<true><<<ceil_div(n, per), MARCH_THREADS, 0, st>>>(cp, cb, xyzr, nrm, n, out_order, ao);
+        chain(cone_blocks_kernel<true>, ceil_div(n, per), MARCH_THREADS, 0, st, cp, cb, xyzr, nrm, n, out_order, ao);
     } else {
-        cone_blocks_kernel<false><<<ceil_div(n, MARCH_THREADS), MARCH_THREADS, 0, st>>>(cp, cb, xyzr, nrm, n, out_order,
+        chain(cone_blocks_kernel<false>, ceil_div(n, MARCH_THREADS), MARCH_THREADS, 0, st, cp, cb, xyzr, nrm, n, out_order,
                                                                                         ao);
     }
     return cudaGetLastError();

@@ -86,6 +86,7 @@ template<int TX, int TY, int TZ>
 __global__ void __launch_bounds__(TY* TZ, 2) gather_kernel(GridGeo g, const float4* __restrict__ rec_a,
     const int4* __restrict__ rec_b, const uint32_t* __restrict__ start, float* __restrict__ grid,
     TileStats* __restrict__ tiles, FrameScalars* __restrict__ fs, int smax, int rmax) {
+    chain_begin();
     constexpr int NT = TY * TZ;
     extern __shared__ __align__(16) unsigned char smem[];
     float* acc_s = reinterpret_cast<float*>(smem);                      // [TX][NT]
@@ -913,6 +914,7 @@ __global__ void __launch_bounds__(NT, GATHER_RES / NT) gather_fixed_kernel(const
     const float4* __restrict__ rec_a, const int4* __restrict__ rec_b, const uint32_t* __restrict__ start,
     const __grid_constant__ GatherPasses ps, TileStats* __restrict__ tiles, FrameScalars* __restrict__ fs, int rmax,
     const GatherHeavy hv, uint32_t tiles_z) {
+    chain_begin();
     constexpr int NN = TX * TY * TZ;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ GatherShared<TX, TY, TZ, NT> sh;
@@ -979,6 +981,7 @@ __global__ void __launch_bounds__(NT, GATHER_RES / NT) gather_heavy_kernel(const
     const float4* __restrict__ rec_a, const int4* __restrict__ rec_b, const uint32_t* __restrict__ start,
     const __grid_constant__ GatherPasses ps, TileStats* __restrict__ tiles, FrameScalars* __restrict__ fs, int rmax,
     const GatherHeavy hv, uint32_t tiles_x, uint32_t tiles_y) {
+    chain_begin();
     constexpr int NN = TX * TY * TZ;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ GatherShared<TX, TY, TZ, NT> sh;
@@ -1045,6 +1048,7 @@ __global__ void __launch_bounds__(NT, GATHER_RES / NT) gather_heavy_kernel(const
 // Fixed-order reduction of the tile statistics (one block) and the normalisation constants.
 __global__ void __launch_bounds__(1024) finalize_kernel(const TileStats* __restrict__ tiles, uint32_t ntiles,
     FrameScalars* __restrict__ fs, int mass_normalize, int minmax_normalize, double voxel_volume) {
+    chain_begin();
     __shared__ double s_sum[32];
     __shared__ float s_min[32], s_max[32];
     double sum = 0.0;
@@ -1115,6 +1119,7 @@ __global__ void __launch_bounds__(1024) finalize_kernel(const TileStats* __restr
 
 __global__ void __launch_bounds__(256) normalize_scalar_kernel(float* __restrict__ grid, uint64_t n,
     const FrameScalars* __restrict__ fs, int mass_normalize, int minmax_normalize) {
+    chain_begin();
     const float ms = (float) fs->mass_scale;
     const float off = fs->offset, sc = fs->scale;
     for (uint64_t i = blockIdx.x * (uint64_t) blockDim.x + threadIdx.x; i < n; i += (uint64_t) gridDim.x * blockDim.x)
@@ -1125,6 +1130,7 @@ __global__ void __launch_bounds__(256) normalize_scalar_kernel(float* __restrict
 // the last whole vector is done element-wise.
 __global__ void __launch_bounds__(256) normalize_kernel(float* __restrict__ grid, uint64_t n,
     const FrameScalars* __restrict__ fs, int mass_normalize, int minmax_normalize) {
+    chain_begin();
     const float ms = (float) fs->mass_scale;
     const float off = fs->offset, sc = fs->scale;
     float4* g4 = reinterpret_cast<float4*>(grid);
@@ -1207,12 +1213,12 @@ cudaError_t launch_tiles(const GatherConfig& c, const GridGeo& g, size_t smem, c
         hv.done = reinterpret_cast<uint32_t*>(hv.tiles + hv.cap);
     }
     const uint32_t gx = ceil_div(g.s[0], TX), gy = ceil_div(g.s[1], TY), gz = gather_tiles_z(c, g);
-    kern<<<dim3(gx, gy, gz * (uint32_t) ps.count), NT, smem, st>>>(g, rec_a, rec_b, start, ps, tiles, fs, c.rmax, hv, gz);
+    chain(kern, dim3(gx, gy, gz * (uint32_t) ps.count), NT, smem, st, g, rec_a, rec_b, start, ps, tiles, fs, c.rmax, hv, gz);
     if (hv.cap) {
         auto heavy = gather_heavy_kernel<TX, TY, TZ, NT, ACC, BUMP>;
         if ((e = cudaFuncSetAttribute(heavy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) != cudaSuccess)
             return e;
-        heavy<<<sms * (GATHER_RES / NT), NT, smem, st>>>(g, rec_a, rec_b, start, ps, tiles, fs, c.rmax, hv, gx, gy);
+        chain(heavy, sms * (GATHER_RES / NT), NT, smem, st, g, rec_a, rec_b, start, ps, tiles, fs, c.rmax, hv, gx, gy);
     }
     return cudaGetLastError();
 }
@@ -1257,13 +1263,13 @@ cudaError_t launch_gather(const GatherConfig& c, const GridGeo& g, const float4*
     if (e != cudaSuccess)
         return e;
     dim3 grd(ceil_div(g.s[0], c.tx), ceil_div(g.s[1], c.ty), gather_tiles_z(c, g));
-    kern<<<grd, c.ty * c.tz, smem, st>>>(g, rec_a, rec_b, start, ps.out[0], tiles, fs, c.smax, c.rmax);
+    chain(kern, grd, c.ty * c.tz, smem, st, g, rec_a, rec_b, start, ps.out[0], tiles, fs, c.smax, c.rmax);
     return cudaGetLastError();
 }
 
 cudaError_t launch_finalize(const TileStats* tiles, uint32_t ntiles, FrameScalars* fs, int mass_normalize,
     int minmax_normalize, double, double voxel_volume, cudaStream_t st) {
-    finalize_kernel<<<1, 1024, 0, st>>>(tiles, ntiles, fs, mass_normalize, minmax_normalize, voxel_volume);
+    chain(finalize_kernel, 1, 1024, 0, st, tiles, ntiles, fs, mass_normalize, minmax_normalize, voxel_volume);
     return cudaGetLastError();
 }
 
@@ -1274,11 +1280,11 @@ cudaError_t launch_normalize_modes(float* grid, uint64_t nvox, const FrameScalar
     // the grid starts 16-byte aligned (cudaMalloc, or a caller's device buffer checked below)
     if (reinterpret_cast<uintptr_t>(grid) % 16 != 0) {
         const unsigned g1 = (unsigned) std::max<uint64_t>(1, std::min<uint64_t>((nvox + 255) / 256, (uint64_t) sms * 16));
-        normalize_scalar_kernel<<<g1, 256, 0, st>>>(grid, nvox, fs, mass_normalize, minmax_normalize);
+        chain(normalize_scalar_kernel, g1, 256, 0, st, grid, nvox, fs, mass_normalize, minmax_normalize);
         return cudaGetLastError();
     }
     const unsigned grd = (unsigned) std::max<uint64_t>(1, std::min<uint64_t>((nvox / 4 + 255) / 256, (uint64_t) sms * 8));
-    normalize_kernel<<<grd, 256, 0, st>>>(grid, nvox, fs, mass_normalize, minmax_normalize);
+    chain(normalize_kernel, grd, 256, 0, st, grid, nvox, fs, mass_normalize, minmax_normalize);
     return cudaGetLastError();
 }
 

@@ -89,6 +89,7 @@ template <bool U8>
 __global__ void __launch_bounds__(256) mdao_voxelise_kernel(const MdaoParams mp, const uint32_t* __restrict__ order,
                                                             const float4* __restrict__ xyzr, uint32_t n,
                                                             void* __restrict__ accv) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -196,6 +197,7 @@ __global__ void __launch_bounds__(256) mdao_voxelise_kernel(const MdaoParams mp,
 template <bool U8>
 __global__ void __launch_bounds__(256) mdao_finish_kernel(const void* __restrict__ accv, int64_t nv,
                                                           float* __restrict__ vol) {
+    chain_begin();
     for (int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < nv; i += (int64_t) gridDim.x * blockDim.x) {
         if (U8) {
             const unsigned int a = static_cast<const unsigned int*>(accv)[i];
@@ -218,15 +220,15 @@ cudaError_t launch_mdao_volume(const MdaoParams& mp, const uint32_t* order, cons
     if (n > 0) {
         const unsigned grd = (unsigned) std::max<int64_t>(1, std::min<int64_t>(((int64_t) n + 7) / 8, (int64_t) sms * 16));
         if (mp.unorm8)
-            mdao_voxelise_kernel<true><<<grd, 256, 0, st>>>(mp, order, xyzr, n, acc);
+            chain(mdao_voxelise_kernel<true>, grd, 256, 0, st, mp, order, xyzr, n, acc);
         else
-            mdao_voxelise_kernel<false><<<grd, 256, 0, st>>>(mp, order, xyzr, n, acc);
+            chain(mdao_voxelise_kernel<false>, grd, 256, 0, st, mp, order, xyzr, n, acc);
     }
     const unsigned grd = (unsigned) std::max<int64_t>(1, std::min<int64_t>((nv + 255) / 256, (int64_t) sms * 16));
     if (mp.unorm8)
-        mdao_finish_kernel<true><<<grd, 256, 0, st>>>(acc, nv, vol);
+        chain(mdao_finish_kernel<true>, grd, 256, 0, st, acc, nv, vol);
     else
-        mdao_finish_kernel<false><<<grd, 256, 0, st>>>(acc, nv, vol);
+        chain(mdao_finish_kernel<false>, grd, 256, 0, st, acc, nv, vol);
     return cudaGetLastError();
 }
 

@@ -120,6 +120,7 @@ __device__ __forceinline__ unsigned char unorm8(float v, float sat) {
 
 __global__ void __launch_bounds__(256) fill_feature_tex_kernel(const float* __restrict__ src, int dx, int dy, int dz,
                                                                float sat, unsigned long long surf) {
+    chain_begin();
     const int64_t n = (int64_t) dx * dy * dz;
     const int64_t plane = (int64_t) dx * dy;
     for (int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < n; i += (int64_t) gridDim.x * blockDim.x) {
@@ -226,6 +227,7 @@ __device__ __forceinline__ void put(float* p, float v, bool add) {
 __global__ void __launch_bounds__(TT) mlp_train_kernel(const float* __restrict__ P, const float* __restrict__ X,
     const float* __restrict__ T, const uint32_t* __restrict__ idx, int nbatch, float inv_batch,
     float* __restrict__ partial, float* __restrict__ partial_loss) {
+    chain_begin();
     extern __shared__ __align__(16) unsigned char train_smem[];
     TrainShared& S = *reinterpret_cast<TrainShared*>(train_smem);
     const int t = threadIdx.x;
@@ -371,6 +373,7 @@ __global__ void __launch_bounds__(TT) mlp_train_kernel(const float* __restrict__
 // eighth of the partials each, added up in warp order. The loss follows the gradient (grad[MLP_NPARAM]).
 __global__ void __launch_bounds__(256) mlp_reduce_kernel(const float* __restrict__ partial, int nblk,
     const float* __restrict__ partial_loss, float* __restrict__ grad) {
+    chain_begin();
     __shared__ float s_g[8][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int p = blockIdx.x * 32 + lane;
@@ -393,6 +396,7 @@ __global__ void __launch_bounds__(256) mlp_reduce_kernel(const float* __restrict
 
 __global__ void __launch_bounds__(256) mlp_adam_kernel(float* __restrict__ P, const float* __restrict__ g,
     float* __restrict__ m, float* __restrict__ v, float lr, float b1, float b2, float eps, float c1, float c2) {
+    chain_begin();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= MLP_NPARAM)
         return;
@@ -626,6 +630,7 @@ __device__ __forceinline__ void store_pairs(uint8_t* sA, int row, const uint32_t
 
 template<bool FEATURES_IN>
 __global__ void __launch_bounds__(tc::THREADS, tc::CTAS) mlp_infer_tc_kernel(const MlpInferArgs args, const ConeParams cp) {
+    chain_begin();
     extern __shared__ __align__(1024) uint8_t tc_smem[];
     uint8_t* sA = tc_smem;
     uint8_t* sW1 = tc_smem + tc::A_BYTES;
@@ -939,7 +944,7 @@ void FeatureTex::release() {
 cudaError_t launch_fill_feature_tex(const ConeLevel& L, float sat, const FeatureTex& t, cudaStream_t st) {
     const int64_t n = (int64_t) L.d[0] * L.d[1] * L.d[2];
     const unsigned grd = (unsigned) std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 152 * 16));
-    fill_feature_tex_kernel<<<grd, 256, 0, st>>>(L.v, L.d[0], L.d[1], L.d[2], sat, t.surf);
+    chain(fill_feature_tex_kernel, grd, 256, 0, st, L.v, L.d[0], L.d[1], L.d[2], sat, t.surf);
     return cudaGetLastError();
 }
 
@@ -958,8 +963,8 @@ cudaError_t launch_mlp_train_step(const float* P, const float* X, const float* T
     cudaError_t e = cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess)
         return e;
-    mlp_train_kernel<<<nblk, TT, smem, st>>>(P, X, T, idx, nbatch, 1.0f / (float) nbatch, partial, partial_loss);
-    mlp_reduce_kernel<<<(MLP_NPARAM + 32) / 32, 256, 0, st>>>(partial, nblk, partial_loss, grad);
+    chain(mlp_train_kernel, nblk, TT, smem, st, P, X, T, idx, nbatch, 1.0f / (float) nbatch, partial, partial_loss);
+    chain(mlp_reduce_kernel, (MLP_NPARAM + 32) / 32, 256, 0, st, partial, nblk, partial_loss, grad);
     return cudaGetLastError();
 }
 
@@ -967,7 +972,7 @@ cudaError_t launch_mlp_adam(float* P, const float* g, float* m, float* v, float 
     int step, cudaStream_t st) {
     const float c1 = 1.0f / (1.0f - powf(b1, (float) step));
     const float c2 = 1.0f / (1.0f - powf(b2, (float) step));
-    mlp_adam_kernel<<<ceil_div(MLP_NPARAM, 256), 256, 0, st>>>(P, g, m, v, lr, b1, b2, eps, c1, c2);
+    chain(mlp_adam_kernel, ceil_div(MLP_NPARAM, 256), 256, 0, st, P, g, m, v, lr, b1, b2, eps, c1, c2);
     return cudaGetLastError();
 }
 
@@ -1002,11 +1007,11 @@ cudaError_t launch_mlp_infer(const MlpInferArgs& a, const ConeParams& cp, bool f
     if (features_in) {
         e = cudaFuncSetAttribute(mlp_infer_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::DYN_SMEM);
         if (e == cudaSuccess)
-            mlp_infer_tc_kernel<true><<<grid, tc::THREADS, tc::DYN_SMEM, st>>>(a, cp);
+            chain(mlp_infer_tc_kernel<true>, grid, tc::THREADS, tc::DYN_SMEM, st, a, cp);
     } else {
         e = cudaFuncSetAttribute(mlp_infer_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::DYN_SMEM);
         if (e == cudaSuccess)
-            mlp_infer_tc_kernel<false><<<grid, tc::THREADS, tc::DYN_SMEM, st>>>(a, cp);
+            chain(mlp_infer_tc_kernel<false>, grid, tc::THREADS, tc::DYN_SMEM, st, a, cp);
     }
     return e != cudaSuccess ? e : cudaGetLastError();
 }

@@ -70,6 +70,32 @@ struct TileStats {
     float vmin, vmax;
 };
 
+// A frame's kernels are launched as a chain (programmatic stream serialization): a kernel's launch is prepared while its
+// predecessor runs, its blocks start as the predecessor's leave, and chain_begin(), the first statement of every chained
+// kernel, holds them until the predecessor has finished and its writes are visible. That takes about 1.2 us out of every
+// gap between kernels, which bound small frames (20k density 125 -> 98 us, uniform 100k 325 -> 292 us). Predecessors do not
+// trigger the launch early: the waiting blocks would gain nothing more and take the room of other streams' kernels
+// (32 trajectory frames on four lanes 18.4 -> 21.1 ms). A kernel must not return before chain_begin(): its successor would
+// no longer wait for the kernels before it.
+__device__ __forceinline__ void chain_begin() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template<class... Params, class... Args>
+inline cudaError_t chain(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 __host__ __device__ inline uint32_t ceil_div(uint32_t a, uint32_t b) {
     return (a + b - 1) / b;
 }
