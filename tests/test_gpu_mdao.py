@@ -96,3 +96,19 @@ def test_mdao_empty_frame(ctx):
     ao = run(ctx, f, np.zeros((0, 3), np.float32))
     assert ao.size == 0
     assert not ctx.ao_volume(0).any()
+
+
+@pytest.mark.parametrize("n,rmin,rmax,vs", [(1, 5.0, 5.0, 64), (7, 8.0, 19.0, 160), (2_500, 0.05, 6.0, 96),
+                                            (80_003, 0.02, 0.7, 64)])
+@pytest.mark.parametrize("unorm8", [1, 0])
+def test_mdao_volume_of_sphere_batches(ctx, n, rmin, rmax, vs, unorm8):
+    """Warps with one to sixteen spheres, the last ones short; point squares wider than 64 pixels and disks of more than
+    4096 fragments next to spheres below a voxel; some centres outside the clip box. Bit for bit."""
+    f = frame(n=n, seed=34)
+    rng = np.random.default_rng(n)
+    f.xyzr[:, 3] = np.exp(rng.uniform(np.log(rmin), np.log(rmax), n)).astype(np.float32)
+    f.xyzr[::5, :3] += np.float32(9.0)
+    run(ctx, f, synth.random_normals(n, 3), mdao_volume_size=vs, mdao_unorm8=unorm8)
+    dims, _, _ = oracle.mdao_dims(f.bbox, vs)
+    ref = oracle.mdao_volume_f32(f.xyzr, f.bbox, dims, unorm8=bool(unorm8))
+    assert np.array_equal(ctx.ao_volume(0), ref)
