@@ -82,8 +82,11 @@ __device__ __forceinline__ void tile_extent(const GridGeo& g, FrameScalars* fs, 
     ex.khi[a] = khi;
 }
 
+// Bound by latency at 14 active lanes per instruction (the nodes' candidate lists differ). Three CTAs per SM (80 registers,
+// 1024 staged records: a tile of an LJ liquid's 940 in one chunk) and the row table's scan by the whole CTA: LJ 864k
+// 0.247 ms, where two CTAs with 2048 records and a one-warp scan took 0.346; 768 records 0.32, four CTAs 0.26.
 template<int TX, int TY, int TZ>
-__global__ void __launch_bounds__(TY* TZ, 2) gather_kernel(GridGeo g, const float4* __restrict__ rec_a,
+__global__ void __launch_bounds__(TY* TZ, 3) gather_kernel(GridGeo g, const float4* __restrict__ rec_a,
     const int4* __restrict__ rec_b, const uint32_t* __restrict__ start, float* __restrict__ grid,
     TileStats* __restrict__ tiles, FrameScalars* __restrict__ fs, int smax, int rmax) {
     chain_begin();
@@ -98,6 +101,7 @@ __global__ void __launch_bounds__(TY* TZ, 2) gather_kernel(GridGeo g, const floa
     __shared__ double s_dsum[NT / 32];
     __shared__ float s_fmin[NT / 32], s_fmax[NT / 32];
     __shared__ Extent s_ex;
+    __shared__ uint32_t s_wsum[NT / 32];
 
     const int t = threadIdx.x;
     const int ty = t % TY;
@@ -158,38 +162,48 @@ __global__ void __launch_bounds__(TY* TZ, 2) gather_kernel(GridGeo g, const floa
                         const int pz1 = min(nwz, pz0 + planes_per_chunk);
                         const int nrows = (pz1 - pz0) * nwy;
                         __syncthreads();  // previous users of the row table are done
-                        // row table: begin and staged count of every cell row of the chunk
-                        for (int r = t; r < nrows; r += NT) {
-                            const int zz = wlo[2] + pz0 + r / nwy;
-                            const int yy = wlo[1] + r % nwy;
-                            const uint32_t rowkey = ((uint32_t) (zz + 1) * g.nb[1] + (uint32_t) (yy + 1)) * g.nb[0];
-                            const uint32_t b = start[rowkey + bx_lo];
-                            const uint32_t e = start[rowkey + bx_end];
-                            row_beg[r] = b;
-                            row_off[r + 1] = e - b;
-                        }
-                        __syncthreads();
-                        // exclusive scan of the row counts (one warp)
-                        if (t < 32) {
-                            uint32_t carry = 0;
-                            for (int base = 0; base < nrows; base += 32) {
-                                const int r = base + t;
-                                uint32_t v = r < nrows ? row_off[r + 1] : 0u;
+                        // row table: every cell row's records, and their exclusive scan over the rows, two rows per
+                        // thread (rmax <= 2 NT)
+                        uint32_t total = 0, cnt[2], sum = 0;
 #pragma unroll
-                                for (int o = 1; o < 32; o <<= 1) {
-                                    uint32_t u = __shfl_up_sync(0xffffffffu, v, o);
-                                    if (t >= o)
-                                        v += u;
-                                }
-                                if (r < nrows)
-                                    row_off[r + 1] = carry + v;
-                                carry += __shfl_sync(0xffffffffu, v, 31);
+                        for (int e = 0; e < 2; ++e) {
+                            const int r = 2 * t + e;
+                            cnt[e] = 0;
+                            if (r < nrows) {
+                                const int zr = r / nwy;
+                                const int zz = wlo[2] + pz0 + zr;
+                                const int yy = wlo[1] + r - zr * nwy;
+                                const uint32_t rowkey = ((uint32_t) (zz + 1) * g.nb[1] + (uint32_t) (yy + 1)) * g.nb[0];
+                                const uint32_t b = start[rowkey + bx_lo];
+                                cnt[e] = start[rowkey + bx_end] - b;
+                                row_beg[r] = b;
                             }
-                            if (t == 0)
-                                row_off[0] = 0;
+                            sum += cnt[e];
                         }
+                        uint32_t incl = sum;
+#pragma unroll
+                        for (int o = 1; o < 32; o <<= 1) {
+                            const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+                            if ((t & 31) >= o)
+                                incl += u;
+                        }
+                        if ((t & 31) == 31)
+                            s_wsum[t >> 5] = incl;
                         __syncthreads();
-                        const uint32_t total = row_off[nrows];
+                        uint32_t pre = incl - sum;
+#pragma unroll
+                        for (int w = 0; w < NT / 32; ++w) {
+                            const uint32_t v = s_wsum[w];
+                            pre += w < (t >> 5) ? v : 0u;
+                            total += v;
+                        }
+                        if (2 * t < nrows)
+                            row_off[2 * t] = pre;
+                        if (2 * t + 1 < nrows)
+                            row_off[2 * t + 1] = pre + cnt[0];
+                        if (t == 0)
+                            row_off[nrows] = total;
+                        __syncthreads();
                         for (uint32_t cb = 0; cb < total; cb += (uint32_t) smax) {
                             const uint32_t cn = min((uint32_t) smax, total - cb);
                             if (cb > 0)
