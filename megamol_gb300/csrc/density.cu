@@ -1180,15 +1180,6 @@ __global__ void __launch_bounds__(256) normalize_kernel(float* __restrict__ grid
 
 }  // namespace
 
-size_t gather_smem_bytes(const GatherConfig& c) {
-    if (c.mode == GATHER_EXACT) {  // 64-bit sums, 32 bytes per thread of staged particles, the row table
-        const size_t nt = c.tx == 32 ? 512 : 256;
-        return (size_t) c.tx * c.ty * c.tz * sizeof(unsigned long long) + nt * 32 + (size_t) (2 * c.rmax + 1) * sizeof(uint32_t);
-    }
-    return (size_t) 2 * c.tx * c.ty * c.tz * sizeof(float) + (size_t) c.smax * (sizeof(float4) + sizeof(uint4)) +
-           (size_t) (2 * c.rmax + 1) * sizeof(uint32_t);
-}
-
 // z tiles of the slab [zlo, zhi): from the tile holding plane zlo to the one holding plane zhi - 1
 uint32_t gather_tiles_z(const GatherConfig& c, const GridGeo& g) {
     return ceil_div((uint32_t) g.zhi, (uint32_t) c.tz) - (uint32_t) (g.zlo / c.tz);
@@ -1214,10 +1205,12 @@ GatherHeavy gather_heavy_plan(const GatherConfig& c, uint32_t n, int sms, size_t
 
 namespace {
 template<int TX, int TY, int TZ, int NT, int ACC, bool BUMP>
-cudaError_t launch_tiles(const GatherConfig& c, const GridGeo& g, size_t smem, cudaStream_t st, const float4* rec_a,
+cudaError_t launch_tiles(const GatherConfig& c, const GridGeo& g, cudaStream_t st, const float4* rec_a,
     const int4* rec_b, const uint32_t* start, const GatherPasses& ps, TileStats* tiles, FrameScalars* fs, GatherHeavy hv,
     void* hbuf, int sms) {
     auto kern = gather_fixed_kernel<TX, TY, TZ, NT, ACC, BUMP>;
+    // 64-bit sums, 32 bytes of staged particle per thread, the row table
+    const size_t smem = (size_t) TX * TY * TZ * sizeof(unsigned long long) + NT * 32 + (size_t) (2 * c.rmax + 1) * sizeof(uint32_t);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
     if (e != cudaSuccess)
         return e;
@@ -1238,15 +1231,22 @@ cudaError_t launch_tiles(const GatherConfig& c, const GridGeo& g, size_t smem, c
 }
 
 template<int ACC, bool BUMP>
-cudaError_t launch_exact(const GatherConfig& c, const GridGeo& g, size_t smem, cudaStream_t st, const float4* rec_a,
+cudaError_t launch_exact(const GatherConfig& c, const GridGeo& g, cudaStream_t st, const float4* rec_a,
     const int4* rec_b, const uint32_t* start, const GatherPasses& ps, TileStats* tiles, FrameScalars* fs,
     const GatherHeavy& hv, void* hbuf, int sms) {
-    if (c.tx == 16 && c.ty == 16 && c.tz == 16)
-        return launch_tiles<16, 16, 16, 256, ACC, BUMP>(c, g, smem, st, rec_a, rec_b, start, ps, tiles, fs, hv, hbuf, sms);
+    if (c.tx == 16 && c.ty == 16 && c.tz == 16) {
+        // 512 threads per tile where the tiles leave SMs idle (20k, 27 tiles: 13.0 against 15.0 us) and for the FP64
+        // sums, whose atomics wait longest (vector 500k 0.128 against 0.140 ms); else 256, four CTAs per SM out of step
+        // with one another (LJ 4M 0.268 against 0.333 ms)
+        if constexpr (ACC != ACC_DOUBLE)
+            if (gather_tile_count(c, g) * (uint32_t) ps.count > (uint32_t) sms)
+                return launch_tiles<16, 16, 16, 256, ACC, BUMP>(c, g, st, rec_a, rec_b, start, ps, tiles, fs, hv, hbuf, sms);
+        return launch_tiles<16, 16, 16, 512, ACC, BUMP>(c, g, st, rec_a, rec_b, start, ps, tiles, fs, hv, hbuf, sms);
+    }
     if (c.tx == 16 && c.ty == 8 && c.tz == 8)
-        return launch_tiles<16, 8, 8, 256, ACC, BUMP>(c, g, smem, st, rec_a, rec_b, start, ps, tiles, fs, hv, hbuf, sms);
+        return launch_tiles<16, 8, 8, 256, ACC, BUMP>(c, g, st, rec_a, rec_b, start, ps, tiles, fs, hv, hbuf, sms);
     if (c.tx == 32 && c.ty == 16 && c.tz == 8)
-        return launch_tiles<32, 16, 8, 512, ACC, BUMP>(c, g, smem, st, rec_a, rec_b, start, ps, tiles, fs, hv, hbuf, sms);
+        return launch_tiles<32, 16, 8, 512, ACC, BUMP>(c, g, st, rec_a, rec_b, start, ps, tiles, fs, hv, hbuf, sms);
     return cudaErrorInvalidValue;
 }
 }  // namespace
@@ -1254,13 +1254,12 @@ cudaError_t launch_exact(const GatherConfig& c, const GridGeo& g, size_t smem, c
 cudaError_t launch_gather(const GatherConfig& c, const GridGeo& g, const float4* rec_a, const int4* rec_b,
     const uint32_t* start, const GatherPasses& ps, TileStats* tiles, FrameScalars* fs, const GatherHeavy& hv, void* hbuf,
     int sms, cudaStream_t st) {
-    const size_t smem = gather_smem_bytes(c);
     if (c.mode == GATHER_EXACT) {
         const bool bump = g.kernel == 0;
         auto run = [&](auto acc) {
             constexpr int ACC = decltype(acc)::value;
-            return bump ? launch_exact<ACC, true>(c, g, smem, st, rec_a, rec_b, start, ps, tiles, fs, hv, hbuf, sms)
-                        : launch_exact<ACC, false>(c, g, smem, st, rec_a, rec_b, start, ps, tiles, fs, hv, hbuf, sms);
+            return bump ? launch_exact<ACC, true>(c, g, st, rec_a, rec_b, start, ps, tiles, fs, hv, hbuf, sms)
+                        : launch_exact<ACC, false>(c, g, st, rec_a, rec_b, start, ps, tiles, fs, hv, hbuf, sms);
         };
         if (ps.mode == GatherPasses::DOUBLE)
             return run(std::integral_constant<int, ACC_DOUBLE>{});
@@ -1273,6 +1272,8 @@ cudaError_t launch_gather(const GatherConfig& c, const GridGeo& g, const float4*
     if (c.tx != GATHER_TX || c.ty != GATHER_TY || c.tz != GATHER_TZ)
         return cudaErrorInvalidValue;
     auto kern = gather_kernel<GATHER_TX, GATHER_TY, GATHER_TZ>;
+    const size_t smem = (size_t) 2 * c.tx * c.ty * c.tz * sizeof(float) + (size_t) c.smax * (sizeof(float4) + sizeof(uint4)) +
+                        (size_t) (2 * c.rmax + 1) * sizeof(uint32_t);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
     if (e != cudaSuccess)
         return e;

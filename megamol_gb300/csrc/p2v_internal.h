@@ -143,7 +143,6 @@ cudaError_t launch_vector_grid(const uint32_t* order, const float* dens, const f
                                const VectorGridGeo& geo, uint32_t count, float* pos, float* dir, float* col, float* info,
                                int sms, cudaStream_t st);
 
-size_t gather_smem_bytes(const GatherConfig& c);
 // The crowded-tile plan of a frame of n particles; bytes: the buffer launch_gather takes for it (0: none)
 GatherHeavy gather_heavy_plan(const GatherConfig& c, uint32_t n, int sms, size_t* bytes);
 cudaError_t launch_gather(const GatherConfig& c, const GridGeo& g, const float4* rec_a, const int4* rec_b,

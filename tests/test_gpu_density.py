@@ -247,7 +247,7 @@ def crowd(n, edge, spread, radius, seed):
 # n, box edge, crowd spread, radius, resolution: a tile one CTA may just walk alone and the next size, which queues its
 # parts; many parts; more crowded tiles than the queue holds; more records than one CTA's sums take, without a queue
 CROWDS = [(2 * 32_768, 24.0, 0.2, 0.9, 25), (2 * 32_768 + 2, 24.0, 0.2, 0.9, 25), (300_000, 48.0, 1.5, 0.9, 49),
-          (40_000, 64.0, 20.0, 8.0, 65), (20_000, 15.0, 3.0, 5.0, 16)]
+          (40_000, 64.0, 20.0, 8.0, 65), (20_000, 15.0, 3.0, 5.0, 16), (300_000, 96.0, 1.5, 0.9, 97)]
 
 
 @pytest.mark.parametrize("kernel", [p2v.KERNEL_BUMP, p2v.KERNEL_GAUSS3])
