@@ -74,6 +74,23 @@ __device__ __forceinline__ bool support_misses_nodes(const float q[3], float r, 
     return miss;
 }
 
+// A particle's bin key (nbins: invalid), its cell c and its position q in cells.
+__device__ __forceinline__ bool cell_key(const float4& p, const GridGeo& g, uint32_t& key, int32_t c[3], float q[3]) {
+    const float pc[3] = {p.x, p.y, p.z};
+    bool valid = isfinite(p.x) && isfinite(p.y) && isfinite(p.z) && isfinite(p.w) && p.w > 0.0f;
+    uint32_t bin[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        q[a] = (pc[a] - g.minf[a]) / g.hf[a];
+        valid = valid && fabsf(q[a]) < 1073741824.0f;
+        c[a] = clamp_cell(q[a]);
+        const int32_t b = c[a] < -1 ? -1 : (c[a] > g.s[a] ? g.s[a] : c[a]);
+        bin[a] = static_cast<uint32_t>(b + 1);
+    }
+    key = valid ? (bin[2] * g.nb[1] + bin[1]) * g.nb[0] + bin[0] : g.nbins;
+    return valid;
+}
+
 // Grid-stride over the list: each thread packs several particles and keeps running reductions, so the
 // frame-wide maxima and counts cost one atomic per block rather than per 256 particles. empty_flag (a power of
 // two above every cell key, or 0): added to the key of a particle whose support holds no node, so that the
@@ -85,7 +102,7 @@ constexpr int PACK_AHEAD = 2;  // (4: mixed 64M 0.43 against 0.39 ms)
 
 template<class T, int NC, bool ALIGNED>
 __global__ void __launch_bounds__(256) pack_keys_kernel(ListDesc L, GridGeo g, float4* __restrict__ xyzr,
-    uint32_t* __restrict__ keys, uint32_t* __restrict__ counts, uint32_t* __restrict__ rank,
+    uint32_t* __restrict__ keys, uint32_t* __restrict__ counts, uint8_t* __restrict__ rank,
     FrameScalars* __restrict__ fs, uint32_t empty_flag) {
     chain_begin();
     __shared__ int32_t s_cmin[3][8], s_cmax[3][8];
@@ -116,38 +133,24 @@ __global__ void __launch_bounds__(256) pack_keys_kernel(ListDesc L, GridGeo g, f
             const uint64_t i = i0 + u * step;
             if (i >= L.count)
                 break;
-            const float r = p[u].w;
-            const float pc[3] = {p[u].x, p[u].y, p[u].z};
-            bool valid = isfinite(pc[0]) && isfinite(pc[1]) && isfinite(pc[2]) && isfinite(r) && r > 0.0f;
-            uint32_t bin[3];
             int32_t c[3];
-            float qa[3];
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                const float q = (pc[a] - g.minf[a]) / g.hf[a];
-                qa[a] = q;
-                valid = valid && fabsf(q) < 1073741824.0f;
-                c[a] = clamp_cell(q);
-                const int32_t b = c[a] < -1 ? -1 : (c[a] > g.s[a] ? g.s[a] : c[a]);
-                bin[a] = static_cast<uint32_t>(b + 1);
-            }
-            key[u] = g.nbins;
-            if (valid) {
-                key[u] = (bin[2] * g.nb[1] + bin[1]) * g.nb[0] + bin[0];
+            float q[3];
+            if (cell_key(p[u], g, key[u], c, q)) {
 #pragma unroll
                 for (int a = 0; a < 3; ++a) {
                     cell[a] = min(cell[a], c[a]);
                     cellhi[a] = max(cellhi[a], c[a]);
                 }
-                rbits = max(rbits, __float_as_uint(r));
-                if (empty_flag && support_misses_nodes(qa, r, g))
+                rbits = max(rbits, __float_as_uint(p[u].w));
+                if (empty_flag && support_misses_nodes(q, p[u].w, g))
                     key[u] |= empty_flag;
             } else {
                 ++drop;
             }
             const uint64_t o = L.offset + i;
-            xyzr[o] = p[u];
-            keys[o] = key[u];
+            // streaming stores: the cell counts should stay in L2
+            __stcs(xyzr + o, p[u]);
+            __stcs(keys + o, key[u]);
         }
         if (counts) {
             uint32_t rk[PACK_AHEAD];
@@ -158,7 +161,7 @@ __global__ void __launch_bounds__(256) pack_keys_kernel(ListDesc L, GridGeo g, f
 #pragma unroll
             for (int u = 0; u < PACK_AHEAD; ++u)
                 if (i0 + u * step < L.count)
-                    rank[L.offset + i0 + u * step] = rk[u];
+                    __stcs(rank + L.offset + i0 + u * step, (uint8_t) min(rk[u], 255u));
         }
     }
     // block reduction: one atomic per block and quantity
@@ -651,6 +654,14 @@ __global__ void __launch_bounds__(256) cell_gap_fill_kernel(const uint4* __restr
 }
 
 // ---- counting sort by cell ----
+// counts[key] and the arrival ranks in a pass of their own (!counts_in_packing). A rank past BIN_CELL_MAX is not used: one byte.
+__global__ void __launch_bounds__(256) count_bins_kernel(const uint32_t* __restrict__ keys, uint32_t n,
+                                                         uint32_t* __restrict__ counts, uint8_t* __restrict__ rank) {
+    chain_begin();
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        __stcs(rank + i, (uint8_t) min(atomicAdd(counts + __ldcs(keys + i), 1u), 255u));
+}
+
 constexpr int SCAN_THREADS = 256, SCAN_ITEMS = 16, SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
 // 16 consecutive counts of thread `tid` in tile `tile` (zeros past nb); true when all 16 exist
@@ -711,11 +722,9 @@ __global__ void __launch_bounds__(SCAN_THREADS) bin_tile_sums_kernel(const uint3
     }
 }
 
-// Step 2: start[c] = the sums of the tiles before + the scan inside the tile, for c in [0, nb); cells holding two or more
-// particles are appended to `multi` (their order inside the cell is fixed by order_bins_kernel).
+// Step 2: start[c] = the sums of the tiles before + the scan inside the tile, for c in [0, nb).
 __global__ void __launch_bounds__(SCAN_THREADS) bin_starts_kernel(const uint32_t* __restrict__ counts, uint32_t nb,
-    const uint32_t* __restrict__ tsum, uint32_t* __restrict__ start, uint32_t* __restrict__ multi,
-    FrameScalars* __restrict__ fs) {
+    const uint32_t* __restrict__ tsum, uint32_t* __restrict__ start) {
     chain_begin();
     __shared__ uint32_t s_warp[SCAN_THREADS / 32], s_before[SCAN_THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -730,30 +739,19 @@ __global__ void __launch_bounds__(SCAN_THREADS) bin_starts_kernel(const uint32_t
     const uint64_t b0 = (uint64_t) blockIdx.x * SCAN_TILE + (uint64_t) tid * SCAN_ITEMS;
     uint32_t v[SCAN_ITEMS];
     const bool full = load_counts(counts, nb, b0, v);
-    uint32_t sum = 0, nm = 0;
+    uint32_t sum = 0;
 #pragma unroll
-    for (int e = 0; e < SCAN_ITEMS; ++e) {
+    for (int e = 0; e < SCAN_ITEMS; ++e)
         sum += v[e];
-        nm += v[e] >= 2u ? 1u : 0u;
-    }
-    uint32_t incl = sum, mincl = nm;
+    uint32_t incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-        const uint32_t tm = __shfl_up_sync(0xffffffffu, mincl, o);
-        if (lane >= o) {
+        if (lane >= o)
             incl += t;
-            mincl += tm;
-        }
     }
     if (lane == 31)
         s_warp[w] = incl;
-    // the warp's multi-particle cells take consecutive list entries
-    const uint32_t mtot = __shfl_sync(0xffffffffu, mincl, 31);
-    uint32_t mbase = 0;
-    if (lane == 31 && mtot)
-        mbase = atomicAdd(&fs->bin_nmulti, mtot);
-    mbase = __shfl_sync(0xffffffffu, mbase, 31) + mincl - nm;
     __syncthreads();
     uint32_t wpre = 0;
     for (int k = 0; k < w; ++k)
@@ -763,8 +761,6 @@ __global__ void __launch_bounds__(SCAN_THREADS) bin_starts_kernel(const uint32_t
         run += s_before[k];
 #pragma unroll
     for (int e = 0; e < SCAN_ITEMS; ++e) {
-        if (v[e] >= 2u)
-            multi[mbase++] = (uint32_t) (b0 + e);
         const uint32_t x = run;
         run += v[e];
         v[e] = x;
@@ -781,20 +777,50 @@ __global__ void __launch_bounds__(SCAN_THREADS) bin_starts_kernel(const uint32_t
     }
 }
 
-// Each particle takes slot start[key] + rank of its cell (arrival order within the cell, fixed by
-// order_bins_kernel) and writes its index and its 32-byte gather record there. The sorted keys are not
-// written: the cell starts hold them (keys_from_starts_kernel rebuilds them for the binning readback).
+// The counting sort moves indices first and particles once. Each particle's index goes to slot start[key] + rank of its
+// cell (arrival order; 4 bytes a particle stay in L2 however the particles are ordered), then records_kernel takes the
+// slots in order: a particle's place in its cell is the number of smaller indices there, so the result is the stable sort
+// by key, and the stores of the records are contiguous. Records scattered in the particles' order, and the cells of two and
+// more rewritten in index order after, took 219 + 79 us for 4.4 M particles in no spatial order and 504 + 114 for 8 M; this
+// takes 43 + 47 and 78 + 85 (about 60 bytes a particle written and 30 to 50 read); in lattice order (LJ 4M) there is no difference
+// beyond the byte-sized ranks. The sorted keys are not written: the cell starts hold them (keys_from_starts_kernel rebuilds
+// them for the binning readback).
 __global__ void __launch_bounds__(256) scatter_bins_kernel(const uint32_t* __restrict__ keys_in,
-    const uint32_t* __restrict__ rank, const float4* __restrict__ xyzr, uint32_t n,
-    const uint32_t* __restrict__ start, uint32_t* __restrict__ vals_out, float4* __restrict__ rec_a,
-    int4* __restrict__ rec_b, float4* __restrict__ xyzr_out, GridGeo geo, const FrameScalars* __restrict__ fs) {
+    const uint8_t* __restrict__ rank, uint32_t n, const uint32_t* __restrict__ start, uint32_t* __restrict__ arrived,
+    const FrameScalars* __restrict__ fs) {
     chain_begin();
     if (fs->bin_maxcount > BIN_CELL_MAX)
         return;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t slot = start[keys_in[i]] + rank[i];
-        vals_out[slot] = i;
-        const float4 p = xyzr[i];
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        arrived[start[__ldcs(keys_in + i)] + __ldcs(rank + i)] = i;
+}
+
+// A frame with a cell of more than BIN_CELL_MAX particles goes to the radix sort instead, and takes its histograms here.
+__global__ void __launch_bounds__(256) records_kernel(const uint32_t* __restrict__ keys, SortPlan pl,
+    uint32_t* __restrict__ hist, uint32_t* __restrict__ done, uint32_t* __restrict__ status, uint64_t status_words,
+    uint32_t hist_blocks, uint32_t n, const uint32_t* __restrict__ arrived, uint32_t* __restrict__ vals,
+    const uint32_t* __restrict__ start, const float4* __restrict__ xyzr, float4* __restrict__ rec_a,
+    int4* __restrict__ rec_b, float4* __restrict__ xyzr_out, GridGeo geo, const FrameScalars* __restrict__ fs) {
+    chain_begin();
+    if (fs->bin_maxcount > BIN_CELL_MAX) {
+        radix_hist(keys, n, pl, hist, done, status, status_words, hist_blocks);
+        return;
+    }
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+        const uint32_t v = arrived[j];
+        const float4 p = xyzr[v];
+        uint32_t key;
+        int32_t c[3];
+        float q[3];
+        cell_key(p, geo, key, c, q);
+        const uint32_t s = start[key], e = key < geo.nbins ? start[key + 1] : n;
+        uint32_t slot = j;
+        if (e - s > 1u) {
+            slot = s;
+            for (uint32_t a = s; a < e; ++a)
+                slot += arrived[a] < v ? 1u : 0u;
+        }
+        vals[slot] = v;
         float4 A;
         int4 B;
         make_record(p, geo, A, B);
@@ -802,51 +828,6 @@ __global__ void __launch_bounds__(256) scatter_bins_kernel(const uint32_t* __res
         rec_b[REC_STRIDE * (size_t) slot] = B;
         if (xyzr_out)
             xyzr_out[slot] = p;
-    }
-}
-
-// Every cell with two or more particles (the list `multi`) puts them in index order (an insertion sort of
-// at most BIN_CELL_MAX entries) and rewrites their values and records: the result is the stable sort by key. A frame with
-// a fuller cell goes to the radix sort instead, and takes its histograms here.
-__global__ void __launch_bounds__(256) order_bins_kernel(const uint32_t* __restrict__ keys, SortPlan pl,
-    uint32_t* __restrict__ hist, uint32_t* __restrict__ done, uint32_t* __restrict__ status, uint64_t status_words,
-    uint32_t hist_blocks, uint32_t n, uint32_t nbins, const uint32_t* __restrict__ multi,
-    uint32_t* __restrict__ vals, const uint32_t* __restrict__ start, const float4* __restrict__ xyzr,
-    float4* __restrict__ rec_a, int4* __restrict__ rec_b, float4* __restrict__ xyzr_out, GridGeo geo,
-    const FrameScalars* __restrict__ fs) {
-    chain_begin();
-    if (fs->bin_maxcount > BIN_CELL_MAX) {
-        radix_hist(keys, n, pl, hist, done, status, status_words, hist_blocks);
-        return;
-    }
-    const uint32_t nm = fs->bin_nmulti;
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nm; q += gridDim.x * blockDim.x) {
-        const uint32_t k = multi[q];
-        const uint32_t j = start[k];
-        const uint32_t m = (k < nbins ? start[k + 1] : n) - j;
-        uint32_t v[BIN_CELL_MAX];
-        for (uint32_t a = 0; a < m; ++a) {
-            const uint32_t x = vals[j + a];
-            uint32_t b = a;
-            while (b > 0 && v[b - 1] > x) {
-                v[b] = v[b - 1];
-                --b;
-            }
-            v[b] = x;
-        }
-        for (uint32_t a = 0; a < m; ++a) {
-            if (vals[j + a] == v[a])
-                continue;
-            vals[j + a] = v[a];
-            const float4 p = xyzr[v[a]];
-            float4 A;
-            int4 B;
-            make_record(p, geo, A, B);
-            rec_a[REC_STRIDE * (size_t) (j + a)] = A;
-            rec_b[REC_STRIDE * (size_t) (j + a)] = B;
-            if (xyzr_out)
-                xyzr_out[j + a] = p;
-        }
     }
 }
 
@@ -892,7 +873,7 @@ __global__ void count_valid_kernel(const uint32_t* __restrict__ start, uint32_t 
 // host launchers
 // ---------------------------------------------------------------------------------------------
 cudaError_t launch_pack_keys(const ListDesc& L, const GridGeo& g, float4* xyzr, uint32_t* keys, uint32_t* counts,
-    uint32_t* rank, FrameScalars* fs, uint32_t empty_flag, cudaStream_t st) {
+    uint8_t* rank, FrameScalars* fs, uint32_t empty_flag, cudaStream_t st) {
     if (L.count == 0)
         return cudaSuccess;
     const dim3 block(256);
@@ -932,6 +913,13 @@ cudaError_t launch_pack_keys(const ListDesc& L, const GridGeo& g, float4* xyzr, 
         return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
+}
+
+// Below 40 MB of counts (a third of the L2) the packing counts the cells and a pass over the keys is saved; above, the
+// packing's streams push the table out of the L2, and a pass that moves only keys and ranks is faster. Packing and
+// binning, us, in the packing against apart: 33 MB 207 / 216, 50 MB 323 / 311, 67 MB (LJ 4M) 226 / 209, 69 MB 452 / 397.
+bool counts_in_packing(uint32_t nbins) {
+    return nbins < (10u << 20);
 }
 
 namespace {
@@ -1068,18 +1056,20 @@ cudaError_t launch_bin_sort(SortBuffers& b, uint32_t n, const GridGeo& g, uint32
     uint32_t* done = b.hist + HIST_WORDS + MAX_PASSES;
     const uint64_t sw = status_words_of(pl, n);
     if (counting) {
-        // counting sort by cell (counts and arrival ranks from the packing): scan (= the cell starts), scatter, per-cell
-        // index order. Tile sums in the status buffer; the multi-particle cell list in keys[1] (the counting sort writes no
-        // sorted keys there); ranks in vals[0], the gated radix sort takes the identity as its first pass' values
+        // counting sort by cell (counts and arrival ranks from the packing): scan (= the cell starts), scatter of the
+        // indices, records. Tile sums in the status buffer; the indices in arrival order in keys[1] (the counting sort
+        // writes no sorted keys there); ranks in vals[0], the gated radix sort takes the identity as its first pass' values
         const uint32_t ntiles = (uint32_t) bin_scan_words(g.nbins);
         const unsigned pgrid = (unsigned) std::max<uint32_t>(1u, std::min<uint32_t>(ceil_div(n, 256), (uint32_t) sms * 16));
         b.implicit_vals0 = true;
+        if (!counts_in_packing(g.nbins))
+            chain(count_bins_kernel, pgrid, 256, 0, st, b.keys[0], n, counts, reinterpret_cast<uint8_t*>(b.vals[0]));
         chain(bin_tile_sums_kernel, ntiles, SCAN_THREADS, 0, st, counts, nb, b.status, fs);
-        chain(bin_starts_kernel, ntiles, SCAN_THREADS, 0, st, counts, nb, b.status, start, b.keys[1], fs);
-        chain(scatter_bins_kernel, pgrid, 256, 0, st, b.keys[0], b.vals[0], b.xyzr_in, n, start, b.vals[1], b.rec_a,
-                                                   b.rec_b, b.xyzr_out, b.geo, fs);
-        chain(order_bins_kernel, pgrid, 256, 0, st, b.keys[0], pl, b.hist, done, b.status, sw,
-                                                 std::min(pgrid, hist_grid(n, sms)), n, g.nbins, b.keys[1], b.vals[1], start, b.xyzr_in, b.rec_a, b.rec_b, b.xyzr_out, b.geo, fs);
+        chain(bin_starts_kernel, ntiles, SCAN_THREADS, 0, st, counts, nb, b.status, start);
+        chain(scatter_bins_kernel, pgrid, 256, 0, st, b.keys[0], reinterpret_cast<const uint8_t*>(b.vals[0]), n, start,
+              b.keys[1], fs);
+        chain(records_kernel, pgrid, 256, 0, st, b.keys[0], pl, b.hist, done, b.status, sw, std::min(pgrid, hist_grid(n, sms)),
+              n, b.keys[1], b.vals[1], start, b.xyzr_in, b.rec_a, b.rec_b, b.xyzr_out, b.geo, fs);
     } else if (n > 0) {
         chain(radix_hist_kernel, hist_grid(n, sms), 256, 0, st, b.keys[0], n, pl, b.hist, done, b.status, sw);
     }

@@ -627,7 +627,8 @@ p2v_status p2v_ctx::enqueue_frame(Pipe& pp, const p2v_frame* fr, p2v_volume* vol
                 raw_off += (bytes + 15) & ~uint64_t(15);
             }
         }
-        P2V_CUDA_TRY(launch_pack_keys(d, g, xyzr.as<float4>(), keys0.as<uint32_t>(), counts, vals0.as<uint32_t>(), fs,
+        P2V_CUDA_TRY(launch_pack_keys(d, g, xyzr.as<float4>(), keys0.as<uint32_t>(),
+                                      counts_in_packing(g.nbins) ? counts : nullptr, vals0.as<uint8_t>(), fs,
                                       empty_flag, st));
         off += L.count;
     }

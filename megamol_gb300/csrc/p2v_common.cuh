@@ -45,7 +45,6 @@ struct FrameScalars {
     uint32_t dmin_bits, dmax_bits;  // vector aggregator: density range (float bits, densities >= 0)
     uint32_t vcount;        // vector aggregator: nodes with a non-zero density
     uint32_t bin_maxcount;  // counting sort: particles in the fullest cell (0 when the radix path ran alone)
-    uint32_t bin_nmulti;    // counting sort: cells holding two or more particles
     unsigned long long heavy;  // exact gather: queued crowded tiles (from bit 40) and their parts
     double mass;            // FP64 sum of the raw grid
     float vmin, vmax;       // raw grid min / max

@@ -49,7 +49,9 @@ cudaError_t launch_init_frame(FrameScalars* fs, uint32_t* counts, uint32_t nbins
 // counts, rank (the counting sort, else null): particles per key and each particle's arrival rank. empty_flag: 0, or the
 // bit that sort_empty_flag returns, added to the keys of particles whose support holds no grid node.
 cudaError_t launch_pack_keys(const ListDesc& L, const GridGeo& g, float4* xyzr, uint32_t* keys, uint32_t* counts,
-    uint32_t* rank, FrameScalars* fs, uint32_t empty_flag, cudaStream_t st);
+    uint8_t* rank, FrameScalars* fs, uint32_t empty_flag, cudaStream_t st);
+// Whether the packing counts the cells (small tables), or launch_bin_sort in a pass of its own.
+bool counts_in_packing(uint32_t nbins);
 // fs->n_valid = start[nbins] (the gathers do it themselves)
 cudaError_t launch_count_valid(const uint32_t* start, uint32_t nbins, FrameScalars* fs, cudaStream_t st);
 // The power of two above every cell key (max_key) that marks particles whose support holds no node, or 0 when

@@ -179,3 +179,19 @@ def test_runs_of_empty_cells_around_the_chunk_size(ctx, run):
     assert check(ctx, x, (0.0, 0.0, 0.0, 100.0, 100.0, 100.0), (160, 160, 160)) == 0
     keys, _, _ = ctx.binning()
     assert int(keys[1]) - int(keys[0]) == run
+
+
+@pytest.mark.parametrize("res", [(214, 215, 219), (215, 216, 220)])
+def test_counting_around_the_table_limit(ctx, res):
+    """Cell tables below and above 10 * 2^20 cells (the packing counts, or a pass of its own), several lists, invalid
+    particles, and a cell of exactly 32."""
+    assert ((res[0] + 2) * (res[1] + 2) * (res[2] + 2) < 10 << 20) == (res[0] == 214)
+    rng = np.random.default_rng(res[0])
+    x = np.empty((200_001, 4), np.float32)
+    x[:, :3] = rng.uniform(-1, 51, (len(x), 3))
+    x[:, 3] = 0.3
+    h = np.float32(50.0 / (res[0] - 1))
+    x[rng.choice(len(x), 32, replace=False), :3] = (np.float32(20.5) * h, np.float32(0.1), np.float32(0.1))
+    x[rng.choice(len(x), 20, replace=False), 3] = -1.0
+    lists = [p2v.ParticleList(x[a:b], p2v.VERTDATA_FLOAT_XYZR) for a, b in ((0, 7), (7, 100_000), (100_000, len(x)))]
+    assert check(ctx, x, (0.0, 0.0, 0.0, 50.0, 50.0, 50.0), res, lists=lists) in COUNTING
