@@ -72,7 +72,6 @@ struct Pipe {
     DevBuf vdens, vdirs, vkeys0, vkeys1, vvals0, vvals1, vout;  // the vector aggregator's grid outputs
     DevBuf bcount;                         // particles per cell (the counting sort)
     DevBuf xyzr_s, nrm_s;                  // positions and normals in sorted order (the cone AO stages)
-    DevBuf heavy;                          // the exact gather's crowded tiles
     DevBuf cblocks;                        // corner blocks of the plain march's mip levels
     DevBuf bk0, bk1, xyzr_b, nrm_b, ord_b;  // the AO stages' brick order (ao_brick_order)
     bool xyzr_sorted = false;              // the binning of this frame wrote xyzr_s
@@ -127,7 +126,7 @@ struct Pipe {
         for (DevBuf* b : {&raw, &xyzr, &rec_a, &keys0, &keys1, &vals0, &vals1, &status, &hist, &cstart, &gaps,
                           &grid, &tiles, &scal, &nrm, &ao, &mips, &aos_acc, &aos_tex, &mdao_acc, &mdao_vol, &fb_list,
                           &wts, &wsorted, &wsum, &vdens, &vdirs, &vkeys0, &vkeys1, &vvals0, &vvals1, &vout, &bcount, &xyzr_s, &nrm_s, &bk0, &bk1, &xyzr_b, &nrm_b,
-                          &ord_b, &cblocks, &heavy})
+                          &ord_b, &cblocks})
             b->release();
         for (FeatureTex& t : ftex)
             t.release();
@@ -524,10 +523,12 @@ p2v_status p2v_ctx::enqueue_frame(Pipe& pp, const p2v_frame* fr, p2v_volume* vol
     P2V_CUDA_TRY(keys1.ensure(4 * (N + 1)));
     P2V_CUDA_TRY(vals0.ensure(4 * (N + 1)));
     P2V_CUDA_TRY(vals1.ensure(4 * (N + 1)));
-    // the counting sort by cell while its cell table stays near L2-resident: it passes over the table about
-    // four times (16 bytes per cell) and scatters every particle by a table lookup and an atomic, cheap while
-    // the table sits in L2; a table of hundreds of MB turns every lookup into a DRAM sector, where the radix
-    // sort's streaming passes (~150 bytes per particle) win
+    // The counting sort by cell while its cell table stays near L2-resident: it passes over the table about four times and
+    // looks it up or adds to it three times per particle. The radix sort's passes (~150 bytes per particle) also leave the
+    // particles whose support holds no node out of the gather. Whole frames, counting against radix, ms: LJ 4 M (67 MB)
+    // 1.34 / 1.43, 1 M in 20 M cells (78 MB) 1.383 / 1.379, with clusters 8 M (69 MB) 2.27 / 2.28, 15 M (113 MB) 4.35 / 4.24,
+    // 16 M (135 MB) 4.61 / 4.50, 1.6 M in 30 M cells (121 MB) 1.08 / 1.05, 8 M in 187 M cells 5.90 / 5.15: even at about
+    // 75 MB. The line stays higher, because the order of the binning readback and of collected training pairs hangs on it.
     const bool counting = n > 0 && (uint64_t) g.nbins + 1 <= 64ull * n &&
                           4ull * ((uint64_t) g.nbins + 1) <= COUNTING_TABLE_MAX_BYTES;
     if (counting)
@@ -537,7 +538,11 @@ p2v_status p2v_ctx::enqueue_frame(Pipe& pp, const p2v_frame* fr, p2v_volume* vol
     // particle and keeps plain cell keys
     const uint32_t empty_flag = (!counting && P.ao_brick_order == 0) ? sort_empty_flag(g.nbins) : 0u;
     const uint32_t max_key = empty_flag ? (empty_flag | (empty_flag - 1u)) : g.nbins;
-    P2V_CUDA_TRY(status.ensure(4 * (std::max(sort_status_words(n, max_key), bin_scan_words(g.nbins)) + 256)));
+    // the sort's look-back words and tile sums, then (they are dead by then) the gather's crowded tiles
+    size_t hbytes = 0;
+    const GatherHeavy hv = gather_heavy_plan(gc, n, sms, &hbytes);
+    P2V_CUDA_TRY(status.ensure(std::max<size_t>(
+        4 * (std::max(sort_status_words(n, max_key), bin_scan_words(g.nbins)) + 256), hbytes)));
     P2V_CUDA_TRY(hist.ensure(4 * sort_hist_words()));
     P2V_CUDA_TRY(cstart.ensure(4 * ((size_t) g.nbins + 1)));
     P2V_CUDA_TRY(gaps.ensure(sizeof(uint4) * gap_cap));
@@ -793,13 +798,9 @@ p2v_status p2v_ctx::enqueue_frame(Pipe& pp, const p2v_frame* fr, p2v_volume* vol
             }
             ps.out[3] = pp.wsum.as<float>();  // the weights: plain kernel sums
         }
-        size_t hbytes = 0;
-        const GatherHeavy hv = gather_heavy_plan(gc, n, sms, &hbytes);
-        if (hbytes)
-            P2V_CUDA_TRY(pp.heavy.ensure(hbytes));
         {
             const cudaError_t ge = launch_gather(gc, g, sb.rec_a, sb.rec_b, cstart.as<uint32_t>(), ps,
-                                                 tiles.as<TileStats>(), fs, hv, pp.heavy.ptr, sms, st);
+                                                 tiles.as<TileStats>(), fs, hv, status.ptr, sms, st);
             if (ge == cudaErrorInvalidValue)
                 return fail(P2V_EUNSUPPORTED, "density tile %dx%dx%d is not compiled for accumulate=%d", gc.tx, gc.ty,
                             gc.tz, P.accumulate);
