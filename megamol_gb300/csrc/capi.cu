@@ -460,6 +460,7 @@ p2v_status p2v_ctx::enqueue_frame(Pipe& pp, const p2v_frame* fr, p2v_volume* vol
             return fail(P2V_EINVAL, "bounding box has zero extent along %c", "xyz"[a]);
         g.minf[a] = lo;
         g.hf[a] = rangef / static_cast<float>(res[a] - 1);
+        g.ihf[a] = 1.0f / g.hf[a];
         const double hd = std::fabs((double) hi - (double) lo) / (double) (res[a] - 1);
         g.hhi[a] = (float) hd;
         g.hlo[a] = (float) (hd - (double) g.hhi[a]);

@@ -191,64 +191,46 @@ __device__ __forceinline__ float node_grad(const float* g, int64_t base, int64_t
     return __fmul_rn(__fsub_rn(ld_texel<NC>(g + base + hi * stride), ld_texel<NC>(g + base + lo * stride)), scale);
 }
 
-// lo / hi neighbour and scale of node_grad at node i along an axis of s nodes (s >= 2)
-__device__ __forceinline__ void grad_stencil(int i, int s, int cyc, float ih, int& lo, int& hi, float& scale) {
-    lo = i - 1;
-    hi = i + 1;
-    scale = __fmul_rn(0.5f, ih);
-    if (cyc) {
-        lo = lo < 0 ? lo + s : lo;
-        hi = hi >= s ? hi - s : hi;
-    } else if (i == 0) {
-        lo = 0;
-        scale = ih;
-    } else if (i == s - 1) {
-        hi = s - 1;
-        scale = ih;
-    }
-}
-
 template <bool NC>
 __device__ __forceinline__ float4 gradient_normal(const GridGeo& geo, const float* grid, const float4 p) {
     const float pc[3] = {p.x, p.y, p.z};
-    int i0[3], i1[3];
-    float f[3], ih[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        ih[a] = __frcp_rn(geo.hf[a]);
-        float u = __fmul_rn(__fsub_rn(pc[a], geo.minf[a]), ih[a]);
-        u = fminf(fmaxf(u, 0.0f), (float) (geo.s[a] - 1));  // a NaN coordinate becomes 0 (fmaxf)
-        const int k = min((int) u, geo.s[a] - 1);
-        i0[a] = k;
-        i1[a] = min(k + 1, geo.s[a] - 1);
-        f[a] = __fsub_rn(u, (float) k);
-    }
-    const int64_t sx = geo.s[0], sxy = (int64_t) geo.s[0] * geo.s[1];
-    // the common case: along every axis the upper neighbour of node i0 is i1 and the lower one of i1 is i0, so
-    // the gradients at the eight corners read the corners themselves plus 24 outer nodes (32 loads instead of
-    // 48); the same values and the same operations in the same order as the general case below
-    int lo0[3], hi1[3];
-    float sc0[3], sc1[3];
+    int i0[3];
+    float f[3];
     bool fast = true;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        if (geo.s[a] < 2) {
-            fast = false;
-            break;
-        }
-        int hi0, lo1;
-        grad_stencil(i0[a], geo.s[a], geo.cyc[a], ih[a], lo0[a], hi0, sc0[a]);
-        grad_stencil(i1[a], geo.s[a], geo.cyc[a], ih[a], lo1, hi1[a], sc1[a]);
-        fast = fast && hi0 == i1[a] && lo1 == i0[a];
+        float u = __fmul_rn(__fsub_rn(pc[a], geo.minf[a]), geo.ihf[a]);
+        u = fminf(fmaxf(u, 0.0f), (float) (geo.s[a] - 1));  // a NaN coordinate becomes 0 (fmaxf)
+        const int k = min((int) u, geo.s[a] - 1);
+        i0[a] = k;
+        f[a] = __fsub_rn(u, (float) k);
+        fast = fast && k < geo.s[a] - 1;
     }
     float gr[3] = {0.0f, 0.0f, 0.0f};
+    // the common case, a cell with an upper node along every axis: the gradients at its eight corners read the corners and
+    // 24 outer nodes (32 loads instead of 48), four offsets per axis (0, 1 the cell's nodes, 2 the one below, 3 the one
+    // above) and 32-bit node numbers (nbins, which is larger, is one); the same values and the same operations in the same
+    // order as the general case below
     if (fast) {
-        const int64_t zr[2] = {i0[2] * sxy, i1[2] * sxy}, yr[2] = {i0[1] * sx, i1[1] * sx};
-        const int xs[2] = {i0[0], i1[0]};
+        uint32_t at[3][4];
+        float sc[3][2];
+        const uint32_t stride[3] = {1u, (uint32_t) geo.s[0], (uint32_t) geo.s[0] * (uint32_t) geo.s[1]};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const bool first = i0[a] == 0, last = i0[a] == geo.s[a] - 2;
+            const float half = __fmul_rn(0.5f, geo.ihf[a]);
+            sc[a][0] = first && !geo.cyc[a] ? geo.ihf[a] : half;
+            sc[a][1] = last && !geo.cyc[a] ? geo.ihf[a] : half;
+            const uint32_t k = (uint32_t) i0[a] * stride[a], end = (uint32_t) (geo.s[a] - 1) * stride[a];
+            at[a][0] = k;
+            at[a][1] = k + stride[a];
+            at[a][2] = first ? (geo.cyc[a] ? end : 0u) : k - stride[a];
+            at[a][3] = last ? (geo.cyc[a] ? 0u : end) : k + 2u * stride[a];
+        }
         float cv[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c)
-            cv[c] = ld_texel<NC>(grid + zr[(c >> 2) & 1] + yr[(c >> 1) & 1] + xs[c & 1]);
+            cv[c] = ld_texel<NC>(grid + (at[2][(c >> 2) & 1] + at[1][(c >> 1) & 1] + at[0][c & 1]));
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
             const int cx = c & 1, cy = (c >> 1) & 1, cz = (c >> 2) & 1;
@@ -256,28 +238,33 @@ __device__ __forceinline__ float4 gradient_normal(const GridGeo& geo, const floa
             const float wy = cy ? f[1] : __fsub_rn(1.0f, f[1]);
             const float wz = cz ? f[2] : __fsub_rn(1.0f, f[2]);
             const float w = __fmul_rn(__fmul_rn(wx, wy), wz);
-            // x: corner cx = 0 reads (lo(i0), i1), cx = 1 reads (i0, hi(i1))
-            const float xlo = cx ? cv[c ^ 1] : ld_texel<NC>(grid + zr[cz] + yr[cy] + lo0[0]);
-            const float xhi = cx ? ld_texel<NC>(grid + zr[cz] + yr[cy] + hi1[0]) : cv[c ^ 1];
-            const float ylo = cy ? cv[c ^ 2] : ld_texel<NC>(grid + zr[cz] + lo0[1] * sx + xs[cx]);
-            const float yhi = cy ? ld_texel<NC>(grid + zr[cz] + hi1[1] * sx + xs[cx]) : cv[c ^ 2];
-            const float zlo = cz ? cv[c ^ 4] : ld_texel<NC>(grid + lo0[2] * sxy + yr[cy] + xs[cx]);
-            const float zhi = cz ? ld_texel<NC>(grid + hi1[2] * sxy + yr[cy] + xs[cx]) : cv[c ^ 4];
-            gr[0] = __fmaf_rn(w, __fmul_rn(__fsub_rn(xhi, xlo), cx ? sc1[0] : sc0[0]), gr[0]);
-            gr[1] = __fmaf_rn(w, __fmul_rn(__fsub_rn(yhi, ylo), cy ? sc1[1] : sc0[1]), gr[1]);
-            gr[2] = __fmaf_rn(w, __fmul_rn(__fsub_rn(zhi, zlo), cz ? sc1[2] : sc0[2]), gr[2]);
+            // the outer neighbour along each axis: below the lower corner, above the upper one
+            const float ox = ld_texel<NC>(grid + (at[2][cz] + at[1][cy] + at[0][2 + cx]));
+            const float oy = ld_texel<NC>(grid + (at[2][cz] + at[1][2 + cy] + at[0][cx]));
+            const float oz = ld_texel<NC>(grid + (at[2][2 + cz] + at[1][cy] + at[0][cx]));
+            const float dx = cx ? __fsub_rn(ox, cv[c ^ 1]) : __fsub_rn(cv[c ^ 1], ox);
+            const float dy = cy ? __fsub_rn(oy, cv[c ^ 2]) : __fsub_rn(cv[c ^ 2], oy);
+            const float dz = cz ? __fsub_rn(oz, cv[c ^ 4]) : __fsub_rn(cv[c ^ 4], oz);
+            gr[0] = __fmaf_rn(w, __fmul_rn(dx, sc[0][cx]), gr[0]);
+            gr[1] = __fmaf_rn(w, __fmul_rn(dy, sc[1][cy]), gr[1]);
+            gr[2] = __fmaf_rn(w, __fmul_rn(dz, sc[2][cz]), gr[2]);
         }
     } else {
+        const int64_t sx = geo.s[0], sxy = (int64_t) geo.s[0] * geo.s[1];
+        int i1[3];
 #pragma unroll
+        for (int a = 0; a < 3; ++a)
+            i1[a] = min(i0[a] + 1, geo.s[a] - 1);
+#pragma unroll 1
         for (int c = 0; c < 8; ++c) {
             const int x = (c & 1) ? i1[0] : i0[0], y = (c & 2) ? i1[1] : i0[1], z = (c & 4) ? i1[2] : i0[2];
             const float wx = (c & 1) ? f[0] : __fsub_rn(1.0f, f[0]);
             const float wy = (c & 2) ? f[1] : __fsub_rn(1.0f, f[1]);
             const float wz = (c & 4) ? f[2] : __fsub_rn(1.0f, f[2]);
             const float w = __fmul_rn(__fmul_rn(wx, wy), wz);
-            gr[0] = __fmaf_rn(w, node_grad<NC>(grid, z * sxy + y * sx, 1, x, geo.s[0], geo.cyc[0], ih[0]), gr[0]);
-            gr[1] = __fmaf_rn(w, node_grad<NC>(grid, z * sxy + x, sx, y, geo.s[1], geo.cyc[1], ih[1]), gr[1]);
-            gr[2] = __fmaf_rn(w, node_grad<NC>(grid, y * sx + x, sxy, z, geo.s[2], geo.cyc[2], ih[2]), gr[2]);
+            gr[0] = __fmaf_rn(w, node_grad<NC>(grid, z * sxy + y * sx, 1, x, geo.s[0], geo.cyc[0], geo.ihf[0]), gr[0]);
+            gr[1] = __fmaf_rn(w, node_grad<NC>(grid, z * sxy + x, sx, y, geo.s[1], geo.cyc[1], geo.ihf[1]), gr[1]);
+            gr[2] = __fmaf_rn(w, node_grad<NC>(grid, y * sx + x, sxy, z, geo.s[2], geo.cyc[2], geo.ihf[2]), gr[2]);
         }
     }
     const float l2 = __fmaf_rn(gr[2], gr[2], __fmaf_rn(gr[1], gr[1], __fmul_rn(gr[0], gr[0])));

@@ -22,6 +22,7 @@ struct GridGeo {
     int32_t cyc[3];      // cyclic per axis
     float minf[3];       // bbox min (reference origin)
     float hf[3];         // reference spacing: float(range) / float(res-1)
+    float ihf[3];        // 1 / hf, rounded
     float hhi[3], hlo[3];// exact spacing (right-left)/(res-1) as an unevaluated float sum
     float ihh[3];        // 1 / hhi
     float sigma;

@@ -167,6 +167,29 @@ def test_library_gradient_normals_match_host_normals(ctx, mode):
     assert np.sqrt(np.mean(d ** 2)) <= 1e-5 and d.max() <= 1e-3, (np.sqrt(np.mean(d ** 2)), d.max())
 
 
+@pytest.mark.parametrize("res,cyclic", [((2, 9, 3), 0), ((17, 16, 18), 0), ((17, 16, 18), 1), ((12, 9, 10), 1)])
+def test_gradient_normals_at_the_grid_faces(ctx, res, cyclic):
+    """First, last and only cells of open and cyclic axes, particles on the upper faces (no upper node) and outside the
+    box (clamped to it), against normals from the host's differences: the bounds of the test above."""
+    rng = np.random.default_rng(sum(res) + cyclic)
+    n, edge = 3000, 8.0
+    x = np.empty((n, 4), np.float32)
+    x[:, :3] = rng.uniform(-0.5, edge + 0.5, (n, 3))
+    for a in range(3):
+        x[a * 100:a * 100 + 100, a] = edge
+    x[:, 3] = 0.75 * edge / (max(res) - 1)
+    x[::2, 3] = 1.25 * edge / (min(res) - 1)
+    f = synth.Frame(x, (0.0, 0.0, 0.0, edge, edge, edge), res)
+    kw = dict(ao_mode=p2v.AO_CONE, ao_cones=8, ao_steps=32, ao_levels=3 if min(res) > 2 else 1, ao_early_exit=0, cyclX=cyclic, cyclY=cyclic,
+              cyclZ=cyclic)
+    ao, vol, _ = run_ao(ctx, f, np.zeros((n, 3), np.float32), ao_normals=p2v.NORMALS_GRADIENT, **kw)
+    nrm = synth.gradient_normals(x, vol, f.bbox, cyclic=bool(cyclic))
+    host, _, _ = run_ao(ctx, f, nrm, **kw)
+    d = np.abs(ao.astype(np.float64) - host)
+    assert np.isfinite(ao).all()
+    assert np.sqrt(np.mean(d ** 2)) <= 1e-5 and d.max() <= 1e-3, (np.sqrt(np.mean(d ** 2)), d.max())
+
+
 def test_gradient_normals_ao_pipeline_lj_small(ctx):
     """A small LJ-liquid frame with gradient normals (the headline workload's normal definition)."""
     f = synth.lj_liquid(cells=24, res=64, seed=31)
