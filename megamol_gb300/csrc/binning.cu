@@ -105,8 +105,7 @@ __global__ void __launch_bounds__(256) pack_keys_kernel(ListDesc L, GridGeo g, f
     uint32_t* __restrict__ keys, uint32_t* __restrict__ counts, uint8_t* __restrict__ rank,
     FrameScalars* __restrict__ fs, uint32_t empty_flag) {
     chain_begin();
-    __shared__ int32_t s_cmin[3][8], s_cmax[3][8];
-    __shared__ uint32_t s_rmax[8], s_drop[8];
+    __shared__ int s_part[8][8];
     int32_t cell[3] = {INT32_MAX, INT32_MAX, INT32_MAX};
     int32_t cellhi[3] = {INT32_MIN, INT32_MIN, INT32_MIN};
     uint32_t rbits = 0u, drop = 0u;
@@ -164,48 +163,42 @@ __global__ void __launch_bounds__(256) pack_keys_kernel(ListDesc L, GridGeo g, f
                     __stcs(rank + L.offset + i0 + u * step, (uint8_t) min(rk[u], 255u));
         }
     }
-    // block reduction: one atomic per block and quantity
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        rbits = max(rbits, __shfl_xor_sync(0xffffffffu, rbits, o));
-        drop += __shfl_xor_sync(0xffffffffu, drop, o);
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            cell[a] = min(cell[a], __shfl_xor_sync(0xffffffffu, cell[a], o));
-            cellhi[a] = max(cellhi[a], __shfl_xor_sync(0xffffffffu, cellhi[a], o));
-        }
-    }
+    // The block's extremes, all as maxima (a minimum of c is a maximum of ~c), one quantity per thread of the first eight,
+    // in the order of FrameScalars' first words. An extreme that is no news costs a load: additions to one address are
+    // served one after the other, about 10 ns a block.
     const int w = threadIdx.x >> 5;
-    if (lane_id() == 0) {
-        s_rmax[w] = rbits;
-        s_drop[w] = drop;
+    const int part[7] = {(int) rbits, ~cell[0], ~cell[1], ~cell[2], cellhi[0], cellhi[1], cellhi[2]};
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            s_cmin[a][w] = cell[a];
-            s_cmax[a][w] = cellhi[a];
-        }
+    for (int q = 0; q < 7; ++q) {
+        const int m = __reduce_max_sync(0xffffffffu, part[q]);
+        if (lane_id() == 0)
+            s_part[q][w] = m;
     }
+    drop = __reduce_add_sync(0xffffffffu, drop);
+    if (lane_id() == 0)
+        s_part[7][w] = (int) drop;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        const int nw = blockDim.x >> 5;
-        for (int k = 1; k < nw; ++k) {
-            s_rmax[0] = max(s_rmax[0], s_rmax[k]);
-            s_drop[0] += s_drop[k];
-            for (int a = 0; a < 3; ++a) {
-                s_cmin[a][0] = min(s_cmin[a][0], s_cmin[a][k]);
-                s_cmax[a][0] = max(s_cmax[a][0], s_cmax[a][k]);
-            }
+    const int q = threadIdx.x;
+    if (q < 7) {
+        int m = s_part[q][0];
+#pragma unroll
+        for (int k = 1; k < 8; ++k)
+            m = max(m, s_part[q][k]);
+        int* const at = q == 0 ? reinterpret_cast<int*>(&fs->rmax_bits) : (q < 4 ? &fs->cmin[q - 1] : &fs->cmax[q - 4]);
+        const int now = *reinterpret_cast<volatile int*>(at);
+        if (q >= 1 && q < 4) {
+            if (~m < now)
+                atomicMin(at, ~m);
+        } else if (m > now) {
+            atomicMax(at, m);
         }
-        if (s_rmax[0])
-            atomicMax(&fs->rmax_bits, s_rmax[0]);
-        if (s_drop[0])
-            atomicAdd(&fs->n_dropped, s_drop[0]);
-        for (int a = 0; a < 3; ++a) {
-            if (s_cmin[a][0] != INT32_MAX)
-                atomicMin(&fs->cmin[a], s_cmin[a][0]);
-            if (s_cmax[a][0] != INT32_MIN)
-                atomicMax(&fs->cmax[a], s_cmax[a][0]);
-        }
+    } else if (q == 7) {
+        uint32_t d = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            d += (uint32_t) s_part[7][k];
+        if (d)
+            atomicAdd(&fs->n_dropped, d);
     }
 }
 
@@ -878,8 +871,10 @@ cudaError_t launch_pack_keys(const ListDesc& L, const GridGeo& g, float4* xyzr, 
     if (L.count == 0)
         return cudaSuccess;
     const dim3 block(256);
-    // about 8 particles per thread; at most 64 resident-sized blocks per SM
-    const dim3 grid((unsigned) std::max<uint64_t>(1, std::min<uint64_t>((L.count + 2047) / 2048, 152ull * 64)));
+    // 2 particles per thread (one round) while that is at most eight blocks per SM, then about 8; at most 64 blocks per SM
+    const uint64_t one_round = (L.count + 256 * PACK_AHEAD - 1) / (256 * PACK_AHEAD);
+    const dim3 grid((unsigned) std::max<uint64_t>(std::min<uint64_t>(one_round, 152ull * 8),
+                                                  std::min<uint64_t>((L.count + 2047) / 2048, 152ull * 64)));
     const uintptr_t addr = reinterpret_cast<uintptr_t>(L.data);
     switch (L.type) {
     case 1: {  // FLOAT_XYZ
