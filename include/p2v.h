@@ -251,7 +251,7 @@ typedef struct p2v_stats {
     uint32_t device_error;       /* nonzero: a bounded device wait gave up (status P2V_ETIMEOUT) */
     uint32_t ao_fallback;        /* learned AO: particles that fell back to the cone march */
     uint32_t cell_max_count;     /* binning: particles in the fullest cell when the counting sort by cell was
-                                    tried (it takes frames whose cells hold at most 32), 0 = radix sort only */
+                                    tried (it takes frames whose cells hold at most 255), 0 = radix sort only */
     uint32_t ao_fetches;         /* learned AO: texture fetches per particle of its inference kernel (0 otherwise) */
     double ms_ao_kernel;         /* CUDA events around the AO stage's main kernel alone (the learned AO's inference
                                     or the plain cone march; 0 for other AO modes or untimed frames) */

@@ -2,7 +2,7 @@
 // every particle's gather record in sorted order, and the per-cell start table of the sorted order.
 // Two sorts give the same permutation bit for bit: a counting sort by cell (histogram, scan of the cell
 // counts = the start table, scatter of the indices, records in index order within the cells; taken while no
-// cell holds more than 32 particles) and a stable LSD radix sort (onesweep: one read and
+// cell holds more than BIN_CELL_MAX particles) and a stable LSD radix sort (onesweep: one read and
 // one write of the keys per 8- or 9-bit digit, decoupled look-back across tiles), which runs alone for
 // sparse frames and as the device-side fallback of the counting sort.
 //
@@ -246,8 +246,6 @@ SortPlan sort_plan(uint32_t max_key, bool odd = false) {
     }
     return pl;
 }
-
-constexpr uint32_t BIN_CELL_MAX = 32;  // the counting sort orders cells of up to this many particles
 
 // The radix path runs unless the counting sort (bin_tile_sums / bin_starts / scatter_bins / records) took the
 // frame: with a gate, every radix kernel returns at once when the frame's fullest cell fits the counting

@@ -2107,7 +2107,7 @@ p2v_status p2v_get_binning(p2v_ctx* c, uint32_t* keys, uint32_t* order, uint64_t
     if (e == cudaSuccess)
         e = cudaDeviceSynchronize();
     // the counting sort by cell writes no sorted keys: rebuild them from the cell starts
-    const bool counted = c->stats.cell_max_count > 0 && c->stats.cell_max_count <= 32;
+    const bool counted = c->stats.cell_max_count > 0 && c->stats.cell_max_count <= BIN_CELL_MAX;
     if (e == cudaSuccess && keys && pp.last_n && counted) {
         e = launch_keys_from_starts(pp.cstart.as<uint32_t>(), pp.last_nbins, pp.last_n,
                                     const_cast<uint32_t*>(pp.last_keys), c->sms, 0);

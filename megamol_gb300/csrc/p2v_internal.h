@@ -23,6 +23,10 @@ struct ListDesc {
 
 // The counting sort by cell is taken while its count table stays at most this large (near L2-resident).
 constexpr uint64_t COUNTING_TABLE_MAX_BYTES = 128ull << 20;
+// The counting sort takes frames whose cells hold at most this many particles (an arrival rank is a byte). A particle counts
+// the smaller indices of its cell, reads of the L1 that the lanes of a crowded cell share: trajectories of blobs take
+// 17.4 ms with 255 and 18.1 with 32, from where on the radix sort took the frame.
+constexpr uint32_t BIN_CELL_MAX = 255;
 
 struct SortBuffers {
     uint32_t* keys[2];
@@ -69,7 +73,7 @@ cudaError_t launch_keys_from_starts(const uint32_t* start, uint32_t nbins, uint3
 size_t bin_scan_words(uint32_t nbins);
 // The particle binning (after launch_init_frame and launch_pack_keys): the stable sort of the bin keys (keys[0]) with the
 // gather records, and the cell start table (nbins + 1 entries). counts (from the packing, ranks in vals[0]) selects the
-// counting sort by cell, whose per-cell ordering handles cells of up to 32 particles; a fuller cell sends
+// counting sort by cell, whose per-cell ordering handles cells of up to BIN_CELL_MAX particles; a fuller cell sends
 // the frame through the radix sort on the device. counts == nullptr: the radix sort alone.
 cudaError_t launch_bin_sort(SortBuffers& b, uint32_t n, const GridGeo& g, uint32_t* counts, uint32_t* start,
     uint4* gaps, uint32_t gap_cap, FrameScalars* fs, int sms, cudaStream_t st);

@@ -195,3 +195,17 @@ def test_counting_around_the_table_limit(ctx, res):
     x[rng.choice(len(x), 20, replace=False), 3] = -1.0
     lists = [p2v.ParticleList(x[a:b], p2v.VERTDATA_FLOAT_XYZR) for a, b in ((0, 7), (7, 100_000), (100_000, len(x)))]
     assert check(ctx, x, (0.0, 0.0, 0.0, 50.0, 50.0, 50.0), res, lists=lists) in COUNTING
+
+
+@pytest.mark.parametrize("fill,invalid", [(255, 1), (256, 1), (1, 255), (1, 256), (150, 200)])
+def test_crowded_cells_at_the_rank_limit(ctx, fill, invalid):
+    """Cells (one of them the invalid one) of up to 255 particles, the most the counting sort orders, and of 256."""
+    rng = np.random.default_rng(fill + 1000 * invalid)
+    n = 30_000
+    x = np.empty((n, 4), np.float32)
+    x[:, :3] = rng.uniform(0, 30, (n, 3))
+    x[:, 3] = 0.6
+    idx = rng.choice(n, fill + invalid, replace=False)
+    x[idx[:fill], :3] = rng.uniform(31.05, 31.5, (fill, 3)).astype(np.float32)  # the last cell: nobody else is there
+    x[idx[fill:], 1] = np.nan
+    assert check(ctx, x, (0.0, 0.0, 0.0, 30.0, 30.0, 30.0), (30, 30, 30)) == max(fill, invalid)
