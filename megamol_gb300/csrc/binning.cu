@@ -101,7 +101,7 @@ __device__ __forceinline__ bool cell_key(const float4& p, const GridGeo& g, uint
 constexpr int PACK_AHEAD = 2;  // (4: mixed 64M 0.43 against 0.39 ms)
 
 template<class T, int NC, bool ALIGNED>
-__global__ void __launch_bounds__(256) pack_keys_kernel(ListDesc L, GridGeo g, float4* __restrict__ xyzr,
+__global__ void __launch_bounds__(256, 6) pack_keys_kernel(ListDesc L, GridGeo g, float4* __restrict__ xyzr,
     uint32_t* __restrict__ keys, uint32_t* __restrict__ counts, uint8_t* __restrict__ rank,
     FrameScalars* __restrict__ fs, uint32_t empty_flag) {
     chain_begin();
@@ -550,15 +550,15 @@ __global__ void __launch_bounds__(SORT_THREADS, 3) onesweep_kernel(const uint32_
 // start[c] = first sorted position whose key is >= c, for c in [0, nbins]. Boundary i of the sorted keys (between
 // keys[i-1] and keys[i]) starts the run of cells (keys[i-1], keys[i]]. A warp takes 32 consecutive boundaries, scans the
 // lengths of their runs, and its lanes write the cells of all 32 runs together (consecutive lanes, consecutive cells:
-// coalesced however long the runs are; each lane finds the boundary owning its cell by a binary search over the scanned
-// lengths). A run of more than RUN_MAX cells (a sparse grid holds runs of millions of empty cells) is queued in chunks of
+// coalesced however long the runs are). A run of more than RUN_MAX cells (a sparse grid holds runs of millions of empty cells) is queued in chunks of
 // at most GAP_CHUNK for cell_gap_fill_kernel. Such runs are disjoint, so the chunks number at most (nbins + 1)
 // (1 / GAP_CHUNK + 1 / (RUN_MAX + 1)), below the nbins / 64 + 2 entries the list holds.
 // After a radix sort whose look-back gave up (err), every particle gets the invalid key nbins and the identity order, a
 // valid sorted state (an empty grid), so that no later stage indexes with unfinished output; the frame reports
 // P2V_ETIMEOUT.
-// Bound by its stores: uniform 16M (338 M cells, runs of 21) 0.39 ms; a search per cell in a table of every 64th cell's
-// start, as sparse frames took before, 1.39 ms.
+// Uniform 16M (338 M cells, runs of 21): 0.25 ms (5.7 GB/ms of stores and keys); with a search over the scanned lengths per
+// cell 0.45 ms, bound by issue; a search per cell in a table of every 64th cell's start, as sparse frames took before,
+// 1.39 ms.
 constexpr uint32_t GAP_CHUNK = 8192;
 constexpr uint32_t RUN_MAX = 8192;
 
@@ -569,7 +569,9 @@ __global__ void __launch_bounds__(256) boundary_starts_kernel(uint32_t* __restri
     if (radix_skipped(gate))
         return;
     const bool failed = (ld_volatile(&fs->error) & ERR_LOOKBACK_TIMEOUT) != 0u;
+    __shared__ uint32_t s_owner[256];
     const uint32_t lane = lane_id();
+    const uint32_t le_mask = 0xFFFFFFFFu >> (31u - lane);
     const uint64_t wstride = (uint64_t) gridDim.x * blockDim.x;
     for (uint64_t base = (uint64_t) blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base <= n; base += wstride) {
         const uint64_t i64 = base + lane;
@@ -589,7 +591,8 @@ __global__ void __launch_bounds__(256) boundary_starts_kernel(uint32_t* __restri
             }
         }
         uint32_t len = lo <= hi ? hi - lo + 1u : 0u;
-        if (len > RUN_MAX) {
+        const bool queued = len > RUN_MAX;
+        if (queued) {
             const uint32_t i = (uint32_t) i64;
             const uint32_t nch = (uint32_t) (((uint64_t) len - 1 + GAP_CHUNK) / GAP_CHUNK);
             const uint32_t slot = atomicAdd(&fs->ngaps, nch);
@@ -612,10 +615,30 @@ __global__ void __launch_bounds__(256) boundary_starts_kernel(uint32_t* __restri
         }
         const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
         const uint32_t pre = incl - len;  // first cell slot of this lane's run
+        if (!failed && !__any_sync(0xffffffffu, queued)) {
+            // the runs of consecutive boundaries follow each other: cell slot j is cell lo(lane 0) + j. Its owner is the
+            // last run that has started, by one reduction and a population count.
+            const uint32_t cell0 = __shfl_sync(0xffffffffu, lo, 0);
+            const uint32_t runs = __ballot_sync(0xffffffffu, len != 0u);
+            if (len)
+                s_owner[(threadIdx.x & ~31u) | __popc(runs & (le_mask >> 1))] = (uint32_t) i64;
+            __syncwarp();
+            const uint32_t head = len ? pre : 0xFFFFFFFFu;
+            const uint32_t* own = s_owner + (threadIdx.x & ~31u) - 1;
+            for (uint32_t j0 = 0; j0 < total; j0 += 32) {
+                const uint32_t heads = __reduce_or_sync(0xffffffffu, head - j0 < 32u ? 1u << (head - j0) : 0u);
+                if (j0 + lane < total)
+                    out[cell0 + j0 + lane] = own[__popc(heads & le_mask)];
+                own += __popc(heads);
+            }
+            __syncwarp();
+            continue;
+        }
         for (uint32_t j0 = 0; j0 < total; j0 += 32) {
             const uint32_t j = j0 + lane;
-            // owner: the last lane whose run starts at or before slot j (lanes with empty runs share the next
-            // lane's start and are passed over: the search ends on the last of equal starts)
+            // a queued run among them, or a failed sort: the owner is the last lane whose run starts at or before slot j
+            // (lanes with empty runs share the next lane's start and are passed over: the search ends on the last of
+            // equal starts)
             uint32_t ow = 0;
 #pragma unroll
             for (int step = 16; step > 0; step >>= 1) {
