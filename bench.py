@@ -542,16 +542,16 @@ def run_ours(args):
         # reads no index list), the sorted records, cell starts
         "ms_binning": f.n * (16 + (4 + 16 * radix_passes - 4 if radix_passes else 8) + 32) + nb * 8,
         "ms_density": f.n * 16 + V * 4 + nb * 4,   # sorted records once, the grid written, cell starts
-        "ms_normalize": V * 8,                      # statistics read + normalised write
-        # mip levels read and written, positions + normals in, AO out, the levels read once
-        "ms_ao": sum(4 * (vox[l] + vox[l + 1]) for l in range(len(vox) - 1)) + f.n * (16 + 12 + 4) + 4 * sum(vox),
+        "ms_normalize": V * 8 + sum(vox[1:2]) * 4,  # raw grid read, normalised grid and first mip level written
+        # the other mip levels read and written, positions + normals in, AO out, the levels read once
+        "ms_ao": sum(4 * (vox[l] + vox[l + 1]) for l in range(1, len(vox) - 1)) + f.n * (16 + 12 + 4) + 4 * sum(vox),
     }
-    names = {"ms_binning": "p2v::pack_keys_kernel + " + ("counting sort by cell (scatter_bins_kernel, order_bins_kernel)"
+    names = {"ms_binning": "p2v::pack_keys_kernel + " + ("counting sort by cell (scatter_bins_kernel, records_kernel)"
                                                          if counting else "onesweep radix sort (onesweep_kernel)"),
-             "ms_density": "p2v::gather_fixed_kernel",
-             "ms_normalize": "p2v::finalize_kernel + normalize_kernel",
+             "ms_density": "p2v::gather_fixed_kernel (+ gather_heavy_kernel)",
+             "ms_normalize": "p2v::finalize_kernel + mip_rows_kernel (normalisation with the first mip level)",
              "ms_ao": ("p2v::mlp_infer_tc_kernel (+ mip levels, feature textures, fallback cone march)"
-                       if use_learned else "p2v::cone_ao_kernel (+ mip levels)")}
+                       if use_learned else "p2v::cone_blocks_kernel (+ mip levels, corner blocks)")}
     stages = {k: {"kernel": names[k], "ms": st[k], "algorithmic_bytes": int(b),
                   "achieved_gbs": b / (st[k] * 1e-3) / 1e9 if st[k] > 0 else None,
                   "frac": b / (st[k] * 1e-3) / 1e9 / peak if st[k] > 0 else None}
@@ -587,17 +587,18 @@ def run_ours(args):
         cpu = {"value": r["value"], "unit": "particles/s", "cores": nthreads, "kind": r["kind"],
                "sample": cpu_sample_text(r)}
 
-    # kernels per frame: scalar init, pack, [the counting sort by cell: histogram, tile sums, tile scan, cell
-    # starts, scatter, in-cell order], digit histogram + scan, the radix passes (9/8-bit digits over the bin
-    # keys; an odd count and launched gated after a counting sort), cell starts (3), gather, finalize +
-    # normalise; AO: normals, mips, sorted normals, then the cone march, or the feature textures (one per mip
-    # level the feature samples read) + tensor-core inference + fallback cone march (each writes the AO in
-    # input order)
+    # kernels per frame: init, pack, the counting sort by cell (cell counts where the packing does not take them, tile sums,
+    # cell starts, scatter, records) or the digit histogram, the radix passes (9/8-bit digits over the bin keys; an odd
+    # count and launched gated after a counting sort), cell starts (2), gather (2 above 32,768 particles), finalize; AO:
+    # normalisation with the first mip level, the other mips, normals, then corner blocks + the cone march, or the
+    # feature textures (one per mip level the feature samples read) + tensor-core inference + fallback cone march (each
+    # writes the AO in input order)
     passes = (key_bits + 8) // 9
     if counting and passes % 2 == 0:
         passes += 1
-    launches_density = 1 + 1 + (6 if counting else 0) + 2 + passes + 3 + 1 + 2
-    launches_ao = 1 + (AO_PARAMS["ao_levels"] - 1) + 1 + (feature_levels(f) + 2 if use_learned else 1)
+    sort = (4 + (1 if nb >= 10 << 20 else 0)) if counting else 1
+    launches_density = 2 + sort + passes + 2 + (2 if f.n > 32768 else 1) + 1
+    launches_ao = (AO_PARAMS["ao_levels"] - 1) + 1 + (feature_levels(f) + 2 if use_learned else 2)
     if rank == 0:
         line = {"metric": "particles/s density+AO", "value": value, "unit": "particles/s", "n_gpus": ws,
                 "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True,

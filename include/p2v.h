@@ -217,8 +217,8 @@ typedef struct p2v_params {
     int32_t ao_brick_order;   /* 1: the cone march and the learned AO take the particles in brick-major order (bricks
                                  of 16 x 4 x 4 cells) instead of cell order, so that neighbouring threads sample
                                  neighbouring texels along all three axes; 0: cell order; -1: brick order for the
-                                 plain cone march only (14 % faster on the LJ frame, 1 % on the mixed-phase
-                                 frame, slower on blob trajectories). The same AO bits either way (0) */
+                                 plain cone march only (the march 5 % faster on the LJ frame, less than the
+                                 reordering costs). The same AO bits either way (0) */
 } p2v_params;
 
 /* AOSphere volume deposit rule: which voxel a particle's volume goes to. CPU (createVolumeCPU,

@@ -97,7 +97,8 @@ struct Pipe {
     uint32_t vg_count = 0;
     float vg_radius = 0.0f, vg_bbox[6] = {}, vg_range[2] = {0.0f, 0.0f};
 
-    cudaError_t init(bool with_stream) {
+    // host_floats: room behind the pinned scalars for the context's own results
+    cudaError_t init(bool with_stream, size_t host_floats = 0) {
         for (auto& e : ev) {
             const cudaError_t r = cudaEventCreate(&e);
             if (r != cudaSuccess)
@@ -118,7 +119,7 @@ struct Pipe {
             if (r != cudaSuccess)
                 return r;
         }
-        return cudaMallocHost(&h_scal, sizeof(FrameScalars));
+        return cudaMallocHost(&h_scal, sizeof(FrameScalars) + sizeof(float) * host_floats);
     }
     void release() {
         if (stream)
@@ -226,7 +227,7 @@ struct p2v_ctx {
     int ext_grid_mem = P2V_MEM_HOST;
     DevBuf mlp_P, mlp_m, mlp_v, mlp_g, mlp_part, mlp_ploss, mlp_w1h, mlp_w2h, mlp_lo, mlp_hi, mlp_idx, mlp_y;
     DevBuf mlp_gx;                       // p2v_mlp_gradients' pairs
-    float* mlp_gh = nullptr;             // its pinned result (gradient and loss)
+    float* mlp_gh = nullptr;             // its pinned result (gradient and loss), behind main.h_scal
     DevBuf tX, tT;                       // collected training pairs
     uint64_t t_pairs = 0, t_cap = 0;
     std::vector<uint32_t> t_valid;       // indices of pairs with features
@@ -1882,10 +1883,11 @@ p2v_status p2v_create(p2v_ctx** out, int device) {
         return P2V_ECUDA;
     }
     cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
-    if (c->main.init(false) != cudaSuccess) {
+    if (c->main.init(false, MLP_NPARAM + 1) != cudaSuccess) {
         p2v_destroy(c);
         return P2V_ENOMEM;
     }
+    c->mlp_gh = reinterpret_cast<float*>(c->main.h_scal + 1);
     *out = c;
     return P2V_OK;
 }
@@ -1920,8 +1922,6 @@ void p2v_destroy(p2v_ctx* c) {
         cudaFreeHost(c->b_segs_h);
     if (c->b_err_h)
         cudaFreeHost(c->b_err_h);
-    if (c->mlp_gh)
-        cudaFreeHost(c->mlp_gh);
     for (DevBuf* b : {&c->mlp_P, &c->mlp_m, &c->mlp_v, &c->mlp_g, &c->mlp_part, &c->mlp_ploss, &c->mlp_gx,
                       &c->mlp_w1h, &c->mlp_w2h, &c->mlp_lo, &c->mlp_hi, &c->mlp_idx, &c->mlp_y, &c->tX, &c->tT})
         b->release();
@@ -2460,8 +2460,7 @@ p2v_status p2v_mlp_gradients(p2v_ctx* c, const float* x, const float* t, uint32_
     const size_t xf = (size_t) n * MLP_IN;
     if (c->mlp_gx.ensure(sizeof(float) * (xf + n)) != cudaSuccess ||
         c->mlp_part.ensure(sizeof(float) * (size_t) mlp_train_blocks((int) n) * MLP_NPARAM) != cudaSuccess ||
-        c->mlp_ploss.ensure(sizeof(float) * mlp_train_blocks((int) n)) != cudaSuccess ||
-        (!c->mlp_gh && cudaMallocHost(&c->mlp_gh, sizeof(float) * (MLP_NPARAM + 1)) != cudaSuccess))
+        c->mlp_ploss.ensure(sizeof(float) * mlp_train_blocks((int) n)) != cudaSuccess)
         return c->fail(P2V_ENOMEM, "gradient buffers");
     float* dx = c->mlp_gx.as<float>();
     cudaStream_t st = c->own_stream;
