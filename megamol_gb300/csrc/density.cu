@@ -1098,7 +1098,7 @@ __global__ void __launch_bounds__(1024) finalize_kernel(const TileStats* __restr
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        const int nw = blockDim.x >> 5;
+        const int nw = (int) min(blockDim.x >> 5, (ntiles + 31u) >> 5);  // the warps that had tiles (27 tiles: 10 -> 8 us)
         for (int w = 1; w < nw; ++w) {
             sum += s_sum[w];
             mn = fminf(mn, s_min[w]);
