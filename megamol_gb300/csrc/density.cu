@@ -453,32 +453,23 @@ __device__ __forceinline__ float small_float(uint32_t x) {
     return __uint_as_float(0x4B000000u | x) - 8388608.0f;
 }
 
-// exp(x) as __expf computes it, and 1 / w. FTZ: results below the normal floats are 0 (they lie far below the fixed
-// point's quantum), which spares the scaling around the special-function unit; w is never subnormal (1 - x of a float x).
-template<bool FTZ>
-__device__ __forceinline__ float exp_fast(float x) {
-    if (!FTZ)
-        return __expf(x);
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__fmul_rn(x, 1.4426950408889634f)));
-    return y;
-}
+// 1 / w within 2^-23 of itself (w is never subnormal: 1 - x of a float x)
 __device__ __forceinline__ float rcp_fast(float w) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(w));
     return y;
 }
 
-// The kernel at squared distance d2 inside the support. The hardware reciprocal and exponential: the kernel's relative
-// error stays below 1e-6 where it exceeds 1e-7 of its peak (at 1/w = 16, e^-16 = 1.1e-7 of the peak, the reciprocal's
-// 2.4e-7 relative error moves e^-1/w by 3.8e-6 of itself).
-template<bool BUMP, bool FTZ>
+// The kernel at squared distance d2 inside the support. With x = 1 / w (bump) or d2 inv (Gaussian) its relative error
+// against exp(-x) grows with x: 2^-23 x from the reciprocal (or the product) and the (2 + 1.173 x) 2^-23 that CUDA
+// documents for __expf, 4.4e-6 at x = 16. Against the kernel's peak (e^-1 and 1) it stays below 1e-6 everywhere.
+template<bool BUMP>
 __device__ __forceinline__ float kernel_value(float d2, float inv, float e45) {
     if (BUMP) {
         const float w = __fmaf_rn(-d2, inv, 1.0f);
-        return w > 0.0f ? exp_fast<FTZ>(-rcp_fast(w)) : 0.0f;
+        return w > 0.0f ? __expf(-rcp_fast(w)) : 0.0f;
     }
-    return fmaxf(exp_fast<FTZ>(-d2 * inv) - e45, 0.0f);
+    return fmaxf(__expf(-d2 * inv) - e45, 0.0f);
 }
 
 // Adds a kernel value to a node of the CTA's sums (smem: [nn] low and [nn] high words, or [nn] 64-bit sums).
@@ -768,7 +759,7 @@ __device__ __forceinline__ uint32_t walk_tile(const GridGeo& g, const float4* __
                                         const float dx = g.hhi[0] * (xf + PA.x);
                                         const float d2 = __fmaf_rn(dx, dx, dyz);
                                         if (d2 < re2)
-                                            add_node<ACC>(smem, NN, row + xl, kernel_value<BUMP, ACC != ACC_DOUBLE>(d2, rinv, E45), pw,
+                                            add_node<ACC>(smem, NN, row + xl, kernel_value<BUMP>(d2, rinv, E45), pw,
                                                           wscale, carry);
                                     }
                                 }

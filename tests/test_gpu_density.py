@@ -273,3 +273,39 @@ def test_crowded_tiles_of_other_shapes(ctx, tile):
     ctx.set_params(tile_x=0, tile_y=0, tile_z=0)
     ref = oracle.density_f64(x, bbox, r, (1, 1, 1), 1.0, oracle.BUMP, NT)
     assert maxrel(vol, ref) <= 1e-6, maxrel(vol, ref)
+
+
+@pytest.mark.parametrize("accumulate", [p2v.ACCUM_EXACT, p2v.ACCUM_KAHAN])
+@pytest.mark.parametrize("radius", [10.0, 7.3, 1.6])
+@pytest.mark.parametrize("kernel", [p2v.KERNEL_BUMP, p2v.KERNEL_GAUSS3])
+def test_kernel_values_within_their_error_bound(ctx, kernel, radius, accumulate):
+    """One particle on a node of a grid of unit spacing (every squared distance is a whole number): each node within the
+    bound its operations give. Bump, x = 1 / w: w is off by at most 2.5 2^-24 (the support's square and its reciprocal,
+    2^-24 of d2 / eps2 < 1 each, and the rounding of w), which moves exp(-x) by x^2 of it; the reciprocal's ulp by
+    x 2^-23. Gaussian: the argument x by three roundings. __expf: (2 + 1.173 x) ulp as documented. Then the float of the
+    sum, and the exact mode's quantum."""
+    if kernel == p2v.KERNEL_GAUSS3:
+        radius /= 3.0
+    res, bbox = (25, 25, 25), (0.0, 0.0, 0.0, 24.0, 24.0, 24.0)
+    x = np.array([[12.0, 12.0, 12.0, radius]], np.float32)
+    vol, _ = run(ctx, [p2v.ParticleList(x)], bbox, res, cyclic=(0, 0, 0), kernel=kernel, accumulate=accumulate)
+    i = np.arange(25, dtype=np.float64) - 12.0
+    d2 = i[:, None, None] ** 2 + i[None, :, None] ** 2 + i[None, None, :] ** 2
+    r = float(x[0, 3])
+    u23 = 2.0 ** -23
+    if kernel == p2v.KERNEL_BUMP:
+        w = 1.0 - d2 / r ** 2
+        arg = 1.0 / np.where(w > 0, w, np.inf)
+        v = np.where(w > 0, np.exp(-arg), 0.0)
+        rel = arg ** 2 * 1.25 * u23 + arg * u23 + (2.0 + 1.173 * arg) * u23
+        err = v * np.expm1(rel)
+    else:
+        arg = d2 / (2.0 * r ** 2)
+        e = np.exp(-arg)
+        v = np.where(arg < 4.5, e - np.exp(-4.5), 0.0)
+        err = e * np.expm1(1.5 * arg * u23 + (2.0 + 1.173 * arg) * u23) + np.exp(-4.5) * (2.0 + 1.173 * 4.5) * u23
+    err = np.where(v > 0, err + v * 2.0 ** -24, 0.0) + 2.0 ** -32
+    ref = oracle.density_f64(x, bbox, res, (0, 0, 0), 1.0, oracle.GAUSS3 if kernel else oracle.BUMP, 1)
+    assert np.allclose(ref, v, rtol=1e-9, atol=1e-15)
+    worst = (np.abs(vol - ref) / err).max()
+    assert worst <= 1.0, worst
