@@ -132,7 +132,8 @@ struct ConeBlocks {
     float wlo, whi;          // normalised coordinates past which every level's samples are zero
     uint32_t nblocks;
 };
-ConeBlocks cone_block_plan(const ConeParams& cp, uint32_t n);
+// unit_texels: every texel lies in [0, 1]
+ConeBlocks cone_block_plan(const ConeParams& cp, bool unit_texels, uint32_t n);
 // builds the blocks and marches the whole frame: particle i's AO goes to ao[out_order[i]] (or ao[i])
 cudaError_t launch_cone_blocks(const ConeParams& cp, ConeBlocks cb, float* blocks, const float4* xyzr, const float4* nrm,
                                uint32_t n, const uint32_t* out_order, float* ao, int sms, cudaStream_t st);

@@ -1320,7 +1320,8 @@ p2v_status p2v_ctx::run_ao(Pipe& pp, const p2v_frame* fr, const GridGeo& g, cons
         if (P.ao_march == P2V_AO_MARCH_WARP) {
             P2V_CUDA_TRY(launch_cone_ao_warp(cp, axyzr, anrm, n, aorder, ao.as<float>(), sms, st));
         } else {
-            const ConeBlocks cb = cone_block_plan(cp, n);
+            // (a level 0 that is not saturated holds the grid's values as they are)
+            const ConeBlocks cb = cone_block_plan(cp, P.ao_volume == P2V_AOVOL_MDAO || cp.sat > 0.0f, n);
             P2V_CUDA_TRY(pp.cblocks.ensure(32 * (size_t) cb.nblocks));
             P2V_CUDA_TRY(launch_cone_blocks(cp, cb, pp.cblocks.as<float>(), axyzr, anrm, n, aorder, ao.as<float>(), sms,
                                             st));

@@ -89,7 +89,8 @@ __device__ __forceinline__ float block_sample(const ConeParams& cp, const ConeBl
 // registers 2.68 ms. SPLIT fills the SMs when the particles do not: uniform 100k 0.136 against 0.187 ms; at 4M it costs
 // 2 % more (2.72 against 2.68 ms).
 // A cone that has left the volume (widened by the coarsest level's border reach) samples only zeros from there on,
-// which leave its sum as it is: it ends there.
+// which leave its sum as it is: it ends there. (Not so an infinite sum, which they turn into NaN: levels whose texels may
+// lie outside [0, 1] get no walls.)
 template<bool SPLIT>
 __global__ void __launch_bounds__(MARCH_THREADS, 12) cone_blocks_kernel(const __grid_constant__ ConeParams cp,
     const __grid_constant__ ConeBlocks cb, const float4* __restrict__ xyzr, const float4* __restrict__ nrm, uint32_t n,
@@ -165,7 +166,7 @@ __global__ void __launch_bounds__(MARCH_THREADS, 12) cone_blocks_kernel(const __
 // per sample of it, and early exit leaves about half of a cone's samples: blocks from 2.5 samples per texel on (the
 // bound is flat: 0.1 to 20 change the uniform 100k frame by 6 %, LJ 4M and the blob trajectory by under 1 %), and at
 // most 2^25 blocks (1 GB) a level.
-ConeBlocks cone_block_plan(const ConeParams& cp, uint32_t n) {
+ConeBlocks cone_block_plan(const ConeParams& cp, bool unit_texels, uint32_t n) {
     ConeBlocks cb{};
     uint32_t samples[MAX_LEVELS] = {};
     for (int k = 0; k < cp.nsteps; ++k) {
@@ -200,11 +201,14 @@ ConeBlocks cone_block_plan(const ConeParams& cp, uint32_t n) {
     // texel coordinate, below 0.0005 texels at 4096 texels per axis
     cb.wlo = -0.501f / dmin;
     cb.whi = 1.0f + 0.501f / dmin;
-    for (int k = 0; k < cp.nsteps; ++k)  // distances that do not grow (a cone length below the offset): no walls
-        if (!(cp.t[k] >= (k > 0 ? cp.t[k - 1] : 0.0f))) {
-            cb.wlo = -INFINITY;
-            cb.whi = INFINITY;
-        }
+    // no walls where distances do not grow (a cone length below the offset), or where a sum may overflow
+    bool walls = unit_texels;
+    for (int k = 0; k < cp.nsteps; ++k)
+        walls = walls && cp.t[k] >= (k > 0 ? cp.t[k - 1] : 0.0f);
+    if (!walls) {
+        cb.wlo = -INFINITY;
+        cb.whi = INFINITY;
+    }
     return cb;
 }
 

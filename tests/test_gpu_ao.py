@@ -289,3 +289,22 @@ def test_mip_levels_of_odd_sizes(ctx, res, norm):
     plain = np.empty_like(vol.ravel())
     ctx.run_frame([L], f.bbox, plain)
     assert np.array_equal(plain.reshape(vol.shape), vol, equal_nan=True)
+
+
+@pytest.mark.parametrize("n", [20_000, 152 * 2048 + 77])          # one thread per cone, per particle
+def test_block_march_of_sums_that_overflow(ctx, n):
+    """Raw densities of hundreds without saturation and early exit: a cone's sum grows by that factor a step and
+    overflows, for some cones at the last sample inside the volume. The zeros after it turn the infinity into NaN in both
+    marches."""
+    rng = np.random.default_rng(90)
+    x = np.empty((n, 4), np.float32)
+    x[:, :3] = rng.uniform(0.0, 10.0, (n, 3))
+    x[:, 3] = 4.0 * (20_000 / n) ** (1.0 / 3.0)                    # about 560 at a node, whatever n
+    f = synth.Frame(x, (0.0, 0.0, 0.0, 10.0, 10.0, 10.0), (32, 32, 32))
+    nrm = synth.random_normals(n, 91)
+    kw = dict(ao_mode=p2v.AO_CONE, ao_cones=8, ao_steps=32, ao_levels=3, normalize=0, ao_volume_scale=0.0,
+              ao_early_exit=0, cyclX=0, cyclY=0, cyclZ=0)
+    a, vol, _ = run_ao(ctx, f, nrm, ao_march=p2v.AO_MARCH_THREAD, **kw)
+    b, _, _ = run_ao(ctx, f, nrm, ao_march=p2v.AO_MARCH_WARP, **kw)
+    assert vol.max() > 100.0
+    assert np.array_equal(a, b), (a != b).sum()
