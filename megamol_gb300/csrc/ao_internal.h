@@ -134,6 +134,18 @@ struct ConeBlocks {
 };
 // unit_texels: every texel lies in [0, 1]
 ConeBlocks cone_block_plan(const ConeParams& cp, bool unit_texels, uint32_t n);
+// The plan that finds room: room(bytes) provides the buffer. Where it has no memory for the blocks (up to 1.15 GB a frame)
+// the march samples every level from its texels, which needs block 0 alone and gives the same bits.
+template<class Room>
+cudaError_t fit_cone_blocks(const ConeParams& cp, bool unit_texels, uint32_t n, Room&& room, ConeBlocks& cb) {
+    cb = cone_block_plan(cp, unit_texels, n);
+    const cudaError_t e = room(32 * (size_t) cb.nblocks);
+    if (e != cudaErrorMemoryAllocation)
+        return e;
+    cudaGetLastError();  // the refused allocation is no error of the frame
+    cb = cone_block_plan(cp, unit_texels, 0);
+    return room(32 * (size_t) cb.nblocks);
+}
 // builds the blocks and marches the whole frame: particle i's AO goes to ao[out_order[i]] (or ao[i])
 cudaError_t launch_cone_blocks(const ConeParams& cp, ConeBlocks cb, float* blocks, const float4* xyzr, const float4* nrm,
                                uint32_t n, const uint32_t* out_order, float* ao, int sms, cudaStream_t st);

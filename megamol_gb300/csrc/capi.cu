@@ -1320,9 +1320,19 @@ p2v_status p2v_ctx::run_ao(Pipe& pp, const p2v_frame* fr, const GridGeo& g, cons
         if (P.ao_march == P2V_AO_MARCH_WARP) {
             P2V_CUDA_TRY(launch_cone_ao_warp(cp, axyzr, anrm, n, aorder, ao.as<float>(), sms, st));
         } else {
+            // a captured frame keeps the buffer that its warm-up run found room for
+            auto room = [&](size_t bytes) {
+                cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+                if (bytes > pp.cblocks.bytes) {
+                    const cudaError_t e = cudaStreamIsCapturing(st, &cs);
+                    if (e != cudaSuccess)
+                        return e;
+                }
+                return cs == cudaStreamCaptureStatusNone ? pp.cblocks.ensure(bytes) : cudaErrorMemoryAllocation;
+            };
             // (a level 0 that is not saturated holds the grid's values as they are)
-            const ConeBlocks cb = cone_block_plan(cp, P.ao_volume == P2V_AOVOL_MDAO || cp.sat > 0.0f, n);
-            P2V_CUDA_TRY(pp.cblocks.ensure(32 * (size_t) cb.nblocks));
+            ConeBlocks cb;
+            P2V_CUDA_TRY(fit_cone_blocks(cp, P.ao_volume == P2V_AOVOL_MDAO || cp.sat > 0.0f, n, room, cb));
             P2V_CUDA_TRY(launch_cone_blocks(cp, cb, pp.cblocks.as<float>(), axyzr, anrm, n, aorder, ao.as<float>(), sms,
                                             st));
         }

@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(MARCH_THREADS, 12) cone_blocks_kernel(const __
 // Which levels get blocks, for n particles. A level's blocks cost about 10 ps per texel to build and save about 7 ps
 // per sample of it, and early exit leaves about half of a cone's samples: blocks from 2.5 samples per texel on (the
 // bound is flat: 0.1 to 20 change the uniform 100k frame by 6 %, LJ 4M and the blob trajectory by under 1 %), and at
-// most 2^25 blocks (1 GB) a level.
+// most 2^25 blocks (1 GB) a level. None for n = 0.
 ConeBlocks cone_block_plan(const ConeParams& cp, bool unit_texels, uint32_t n) {
     ConeBlocks cb{};
     uint32_t samples[MAX_LEVELS] = {};
