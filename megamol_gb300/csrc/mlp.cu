@@ -173,8 +173,9 @@ __global__ void __launch_bounds__(128) mlp_collect_kernel(const ConeParams cp, c
 // 32 samples per CTA with two scalar shared-memory reads per multiply-add took 36.
 constexpr int TS = 16;
 constexpr int TT = 256;
-constexpr int XP = 64;            // padded feature count (zeros past MLP_IN)
+constexpr int XP = (MLP_IN + 63) / 64 * 64;  // padded feature count (zeros past MLP_IN)
 constexpr int WP = MLP_H + 1;     // row pitch of the transposed weights (conflict-free transposing stores)
+static_assert(MLP_H == 64 && TS * MLP_H == 4 * TT, "a thread holds one neuron of four samples and a 4 x 4 gradient tile");
 
 struct TrainShared {  // every array 16-byte aligned
     alignas(16) float w1t[MLP_IN * WP];     // W1^T: [feature][neuron]
@@ -348,13 +349,15 @@ __global__ void __launch_bounds__(TT) mlp_train_kernel(const float* __restrict__
             for (int c = 0; c < 4; ++c)
                 put(G + OFF_W2 + (j0 + r) * MLP_H + i0 + c, g[r][c], more);
         __syncthreads();
-        grad_tile<XP>(S.d1, S.x, j0, i0, g);
+        for (int i1 = i0; i1 < XP; i1 += 64) {
+            grad_tile<XP>(S.d1, S.x, j0, i1, g);
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
+            for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-                if (i0 + c < MLP_IN)
-                    put(G + OFF_W1 + (j0 + r) * MLP_IN + i0 + c, g[r][c], more);
+                for (int c = 0; c < 4; ++c)
+                    if (i1 + c < MLP_IN)
+                        put(G + OFF_W1 + (j0 + r) * MLP_IN + i1 + c, g[r][c], more);
+        }
         if (t < 3 * MLP_H) {  // the biases' gradients and the last layer's weights'
             const int k = t % MLP_H, what = t / MLP_H;
             float v = 0.0f;
