@@ -1,7 +1,7 @@
 """GPU test of the cell binning: the sort of the bin keys must equal a CPU stable sort bit for bit (sorted
 keys, permutation and cell starts), for ordinary, ragged, out-of-box, invalid and crowded inputs and at the
 full LJ-liquid size (4,000,000 particles, 256^3 grid, 25-bit keys). Both sorting paths are covered: the
-counting sort by cell (cells of at most 32 particles, ordered by index within the cell) and the radix sort,
+counting sort by cell (cells of at most 255 particles, ordered by index within the cell) and the radix sort,
 alone (cell table much larger than the particle count) or as the fallback for a fuller cell."""
 import numpy as np
 import pytest
@@ -208,4 +208,29 @@ def test_crowded_cells_at_the_rank_limit(ctx, fill, invalid):
     idx = rng.choice(n, fill + invalid, replace=False)
     x[idx[:fill], :3] = rng.uniform(31.05, 31.5, (fill, 3)).astype(np.float32)  # the last cell: nobody else is there
     x[idx[fill:], 1] = np.nan
+    assert check(ctx, x, (0.0, 0.0, 0.0, 30.0, 30.0, 30.0), (30, 30, 30)) == max(fill, invalid)
+
+
+@pytest.mark.parametrize("fill,invalid", [(33, 1), (255, 1), (1, 255), (256, 1), (1, 256)])
+def test_which_sort_takes_a_crowded_cell(ctx, fill, invalid):
+    """The route itself: with a first radix pass that cannot finish (a tile never publishes its counts), a frame of cells
+    of up to 255 particles succeeds, because the counting sort takes it, and one of 256 times out in the radix sort."""
+    rng = np.random.default_rng(fill + 1000 * invalid)
+    n = 30_000  # 8 sort tiles of 4096 keys
+    x = np.empty((n, 4), np.float32)
+    x[:, :3] = rng.uniform(0, 30, (n, 3))
+    x[:, 3] = 0.6
+    idx = rng.choice(n, fill + invalid, replace=False)
+    x[idx[:fill], :3] = rng.uniform(31.05, 31.5, (fill, 3)).astype(np.float32)  # the last cell: nobody else is there
+    x[idx[fill:], 1] = np.nan
+    ctx.set_params(sort_wait_polls=1000, test_hold_sort=1)
+    try:
+        if max(fill, invalid) <= 255:
+            assert check(ctx, x, (0.0, 0.0, 0.0, 30.0, 30.0, 30.0), (30, 30, 30)) == max(fill, invalid)
+        else:
+            with pytest.raises(p2v.P2VError) as err:
+                check(ctx, x, (0.0, 0.0, 0.0, 30.0, 30.0, 30.0), (30, 30, 30))
+            assert err.value.status == p2v.ETIMEOUT
+    finally:
+        ctx.set_params(sort_wait_polls=0, test_hold_sort=0)
     assert check(ctx, x, (0.0, 0.0, 0.0, 30.0, 30.0, 30.0), (30, 30, 30)) == max(fill, invalid)
