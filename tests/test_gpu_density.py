@@ -8,6 +8,7 @@ import os
 
 import numpy as np
 import pytest
+import torch
 
 import oracle
 from megamol_gb300 import build as nbuild
@@ -309,3 +310,31 @@ def test_kernel_values_within_their_error_bound(ctx, kernel, radius, accumulate)
     assert np.allclose(ref, v, rtol=1e-9, atol=1e-15)
     worst = (np.abs(vol - ref) / err).max()
     assert worst <= 1.0, worst
+
+
+@pytest.mark.parametrize("n,records", [
+    (40_000, lambda limit, chunk: limit), (40_000, lambda limit, chunk: limit + 1),
+    (40_000, lambda limit, chunk: 3 * chunk), (40_000, lambda limit, chunk: 3 * chunk + 1),
+    (32_768, lambda limit, chunk: 32_768),                           # no queue: the most one CTA walks alone
+    (32_769, lambda limit, chunk: 32_769),                           # the smallest frame with a queue, all in one tile
+    (1_300_001, lambda limit, chunk: limit), (1_300_001, lambda limit, chunk: limit + 1),
+    (1_300_001, lambda limit, chunk: 5 * chunk),                     # limit and parts from n / SMs
+])
+def test_tiles_at_the_split_limit(ctx, n, records):
+    """One isolated tile (16^3 nodes, the cells from one below it on) whose records all lie in one cell, so that their
+    number is known: the last that its own CTA walks, the first that is queued, parts that end on its last record and one
+    before it. The FP64 bar, and the same bits for a shuffled frame."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    m = records(max(4096, min(32_768, n // sms)), max(2048, min(8192, n // (4 * sms))))
+    rng = np.random.default_rng(m)
+    x = np.empty((n, 4), np.float32)
+    x[:m, :3] = rng.uniform(24.05, 24.95, (m, 3))
+    x[m:, 0] = rng.uniform(33.0, 126.0, n - m)                       # no other tile shares that cell's records
+    x[m:, 1:3] = rng.uniform(0.0, 126.0, (n - m, 2))
+    x[:, 3] = 0.9
+    bbox, r = (0.0, 0.0, 0.0, 127.0, 127.0, 127.0), (128, 128, 128)
+    vol, _ = run(ctx, [p2v.ParticleList(x)], bbox, r, cyclic=(0, 0, 0))
+    ref = oracle.density_f64(x, bbox, r, (0, 0, 0), 1.0, oracle.BUMP, NT)
+    assert maxrel(vol, ref) <= 1e-6, maxrel(vol, ref)
+    again, _ = run(ctx, [p2v.ParticleList(x[rng.permutation(n)])], bbox, r, cyclic=(0, 0, 0))
+    assert np.array_equal(vol, again)
