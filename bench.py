@@ -285,18 +285,19 @@ def run_reference(args):
     for _ in range(max(0, args.warmup)):
         cpu_pipeline(f, nthreads, kern)
     runs = [cpu_pipeline(f, nthreads, kern) for _ in range(args.steps)]
-    tot = {k: sum(r[k] for r in runs) for k in ("s_density", "s_mip", "s_ao", "s_step")}
-    value = 1.0 / (tot["s_density"] / f.n + tot["s_mip"] / f.n + tot["s_ao"] / runs[0]["ao_particles"])
-    cpu = dict(runs[0], **{k: v / args.steps for k, v in tot.items()})
+    # seconds per step of each stage, and the rate of a step from them
+    sec = {k: sum(r[k] for r in runs) / args.steps for k in ("s_density", "s_mip", "s_ao", "s_step")}
+    value = 1.0 / (sec["s_density"] / f.n + sec["s_mip"] / f.n + sec["s_ao"] / runs[0]["ao_particles"])
+    cpu = dict(runs[0], **sec)
     line = {"metric": "particles/s density+AO", "value": value, "unit": "particles/s", "n_gpus": args.gpus,
-            "steps": args.steps, "warmup": args.warmup, "ms_per_step": 1e3 * tot["s_step"] / args.steps,
+            "steps": args.steps, "warmup": args.warmup, "ms_per_step": 1e3 * sec["s_step"],
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
             "impl": "reference",
             "config": dict(desc, ao="plain cone march 8 cones x 32 steps, 3-level mip, normals down the density "
                                     "gradient"),
             "cpu_baseline": {"value": value, "unit": "particles/s", "cores": nthreads, "kind": runs[0]["kind"],
                              "sample": cpu_sample_text(cpu)},
-            "stages_s_per_step": {k: tot[k] / args.steps for k in ("s_density", "s_mip", "s_ao")},
+            "stages_s_per_step": {k: sec[k] for k in ("s_density", "s_mip", "s_ao")},
             "e2e": {"value": value, "unit": "particles/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
     print(json.dumps(line), flush=True)
 
