@@ -203,7 +203,8 @@ typedef struct p2v_params {
                                  lanes run every frame up to its normalised grid, then ONE persistent launch
                                  builds every frame's mip levels and marches every frame's cones from a
                                  device-side work queue; 0 = each lane runs its frames' AO kernels itself
-                                 (overlapping them with other frames' binning and density); -1 = the choice of
+                                 (overlapping them with other frames' binning and density, and marching on
+                                 corner blocks: 38.9 ms against 78.6 on 64 blob frames); -1 = the choice of
                                  p2v_autotune_batch, 0 before it has run (-1) */
     int32_t queue_wait_polls; /* polls of a queue item's dependency wait in that launch before the call gives up
                                  with P2V_ETIMEOUT; 0 = the default (2^22, a second or more) */

@@ -1,7 +1,8 @@
-// Device code of the MDAO cone march, the mip build and the gradient normals, shared by the per-frame
-// kernels (ao.cu) and the persistent batch kernel (batch_ao.cu). Every function is written in explicitly
-// rounded FP32 (or in operations no compiler contracts), so each kernel that inlines it computes the same
-// bits.
+// Device code of the MDAO cone march, the mip build and the gradient normals. The per-frame kernels (ao.cu,
+// cone_blocks.cu) use the gradient normals, the sampler, the R8 mip rule and the cones' combination; the march over texels
+// and the FP32 mip rule are the persistent batch kernel's (batch_ao.cu), where mip_rows_kernel and cone_blocks_kernel do the
+// same operations in the same order on other layouts. Every function is written in explicitly rounded FP32 (or in
+// operations no compiler contracts), so each kernel that inlines it computes the same bits.
 //
 // NC selects how volume texels are loaded: true reads through the non-coherent path (__ldg), which is
 // valid only for data no thread writes during the kernel; false uses plain loads, which the persistent batch
