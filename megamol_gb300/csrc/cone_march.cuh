@@ -87,10 +87,10 @@ __device__ __forceinline__ float trilinear(const ConeLevel& L, float ux, float u
     const float cx = __fmaf_rn(ux, L.fd[0], -0.5f), cy = __fmaf_rn(uy, L.fd[1], -0.5f);
     const float cz = __fmaf_rn(uz, L.fd[2], -0.5f);
     const float fx0 = floorf(cx), fy0 = floorf(cy), fz0 = floorf(cz);
-    const int x0 = (int) fx0, y0 = (int) fy0, z0 = (int) fz0;
+    const int x0 = __float2int_rd(cx), y0 = __float2int_rd(cy), z0 = __float2int_rd(cz);  // saturating, NaN: 0
     const float fx = __fsub_rn(cx, fx0), fy = __fsub_rn(cy, fy0), fz = __fsub_rn(cz, fz0);
     float c000, c100, c010, c110, c001, c101, c011, c111;
-    if (x0 >= 0 && y0 >= 0 && z0 >= 0 && x0 + 1 < L.d[0] && y0 + 1 < L.d[1] && z0 + 1 < L.d[2]) {
+    if (x0 >= 0 && y0 >= 0 && z0 >= 0 && x0 < L.d[0] - 1 && y0 < L.d[1] - 1 && z0 < L.d[2] - 1) {
         const int sy = L.d[0];
         const int64_t sz = (int64_t) L.d[0] * L.d[1];
         const float* b = L.v + (((int64_t) z0 * L.d[1] + y0) * L.d[0] + x0);
@@ -103,14 +103,17 @@ __device__ __forceinline__ float trilinear(const ConeLevel& L, float ux, float u
         c011 = saturate_if(ld_texel<NC>(b + sz + sy), sat);
         c111 = saturate_if(ld_texel<NC>(b + sz + sy + 1), sat);
     } else {
+        // the upper texels without overflow: a coordinate beyond 2^31 texels (an infinite one) converts to the largest
+        // integer, and a compiler may move the addition behind tex_fetch's clamp, whose result then is not in the level
+        const int x1 = min(x0, 0x7FFFFFFE) + 1, y1 = min(y0, 0x7FFFFFFE) + 1, z1 = min(z0, 0x7FFFFFFE) + 1;
         c000 = tex_fetch<NC>(L, x0, y0, z0, border, sat);
-        c100 = tex_fetch<NC>(L, x0 + 1, y0, z0, border, sat);
-        c010 = tex_fetch<NC>(L, x0, y0 + 1, z0, border, sat);
-        c110 = tex_fetch<NC>(L, x0 + 1, y0 + 1, z0, border, sat);
-        c001 = tex_fetch<NC>(L, x0, y0, z0 + 1, border, sat);
-        c101 = tex_fetch<NC>(L, x0 + 1, y0, z0 + 1, border, sat);
-        c011 = tex_fetch<NC>(L, x0, y0 + 1, z0 + 1, border, sat);
-        c111 = tex_fetch<NC>(L, x0 + 1, y0 + 1, z0 + 1, border, sat);
+        c100 = tex_fetch<NC>(L, x1, y0, z0, border, sat);
+        c010 = tex_fetch<NC>(L, x0, y1, z0, border, sat);
+        c110 = tex_fetch<NC>(L, x1, y1, z0, border, sat);
+        c001 = tex_fetch<NC>(L, x0, y0, z1, border, sat);
+        c101 = tex_fetch<NC>(L, x1, y0, z1, border, sat);
+        c011 = tex_fetch<NC>(L, x0, y1, z1, border, sat);
+        c111 = tex_fetch<NC>(L, x1, y1, z1, border, sat);
     }
     const float c00 = lerp_rn(c000, c100, fx), c10 = lerp_rn(c010, c110, fx);
     const float c01 = lerp_rn(c001, c101, fx), c11 = lerp_rn(c011, c111, fx);

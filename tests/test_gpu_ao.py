@@ -308,3 +308,29 @@ def test_block_march_of_sums_that_overflow(ctx, n):
     b, _, _ = run_ao(ctx, f, nrm, ao_march=p2v.AO_MARCH_WARP, **kw)
     assert vol.max() > 100.0
     assert np.array_equal(a, b), (a != b).sum()
+
+
+@pytest.mark.parametrize("over", [
+    dict(ao_mode=p2v.AO_CONE, ao_march=p2v.AO_MARCH_THREAD),
+    dict(ao_mode=p2v.AO_CONE, ao_march=p2v.AO_MARCH_WARP),
+    dict(ao_mode=p2v.AO_CONE, ao_march=p2v.AO_MARCH_THREAD, ao_volume=p2v.AOVOL_MDAO),
+    dict(ao_mode=p2v.AO_AOSPHERE_AXES), dict(ao_mode=p2v.AO_AOSPHERE_NORMAL)])
+@pytest.mark.parametrize("n", [40, 20_000])                        # some levels sampled from their texels, all from blocks
+def test_particles_at_infinity(ctx, n, over):
+    """Particles with infinite, NaN and huge coordinates, whose texel coordinates no integer holds: a cone march gives
+    them AO 1 (nothing around them), and every other particle the AO of the frame without them."""
+    f = synth.uniform(n=n, edge=30.0, seed=92)
+    f.res = (31, 33, 32)
+    nrm = synth.random_normals(n, 93)
+    kw = dict(dict(ao_cones=8, ao_steps=32, ao_levels=3), **over)
+    ref, vol, _ = run_ao(ctx, f, nrm, **kw)
+    far = np.full((12, 4), 15.0, np.float32)
+    far[np.arange(12), np.arange(12) % 3] = np.repeat(np.array([np.inf, -np.inf, np.nan, 1e30], np.float32), 3)
+    far[:, 3] = 0.5
+    if over["ao_mode"] != p2v.AO_CONE:
+        far = far[:9]                                              # (1e30 is finite: its volume goes to a border voxel)
+    g = synth.Frame(np.concatenate([far, f.xyzr]), f.bbox, f.res)
+    ao, vol2, _ = run_ao(ctx, g, np.concatenate([synth.random_normals(len(far), 94), nrm]), **kw)
+    assert np.array_equal(vol, vol2) and np.array_equal(ao[len(far):], ref)
+    if over["ao_mode"] == p2v.AO_CONE:
+        assert np.all(ao[:len(far)] == 1.0)
