@@ -435,16 +435,21 @@ __device__ __forceinline__ void fixed_halves(float v, uint32_t& hi, uint32_t& lo
     lo = __float_as_uint(u) - 0x4B000000u;
 }
 
-// The float nearest (ties to even) to x 2^-32: sums below 1 take one 32-bit conversion, others 32-bit integer
-// operations and one exact conversion (64-bit conversions run on the narrow FP64 pipe of this part).
-__device__ __forceinline__ float fixed_to_float(unsigned long long x) {
-    if ((uint32_t) (x >> 32) == 0u)
-        return __uint2float_rn((uint32_t) x) * FIX_INV;
+// The float nearest (ties to even) to x 2^-32; q receives the rounded sum (the float times 2^32, an integer). Sums whose
+// float lies below 1 take one 32-bit conversion each way, others 32-bit integer operations and one exact conversion (64-bit
+// conversions run on the narrow FP64 pipe of this part).
+__device__ __forceinline__ float fixed_to_float(unsigned long long x, unsigned long long& q) {
+    if (x < 0xFFFFFF80ull) {  // (2^32 - 128 rounds up)
+        const float f = __uint2float_rn((uint32_t) x);
+        q = __float2uint_rn(f);
+        return f * FIX_INV;
+    }
     const int sh = 40 - __clzll(x);  // bits below a 24-bit significand
     unsigned long long m = x >> sh;
     const unsigned long long rem = x & ((1ull << sh) - 1ull), half = 1ull << (sh - 1);
     m += (rem > half || (rem == half && (m & 1ull))) ? 1ull : 0ull;  // m <= 2^24
-    // m * 2^(sh - 32): the significand converts exactly and the scale is a power of two (sh in [9, 40])
+    q = m << sh;
+    // m * 2^(sh - 32): the significand converts exactly and the scale is a power of two (sh in [8, 40])
     return __uint2float_rn((uint32_t) m) * __int_as_float((95 + sh) << 23);
 }
 
@@ -810,8 +815,8 @@ __device__ __forceinline__ float unorder(int b) {
 }
 
 // Writes a tile (x fastest, coalesced) and its statistics. sums: the tile's slot of 64-bit sums, or null: the CTA's own.
-// The density's tile sum is exact in integers (no node pays an FP64 addition: the FP64 pipe of this part is 1/64 of the
-// FP32 rate).
+// The density's tile sum is the exact sum of the floats written, in integers (no node pays an FP64 addition: the FP64 pipe
+// of this part is 1/64 of the FP32 rate).
 template<int TX, int TY, int TZ, int NT, int ACC>
 __device__ __forceinline__ void write_tile(const GridGeo& g, const int o3[3], GatherShared<TX, TY, TZ, NT>& sh,
     const unsigned char* smem, const unsigned long long* sums, bool carry, float winv, float* __restrict__ grid, int ostride,
@@ -843,9 +848,10 @@ __device__ __forceinline__ void write_tile(const GridGeo& g, const int o3[3], Ga
                 break;
             float v;
             if (ACC == ACC_EXACT) {
-                v = fixed_to_float(q[e]);
-                isum += q[e] >> 32;
-                fsum += q[e] & 0xFFFFFFFFull;
+                unsigned long long r;
+                v = fixed_to_float(q[e], r);
+                isum += r >> 32;
+                fsum += r & 0xFFFFFFFFull;
             } else {
                 v = ACC == ACC_FIXED_W ? __ll2float_rn((long long) q[e]) * winv
                                        : __double2float_rn(__longlong_as_double((long long) q[e]));

@@ -4,6 +4,7 @@ Bars: against the FP64 oracle, max-rel error (max|a-b| / max|b|) <= 1e-6 (the ta
 the reference module's own FP32 output (golden fixtures) the difference is bounded by the reference's
 float rounding, <= 2e-5 of the maximum. Integer metadata (resolution, slice distances) must be identical.
 """
+import math
 import os
 
 import numpy as np
@@ -338,3 +339,20 @@ def test_tiles_at_the_split_limit(ctx, n, records):
     assert maxrel(vol, ref) <= 1e-6, maxrel(vol, ref)
     again, _ = run(ctx, [p2v.ParticleList(x[rng.permutation(n)])], bbox, r, cyclic=(0, 0, 0))
     assert np.array_equal(vol, again)
+
+
+@pytest.mark.parametrize("n,radius,tile", [(30_000, 0.9, 16), (30_000, 3.0, 16), (400_000, 2.0, 16), (30_000, 0.9, 8)])
+def test_mass_sum_is_the_sum_of_the_grid(ctx, n, radius, tile):
+    """stats["mass_sum"] is the sum of the floats of the raw grid: exact integers within a tile, one FP64 rounding per tile
+    is the most it may lack (a sum of the unrounded fixed-point values is off by about 1e-9 of it). Nodes below and above
+    1, crowded tiles that are written by their last part."""
+    x = crowd(n, 40.0, 1.5, radius, n)
+    res = (49, 50, 47)
+    if tile != 16:
+        ctx.set_params(tile_x=16, tile_y=8, tile_z=8)
+    vol, _ = run(ctx, [p2v.ParticleList(x)], (0, 0, 0, 40.0, 40.0, 40.0), res)
+    ctx.set_params(tile_x=0, tile_y=0, tile_z=0)
+    exact = math.fsum(vol.ravel().tolist())
+    tiles = 4 * 4 * 3 if tile == 16 else 4 * 7 * 6
+    assert vol.max() > 1.0
+    assert abs(ctx.stats()["mass_sum"] - exact) <= (tiles + 2) * 2.0 ** -53 * exact
