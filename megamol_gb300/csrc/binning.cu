@@ -550,9 +550,9 @@ __global__ void __launch_bounds__(SORT_THREADS, 3) onesweep_kernel(const uint32_
 // start[c] = first sorted position whose key is >= c, for c in [0, nbins]. Boundary i of the sorted keys (between
 // keys[i-1] and keys[i]) starts the run of cells (keys[i-1], keys[i]]. A warp takes 32 consecutive boundaries, scans the
 // lengths of their runs, and its lanes write the cells of all 32 runs together (consecutive lanes, consecutive cells:
-// coalesced however long the runs are). A run of more than RUN_MAX cells (a sparse grid holds runs of millions of empty cells) is queued in chunks of
+// coalesced however long the runs are). A run of more than run_max cells (a sparse grid holds runs of millions of empty cells) is queued in chunks of
 // at most GAP_CHUNK for cell_gap_fill_kernel. Such runs are disjoint, so the chunks number at most (nbins + 1)
-// (1 / GAP_CHUNK + 1 / (RUN_MAX + 1)), below the nbins / 64 + 2 entries the list holds.
+// (1 / GAP_CHUNK + 1 / (run_max + 1)), below the nbins / 64 + 2 entries the list holds (run_max >= 64).
 // After a radix sort whose look-back gave up (err), every particle gets the invalid key nbins and the identity order, a
 // valid sorted state (an empty grid), so that no later stage indexes with unfinished output; the frame reports
 // P2V_ETIMEOUT.
@@ -560,11 +560,10 @@ __global__ void __launch_bounds__(SORT_THREADS, 3) onesweep_kernel(const uint32_
 // cell 0.45 ms, bound by issue; a search per cell in a table of every 64th cell's start, as sparse frames took before,
 // 1.39 ms.
 constexpr uint32_t GAP_CHUNK = 8192;
-constexpr uint32_t RUN_MAX = 8192;
 
 __global__ void __launch_bounds__(256) boundary_starts_kernel(uint32_t* __restrict__ keys,
-    uint32_t* __restrict__ vals, uint32_t n, uint32_t nbins, uint32_t* __restrict__ out, uint4* __restrict__ gaps, uint32_t gap_cap,
-    FrameScalars* __restrict__ fs, const FrameScalars* __restrict__ gate) {
+    uint32_t* __restrict__ vals, uint32_t n, uint32_t nbins, uint32_t run_max, uint32_t* __restrict__ out,
+    uint4* __restrict__ gaps, uint32_t gap_cap, FrameScalars* __restrict__ fs, const FrameScalars* __restrict__ gate) {
     chain_begin();
     if (radix_skipped(gate))
         return;
@@ -591,7 +590,7 @@ __global__ void __launch_bounds__(256) boundary_starts_kernel(uint32_t* __restri
             }
         }
         uint32_t len = lo <= hi ? hi - lo + 1u : 0u;
-        const bool queued = len > RUN_MAX;
+        const bool queued = len > run_max;
         if (queued) {
             const uint32_t i = (uint32_t) i64;
             const uint32_t nch = (uint32_t) (((uint64_t) len - 1 + GAP_CHUNK) / GAP_CHUNK);
@@ -1059,6 +1058,17 @@ size_t bin_scan_words(uint32_t nbins) {
     return (size_t) ceil_div(nbins + 1, SCAN_TILE);
 }
 
+namespace {
+// The longest run of empty cells that boundary_starts_kernel writes itself. A warp writes its 32 runs one after the other,
+// about 0.1 us for 32 cells, while few boundaries leave most of the SMs idle; a queued run takes about 0.7 us of one of
+// the fill's 304 blocks. The two are even at runs of n / 25 to n / 40. Binning, all but the shortest runs queued (64) /
+// this rule / 8192 always, ms: 300 particles in 0.3 M cells 0.026 / 0.026 / 0.065, 10,000 in 65 M 0.091 / 0.091 / 0.249,
+// 30,000 in 16 M 0.089 / 0.075 / 0.072, 300,000 in 126 M 0.62 / 0.15 / 0.15.
+uint32_t longest_run(uint32_t n) {
+    return std::max<uint32_t>(64u, std::min<uint32_t>(8192u, n / 25));
+}
+}  // namespace
+
 cudaError_t launch_bin_sort(SortBuffers& b, uint32_t n, const GridGeo& g, uint32_t* counts, uint32_t* start,
                             uint4* gaps, uint32_t gap_cap, FrameScalars* fs, int sms,
                             cudaStream_t st) {
@@ -1096,8 +1106,8 @@ cudaError_t launch_bin_sort(SortBuffers& b, uint32_t n, const GridGeo& g, uint32
             return e;
     }
     const unsigned grid = (unsigned) std::max<uint32_t>(1u, std::min<uint32_t>(ceil_div(n + 1, 256), sms * 8));
-    chain(boundary_starts_kernel, grid, 256, 0, st, b.keys[b.result], b.vals[b.result], n, g.nbins, start, gaps, gap_cap, fs,
-                                                 gate);
+    chain(boundary_starts_kernel, grid, 256, 0, st, b.keys[b.result], b.vals[b.result], n, g.nbins, longest_run(n), start,
+          gaps, gap_cap, fs, gate);
     chain(cell_gap_fill_kernel, sms * 2, 256, 0, st, gaps, gap_cap, start, fs, gate);
     return cudaGetLastError();
 }

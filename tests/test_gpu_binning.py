@@ -234,3 +234,15 @@ def test_which_sort_takes_a_crowded_cell(ctx, fill, invalid):
     finally:
         ctx.set_params(sort_wait_polls=0, test_hold_sort=0)
     assert check(ctx, x, (0.0, 0.0, 0.0, 30.0, 30.0, 30.0), (30, 30, 30)) == max(fill, invalid)
+
+
+@pytest.mark.parametrize("n,res", [(1_600, 64), (2_500, 100), (25_000, 220), (100_000, 256), (300_000, 330)])
+@pytest.mark.parametrize("spread", [None, 0.5])
+def test_sparse_frames_around_the_longest_run(ctx, n, res, spread):
+    """Runs of empty cells on both sides of the longest that a warp writes itself (64 cells for the smallest frames, n / 25,
+    8192 for the largest), evenly spread and around one blob."""
+    rng = np.random.default_rng(n)
+    x = np.empty((n, 4), np.float32)
+    x[:, :3] = rng.uniform(0, 10, (n, 3)) if spread is None else np.clip(5 + rng.normal(0, spread, (n, 3)), 0, 10)
+    x[:, 3] = 8.0 / res
+    check(ctx, x, (0.0, 0.0, 0.0, 10.0, 10.0, 10.0), (res, res, res))
