@@ -507,7 +507,8 @@ p2v_status p2v_ctx::enqueue_frame(Pipe& pp, const p2v_frame* fr, p2v_volume* vol
     const uint32_t n = (uint32_t) N;
     GatherConfig gc{};
     if (P.accumulate == P2V_ACCUM_KAHAN) {
-        gc = GatherConfig{GATHER_KAHAN, 8, 16, 16, 1024, 512};
+        gc = GatherConfig{GATHER_KAHAN, 8, 16, 16, 0, 512};
+        gc.smax = kahan_staged(gather_tile_count(gc, g), sms);
     } else if (P.accumulate == P2V_ACCUM_EXACT) {
         gc = GatherConfig{GATHER_EXACT, 16, 16, 16, 0, 512};
         if (P.tile_x > 0 || P.tile_y > 0 || P.tile_z > 0)

@@ -82,9 +82,9 @@ __device__ __forceinline__ void tile_extent(const GridGeo& g, FrameScalars* fs, 
     ex.khi[a] = khi;
 }
 
-// Bound by latency at 14 active lanes per instruction (the nodes' candidate lists differ). Three CTAs per SM (80 registers,
-// 1024 staged records: a tile of an LJ liquid's 940 in one chunk) and the row table's scan by the whole CTA: LJ 864k
-// 0.247 ms, where two CTAs with 2048 records and a one-warp scan took 0.346; 768 records 0.32, four CTAs 0.26.
+// Bound by latency at 14 active lanes per instruction (the nodes' candidate lists differ). Three CTAs per SM (80 registers)
+// and the row table's scan by the whole CTA: LJ 864k 0.260 ms, where two CTAs and a one-warp scan took 0.367; four CTAs
+// 0.26. How many records it stages: kahan_staged.
 template<int TX, int TY, int TZ>
 __global__ void __launch_bounds__(TY* TZ, 3) gather_kernel(GridGeo g, const float4* __restrict__ rec_a,
     const int4* __restrict__ rec_b, const uint32_t* __restrict__ start, float* __restrict__ grid,
@@ -1184,6 +1184,14 @@ uint32_t gather_tiles_z(const GatherConfig& c, const GridGeo& g) {
 
 uint32_t gather_tile_count(const GatherConfig& c, const GridGeo& g) {
     return ceil_div(g.s[0], c.tx) * ceil_div(g.s[1], c.ty) * gather_tiles_z(c, g);
+}
+
+// A chunk of staged records occupies only the threads whose rows it holds, so a crowded tile goes as fast as its chunks are
+// large: as many records as fit beside the tile's sums for the CTAs that an SM gets. Density, ms, 1024 records always / this
+// rule: 20k particles in 12 tiles of a 17^3 grid 4.51 / 1.10, 100k in 54 tiles 0.60 / 0.19, 500k in 250 tiles 0.44 / 0.25, a
+// blob of 500k in 1024 tiles 1.42 / 1.02, LJ 864k (940 records a tile: one chunk) 0.256 / 0.260. 2048 for two CTAs: LJ 0.342.
+int kahan_staged(uint32_t tiles, int sms) {
+    return tiles <= (uint32_t) sms ? 6400 : tiles <= 2u * (uint32_t) sms ? 2816 : 1728;
 }
 
 GatherHeavy gather_heavy_plan(const GatherConfig& c, uint32_t n, int sms, size_t* bytes) {

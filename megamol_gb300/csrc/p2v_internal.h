@@ -155,6 +155,8 @@ cudaError_t launch_gather(const GatherConfig& c, const GridGeo& g, const float4*
     const uint32_t* start, const GatherPasses& ps, TileStats* tiles, FrameScalars* fs, const GatherHeavy& hv, void* hbuf,
     int sms, cudaStream_t st);
 uint32_t gather_tile_count(const GatherConfig& c, const GridGeo& g);
+// Records that the Kahan gather stages at a time, for a grid of so many tiles
+int kahan_staged(uint32_t tiles, int sms);
 // Reduce the tile statistics (fixed order, FP64 sum) and derive the normalisation of the grid.
 cudaError_t launch_finalize(const TileStats* tiles, uint32_t ntiles, FrameScalars* fs, int mass_normalize,
     int minmax_normalize, double n_scale, double voxel_volume, cudaStream_t st);

@@ -356,3 +356,17 @@ def test_mass_sum_is_the_sum_of_the_grid(ctx, n, radius, tile):
     tiles = 4 * 4 * 3 if tile == 16 else 4 * 7 * 6
     assert vol.max() > 1.0
     assert abs(ctx.stats()["mass_sum"] - exact) <= (tiles + 2) * 2.0 ** -53 * exact
+
+
+@pytest.mark.parametrize("res", [(17, 17, 17), (48, 47, 49), (80, 81, 79), (97, 97, 96)])
+@pytest.mark.parametrize("n,spread", [(1_000, 0.5), (60_000, 1.0), (60_000, 6.0)])
+def test_kahan_gather_of_crowded_tiles(ctx, res, n, spread):
+    """Grids of so few tiles that an SM holds one CTA, two and three (they stage 6400, 2816 and 1728 records at a time), with
+    tiles of fewer records than that and of many chunks: the FP64 bar, and the same bits again."""
+    x = crowd(n, 24.0, spread, 1.2 * 24.0 / 96, n + res[0])
+    bbox = (0, 0, 0, 24.0, 24.0, 24.0)
+    vol, _ = run(ctx, [p2v.ParticleList(x)], bbox, res, accumulate=p2v.ACCUM_KAHAN)
+    ref = oracle.density_f64(x, bbox, res, (1, 1, 1), 1.0, oracle.BUMP, NT)
+    assert maxrel(vol, ref) <= 1e-6, maxrel(vol, ref)
+    again, _ = run(ctx, [p2v.ParticleList(x)], bbox, res, accumulate=p2v.ACCUM_KAHAN)
+    assert np.array_equal(vol, again)
