@@ -246,8 +246,10 @@ cudaError_t launch_mdao_volume(const MdaoParams& mp, const uint32_t* order, cons
     if (e != cudaSuccess)
         return e;
     if (n > 0) {
-        // spheres per warp: up to 16, fewer where that leaves an SM less than 32 warps
-        const uint32_t batch = std::max<uint32_t>(1u, std::min<uint32_t>(16u, n / (uint32_t) (sms * 32)));
+        // Spheres per warp: up to 16, fewer where that leaves an SM less than 64 warps (40 are resident; large spheres need
+        // more warps than that to share them evenly). Voxelisation at 1 / 2 / 4 / 16 spheres per warp, us: 20,000 of radius
+        // 1.4 voxels 77 / 61 / 58 / 65, of 13 voxels 2440 / 2600 / 3030 / 5530; 250,000 of 1.4 voxels 517 / 301 / 235 / 173.
+        const uint32_t batch = std::max<uint32_t>(1u, std::min<uint32_t>(16u, n / (uint32_t) (sms * 64)));
         const unsigned grd = (unsigned) std::max<uint64_t>(1, std::min<uint64_t>((ceil_div(n, batch) + 7) / 8, (uint64_t) sms * 64));
         if (mp.unorm8)
             chain(mdao_voxelise_kernel<true>, grd, 256, 0, st, mp, order, xyzr, n, batch, acc);

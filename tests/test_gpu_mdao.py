@@ -112,3 +112,13 @@ def test_mdao_volume_of_sphere_batches(ctx, n, rmin, rmax, vs, unorm8):
     dims, _, _ = oracle.mdao_dims(f.bbox, vs)
     ref = oracle.mdao_volume_f32(f.xyzr, f.bbox, dims, unorm8=bool(unorm8))
     assert np.array_equal(ctx.ao_volume(0), ref)
+
+
+@pytest.mark.parametrize("n", [9_727, 19_456, 19_457, 160_001])
+def test_mdao_volume_at_the_batch_limits(ctx, n):
+    """The last size with one sphere per warp, the first with two and the next, and one of sixteen. Bit for bit."""
+    f = frame(n=n, seed=35)
+    f.xyzr[:, 3] = np.random.default_rng(n).uniform(0.05, 0.6, n).astype(np.float32)
+    run(ctx, f, synth.random_normals(n, 3), mdao_volume_size=48, mdao_unorm8=1)
+    dims, _, _ = oracle.mdao_dims(f.bbox, 48)
+    assert np.array_equal(ctx.ao_volume(0), oracle.mdao_volume_f32(f.xyzr, f.bbox, dims, unorm8=True))
