@@ -550,7 +550,8 @@ __global__ void __launch_bounds__(SORT_THREADS, 3) onesweep_kernel(const uint32_
 // start[c] = first sorted position whose key is >= c, for c in [0, nbins]. Boundary i of the sorted keys (between
 // keys[i-1] and keys[i]) starts the run of cells (keys[i-1], keys[i]]. A warp takes 32 consecutive boundaries, scans the
 // lengths of their runs, and its lanes write the cells of all 32 runs together (consecutive lanes, consecutive cells:
-// coalesced however long the runs are). A run of more than run_max cells (a sparse grid holds runs of millions of empty cells) is queued in chunks of
+// coalesced however long the runs are). A run of more than run_max cells (a sparse grid
+// holds runs of millions of empty cells) is queued in chunks of
 // at most GAP_CHUNK for cell_gap_fill_kernel. Such runs are disjoint, so the chunks number at most (nbins + 1)
 // (1 / GAP_CHUNK + 1 / (run_max + 1)), below the nbins / 64 + 2 entries the list holds (run_max >= 64).
 // After a radix sort whose look-back gave up (err), every particle gets the invalid key nbins and the identity order, a
@@ -560,6 +561,34 @@ __global__ void __launch_bounds__(SORT_THREADS, 3) onesweep_kernel(const uint32_
 // cell 0.45 ms, bound by issue; a search per cell in a table of every 64th cell's start, as sparse frames took before,
 // 1.39 ms.
 constexpr uint32_t GAP_CHUNK = 8192;
+
+// Queues a warp's runs [lo, hi] of boundaries base + lane: a lane the chunks of its run, the warp together those of a run of
+// many. (One lane writing a million empty cells' chunks held its warp for as long as a hundred others took: a blob of 1 M
+// in 512 M cells 1.39 -> 0.57 ms of binning. Not inlined: the registers it would take cost the warps without a queued run
+// 10 to 20 %.)
+__device__ __noinline__ void queue_runs(bool queued, uint32_t lo, uint32_t hi, uint32_t base, uint32_t lane,
+                                        uint4* __restrict__ gaps, uint32_t gap_cap, FrameScalars* __restrict__ fs) {
+    constexpr uint32_t MANY = 8;
+    const uint32_t nch = queued ? (hi - lo) / GAP_CHUNK + 1u : 0u;
+    const uint32_t slot = queued ? atomicAdd(&fs->ngaps, nch) : 0u;
+    auto put = [&](uint32_t at, uint32_t q, uint32_t first, uint32_t last, uint32_t i) {
+        const uint32_t c0 = first + q * GAP_CHUNK;
+        if ((uint64_t) at + q < gap_cap)
+            gaps[at + q] = make_uint4(c0, last - c0 < GAP_CHUNK ? last : c0 + (GAP_CHUNK - 1u), i, 0u);
+        else
+            atomicOr(&fs->error, ERR_GAP_OVERFLOW);
+    };
+    if (nch < MANY)
+        for (uint32_t q = 0; q < nch; ++q)
+            put(slot, q, lo, hi, base + lane);
+    for (uint32_t m = __ballot_sync(0xffffffffu, nch >= MANY); m; m &= m - 1u) {
+        const int l = __ffs(m) - 1;
+        const uint32_t first = __shfl_sync(0xffffffffu, lo, l), last = __shfl_sync(0xffffffffu, hi, l);
+        const uint32_t at = __shfl_sync(0xffffffffu, slot, l), k = __shfl_sync(0xffffffffu, nch, l);
+        for (uint32_t q = lane; q < k; q += 32)
+            put(at, q, first, last, base + (uint32_t) l);
+    }
+}
 
 __global__ void __launch_bounds__(256) boundary_starts_kernel(uint32_t* __restrict__ keys,
     uint32_t* __restrict__ vals, uint32_t n, uint32_t nbins, uint32_t run_max, uint32_t* __restrict__ out,
@@ -591,19 +620,11 @@ __global__ void __launch_bounds__(256) boundary_starts_kernel(uint32_t* __restri
         }
         uint32_t len = lo <= hi ? hi - lo + 1u : 0u;
         const bool queued = len > run_max;
-        if (queued) {
-            const uint32_t i = (uint32_t) i64;
-            const uint32_t nch = (uint32_t) (((uint64_t) len - 1 + GAP_CHUNK) / GAP_CHUNK);
-            const uint32_t slot = atomicAdd(&fs->ngaps, nch);
-            for (uint32_t q = 0; q < nch; ++q) {
-                const uint64_t c0 = (uint64_t) lo + (uint64_t) q * GAP_CHUNK;
-                const uint64_t c1 = std::min<uint64_t>(hi, c0 + GAP_CHUNK - 1);
-                if ((uint64_t) slot + q < gap_cap)
-                    gaps[slot + q] = make_uint4((uint32_t) c0, (uint32_t) c1, i, 0u);
-                else
-                    atomicOr(&fs->error, ERR_GAP_OVERFLOW);
-            }
-            len = 0u;
+        const uint32_t queues = __ballot_sync(0xffffffffu, queued);
+        if (queues) {
+            queue_runs(queued, lo, hi, (uint32_t) base, lane, gaps, gap_cap, fs);
+            if (queued)
+                len = 0u;
         }
         uint32_t incl = len;
 #pragma unroll
@@ -614,7 +635,7 @@ __global__ void __launch_bounds__(256) boundary_starts_kernel(uint32_t* __restri
         }
         const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
         const uint32_t pre = incl - len;  // first cell slot of this lane's run
-        if (!failed && !__any_sync(0xffffffffu, queued)) {
+        if (!failed && !queues) {
             // the runs of consecutive boundaries follow each other: cell slot j is cell lo(lane 0) + j. Its owner is the
             // last run that has started, by one reduction and a population count.
             const uint32_t cell0 = __shfl_sync(0xffffffffu, lo, 0);
@@ -662,7 +683,7 @@ __global__ void __launch_bounds__(256) cell_gap_fill_kernel(const uint4* __restr
     const uint32_t ng = min(fs->ngaps, gap_cap);
     for (uint32_t g = blockIdx.x; g < ng; g += gridDim.x) {
         const uint4 e = gaps[g];
-        for (uint32_t c = e.x + threadIdx.x; c <= e.y; c += blockDim.x)
+        for (uint64_t c = (uint64_t) e.x + threadIdx.x; c <= e.y; c += blockDim.x)  // (e.y may lie near 2^32)
             start[c] = e.z;
     }
 }
@@ -1105,7 +1126,8 @@ cudaError_t launch_bin_sort(SortBuffers& b, uint32_t n, const GridGeo& g, uint32
         if (e != cudaSuccess)
             return e;
     }
-    const unsigned grid = (unsigned) std::max<uint32_t>(1u, std::min<uint32_t>(ceil_div(n + 1, 256), sms * 8));
+    // (gated, the blocks return at once in most frames; else 32 per SM: uniform 16M 1.06 ms of binning against 1.07 with 8)
+    const unsigned grid = (unsigned) std::max<uint32_t>(1u, std::min<uint32_t>(ceil_div(n + 1, 256), sms * (gate ? 8 : 32)));
     chain(boundary_starts_kernel, grid, 256, 0, st, b.keys[b.result], b.vals[b.result], n, g.nbins, longest_run(n), start,
           gaps, gap_cap, fs, gate);
     chain(cell_gap_fill_kernel, sms * 2, 256, 0, st, gaps, gap_cap, start, fs, gate);
