@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(TY* TZ, 3) gather_kernel(GridGeo g, const floa
 // Bound by issue slots, and on sparse frames by the latency of the phases around the walk (row table, output): 68 % of
 // the issue slots on LJ 4M. A warp's 32 lanes take 32 (particle, x-row) items at a time; about 11 lanes add a node in an
 // average step of the x loop, and an item costs about 35 instructions around it (LJ 4M 0.278 ms, mixed 64M 1.27 ms,
-// uniform 16M 3.65 ms, four passes of 500k 0.128 ms). Before: one addition per node whose old value gave the carry, a
+// uniform 16M 3.67 ms, four passes of 500k 0.128 ms). Before: one addition per node whose old value gave the carry, a
 // binary search per item, conversions on the special-function unit and whole batches dealt to the warps: 0.369, 1.75,
 // 5.73 and 0.249 ms. Skipping the x loop, uniform 16M takes 1.79 ms, of that 0.18 the box set-up, 0.73 the row table,
 // 0.59 the output.
